@@ -997,10 +997,17 @@ __global__ void __launch_bounds__(256) gemv_tiles_ring_kernel(TileArgs a) {
     }
 }
 
+// TSB_MOE_MMA=0: no int8 matrix instructions, every type takes gemv_tiles_kernel.
+static bool moe_mma_on() {
+    static const bool on = []() { const char* e = getenv("TSB_MOE_MMA"); return !e || atoi(e) != 0; }();
+    return on;
+}
+
 // Whether the ring kernel takes a projection: 4-bit blocks of 32 with their scales in a plane whose 64-row pieces start on 16
-// bytes, and a K whose activations fit beside the ring.
+// bytes, and a K whose activations fit beside the ring.  Both the height of the tiles and the kernel that serves them follow from
+// this one answer.
 static bool moe_ring_ok(int type, int N, int K, bool glu) {
-    if ((type != TSB_MXFP4 && type != TSB_Q4_0) || K % 32 != 0 || N <= 0) return false;
+    if (!moe_mma_on() || (type != TSB_MXFP4 && type != TSB_Q4_0) || K % 32 != 0 || N <= 0) return false;
     const bool mx = type == TSB_MXFP4;
     const long n_out = glu ? N / 2 : N, sb = mx ? 1 : 2;
     if ((n_out * (K / 32) * sb) % 16 != 0) return false;
@@ -1027,9 +1034,10 @@ static int launch_ring(const TileArgs& a, int max_tiles, cudaStream_t s) {
     return TSB_OK;
 }
 
+// `tile_rows`: most rows of a tile in the list (what it was built with); more than MOE_TILE_ROWS only where the ring kernel serves.
 extern "C" int tsb_moe_gemv_tiles(const void* p0, const void* p1, const void* p2, const void* p3, int type, int N, int K,
                                   const void* xq, const void* xds, const void* xb, void* out, const float* bias,
-                                  const float* row_scale, const void* tiles, const int* meta, int max_tiles, int out_f32,
+                                  const float* row_scale, const void* tiles, const int* meta, int max_tiles, int tile_rows, int out_f32,
                                   int act, void* stream) {
     TSB_CHECK_ARG(N > 0 && K > 0 && max_tiles >= 0, "moe_gemv_tiles: bad shape N=%d K=%d tiles=%d", N, K, max_tiles);
     const bool q8 = type == TSB_Q4_K || type == TSB_Q5_K || type == TSB_Q6_K || type == TSB_Q8_0 || type == TSB_MXFP4 ||
@@ -1041,17 +1049,19 @@ extern "C" int tsb_moe_gemv_tiles(const void* p0, const void* p1, const void* p2
     const bool glu = act >= ACT_SWIGLU && act <= ACT_SWIGLU_OAI;
     TSB_CHECK_ARG(!glu || N % 2 == 0, "moe_gemv_tiles: GLU needs an even row count, got %d", N);
     TSB_CHECK_ARG(max_tiles <= 65535, "moe_gemv_tiles: %d tiles exceed the grid limit", max_tiles);
+    const bool ring = moe_ring_ok(type, N, K, glu);
+    TSB_CHECK_ARG(tile_rows > 0 && tile_rows <= (ring ? MOE_RING_ROWS : MOE_TILE_ROWS), "moe_gemv_tiles: tiles of %d rows of weight type %d, K=%d",
+                  tile_rows, type, K);
     if (max_tiles == 0) return TSB_OK;
     TileArgs a;
     a.w = QW{(const uint8_t*)p0, (const uint8_t*)p1, (const uint8_t*)p2, (const uint8_t*)p3, type, N, K};
     a.xq = (const int8_t*)xq; a.xds = (const float2*)xds; a.xb = (const bf16*)xb;
     a.out = out; a.bias = bias; a.row_scale = row_scale; a.tiles = (const int4*)tiles; a.meta = meta;
     a.out_f32 = out_f32; a.act = act; a.n_out = glu ? N / 2 : N;
-    static const bool use_mma = []() { const char* e = getenv("TSB_MOE_MMA"); return !e || atoi(e) != 0; }();
-    if (use_mma && (type == TSB_MXFP4 || type == TSB_Q4_0)) {
+    if (moe_mma_on() && (type == TSB_MXFP4 || type == TSB_Q4_0)) {
         dim3 grid((a.n_out + 63) / 64, max_tiles), block(128);
         cudaStream_t st = (cudaStream_t)stream;
-        if (moe_ring_ok(type, N, K, glu)) {
+        if (ring) {
             if (type == TSB_MXFP4) return glu ? launch_ring<true, true>(a, max_tiles, st) : launch_ring<false, true>(a, max_tiles, st);
             return glu ? launch_ring<true, false>(a, max_tiles, st) : launch_ring<false, false>(a, max_tiles, st);
         }

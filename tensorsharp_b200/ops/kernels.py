@@ -229,7 +229,7 @@ def moe_grouped(*, xq=None, xds=None, xb=None, ids: torch.Tensor, weights: torch
                 down: QuantWeight, act, gate_up_bias=None, down_bias=None, expert_offset: int = 0, shared=None, residual=None) -> torch.Tensor:
     """Grouped expert projections with the routing kept on the device (no host read-back, fixed launch
     sequence): group the (token, slot) pairs by local expert, gather activations into that order, run
-    gate/up and down as tile GEMVs (each tile streams its expert's rows once for up to 8 pairs), and
+    gate/up and down as tile GEMVs (each tile streams its expert's rows once for up to 8 pairs, 16 in 4-bit blocks), and
     sum every token's slots.  ``ids`` are global expert ids [T, k]; pairs whose expert is not in
     ``[expert_offset, expert_offset + gate_up.experts)`` contribute nothing.  Returns f32 [T, D]."""
     lib = _lib()
@@ -265,7 +265,7 @@ def moe_grouped(*, xq=None, xds=None, xb=None, ids: torch.Tensor, weights: torch
     ps = _planes(gate_up)
     native.check(lib.tsb_moe_gemv_tiles(ps[0], ps[1], ps[2], ps[3], C.c_int(int(gate_up.ggml_type)), C.c_int(gate_up.N), C.c_int(K),
                                         _p(sq), _p(sds), _p(sb), _p(gu), _p(gate_up_bias), None, _p(tiles), _p(meta),
-                                        C.c_int(max_tiles), C.c_int(0), C.c_int(a), _stream()), "moe_gemv_tiles(gate_up)")
+                                        C.c_int(max_tiles), C.c_int(rows), C.c_int(0), C.c_int(a), _stream()), "moe_gemv_tiles(gate_up)")
     y = torch.empty((P, D), dtype=torch.float32, device=dev)
     ps = _planes(down)
     if down.uses_q8_activations:
@@ -276,7 +276,7 @@ def moe_grouped(*, xq=None, xds=None, xb=None, ids: torch.Tensor, weights: torch
         gb = gu
     native.check(lib.tsb_moe_gemv_tiles(ps[0], ps[1], ps[2], ps[3], C.c_int(int(down.ggml_type)), C.c_int(D), C.c_int(F_out),
                                         _p(gq), _p(gds), _p(gb), _p(y), _p(down_bias), _p(sw), _p(tiles), _p(meta),
-                                        C.c_int(max_tiles), C.c_int(1), C.c_int(0), _stream()), "moe_gemv_tiles(down)")
+                                        C.c_int(max_tiles), C.c_int(rows), C.c_int(1), C.c_int(0), _stream()), "moe_gemv_tiles(down)")
     _count(4)
     return moe_combine(y, pos, None, T, k, shared, residual)
 

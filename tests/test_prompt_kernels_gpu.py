@@ -1,4 +1,9 @@
 """Kernels of the prompt path and of batched experts against plain tensor arithmetic, at the sizes where their tiles end."""
+import ctypes as C
+import os
+import subprocess
+import sys
+
 import pytest
 import torch
 
@@ -122,6 +127,24 @@ def test_moe_tiles_of_sixteen(t, T, k, E, Kd, Fd):
         want += (torch.einsum("tk,tnk->tn", hd, D[e]) + db[e]) * w[:, j:j + 1].double()
     # a bf16 value on a rounding edge may fall the other way (2^-8 of it) and its int8 code with it (1 / 127 of its group's largest)
     assert rel(got, want) < 5e-3
+
+
+def test_moe_tiles_without_matrix_instructions():
+    """The same with TSB_MOE_MMA=0, which the library reads once per process: every tile then goes to a kernel of eight rows."""
+    r = subprocess.run([sys.executable, "-m", "pytest", "-q", "-x", f"{__file__}::test_moe_tiles_of_sixteen"], capture_output=True, text=True, timeout=600,
+                       env=dict(os.environ, TSB_MOE_MMA="0"))
+    assert r.returncode == 0, r.stdout[-3000:]
+
+
+def test_moe_tile_height_is_checked():
+    lib, w = K()._lib(), QuantWeight.from_float(torch.randn(1, 64, 64, device=DEV), GGMLType.Q8_0)
+    none = C.c_void_p(0)
+    some = K()._p(torch.zeros(1 << 12, dtype=torch.int8, device=DEV))
+
+    def call(rows, max_tiles=0):
+        return lib.tsb_moe_gemv_tiles(*K()._planes(w), C.c_int(int(w.ggml_type)), C.c_int(64), C.c_int(64), some, some, none, some, none, none, some, some,
+                                      C.c_int(max_tiles), C.c_int(rows), C.c_int(1), C.c_int(0), K()._stream())
+    assert call(8) == 0 and call(16) != 0 and call(0) != 0
 
 
 @pytest.mark.parametrize("Hq,Hkv,Dh,rot", [(8, 2, 64, 64), (5, 1, 128, 128), (4, 2, 256, 64), (3, 3, 128, 32), (16, 8, 128, 0)])
