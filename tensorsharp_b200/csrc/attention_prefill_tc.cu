@@ -10,9 +10,10 @@
 //     S(0) S(1) | PV(0) S(2) | PV(1) S(3) | ...        (key tile u: buffer u & 1)
 // P replaces S in place as bf16 (the A operand of PV comes from TMEM), O stays in TMEM until the end.
 //
-//   warps 0 .. 3 : softmax, one thread per row; rescales O itself, and only when the row maximum has grown by more
-//                  than 2^8 since the last time (the running sum uses the same stale maximum, so the result is the
-//                  same; P and the sum are at most 2^8 larger, far inside f32 and bf16 range)
+//   warps 0 .. 3 : softmax, one thread per row; rescales O itself, after the exponentials of the tile, whenever the maximum of one
+//                  of the warp's rows has grown.  (P is rounded to bf16.  Relative to the running maximum the largest weights
+//                  lie at or just below 1, where that costs least; relative to an older one, which would spare most of the
+//                  rescaling, the error of the result was up to a fifth larger.)
 //   warp 4       : TMA producer, K and V rings
 //   warp 5       : TMEM owner, zeroes the V rows past the end of the cache, issues the MMAs
 //
@@ -20,9 +21,9 @@
 // end (barriers, TMEM, first loads, output).  With 64-key tiles a CTA needs half of the SM's tensor memory and less than half
 // of its shared memory, so two CTAs cover each other's gaps; with 128-key tiles one CTA has fewer hand-overs per key.
 // Measured (us; mma.sync kernel of attention.cu / 128-key tiles / 64-key tiles), causal, 32 / 8 heads of 128: 2048 tokens
-// 253 / 55 / 43, 8192 tokens 3107 / 640 / 522 (1054 TFLOP/s), 1024 tokens - / 20.5 / 23.4, 555 tokens on 6100 cached ones
-// 341 / 67 / 98; 64 / 8 heads of 64, 8 x 1024 tokens 423 / 257 / 162, with a window of 128 179 / 197 / 98; 16 / 2 heads of
-// 256, 8192 tokens 4526 / - / 558.
+// 254 / 63 / 51, 8192 tokens 3111 / 655 / 562 (978 TFLOP/s), 1024 tokens 88 / 23 / 26, 555 tokens on 6100 cached ones
+// 360 / 80 / 113; 64 / 8 heads of 64, 8 x 1024 tokens 433 / 276 / 182, with a window of 128 179 / 204 / 106; 16 / 2 heads of
+// 256, 8192 tokens 4530 / - / 620.
 #include "attn_args.cuh"
 #include "tcgen05.cuh"
 
@@ -266,7 +267,7 @@ __global__ void __launch_bounds__(192, PrefillSmem<DH, BN, KS>::PER_SM) attn_pre
         const int qp = pos0 + tok, qp_first = pos0 + tok0 + quad * 32 / G, qp_last = qp_first + (31 / G);
         constexpr float LOG2E = 1.4426950408889634f;
         const float f = a.softcap > 0.f ? 1.f : a.scale, fl = f * LOG2E;
-        float ref = -INFINITY, sum = 0.f;                // the maximum that P is relative to (scaled, times log2 e), the row sum
+        float ref = -INFINITY, sum = 0.f;                // the running maximum (scaled, times log2 e) and the row sum
         bool ok = true;
         for (int i = 0; i < nt; ++i) {
             const int buf = i & 1;
@@ -297,27 +298,10 @@ __global__ void __launch_bounds__(192, PrefillSmem<DH, BN, KS>::PER_SM) attn_pre
             }
             const float top = fmaxf(fmaxf(m[0], m[1]), fmaxf(m[2], m[3])) * fl;
             float corr = 1.f;
-            if (ref == -INFINITY) {
-                ref = top;                               // nothing summed yet: O is zero or not yet written
-            } else if (top > ref + 8.f) {
-                corr = ex2(ref - top);
-                ref = top;
+            if (top > ref) {
+                if (ref != -INFINITY) corr = ex2(ref - top);
+                ref = top;                               // (from -inf: nothing summed yet, O is zero or not yet written)
                 sum *= corr;
-            }
-            if (i > 0 && __any_sync(0xffffffffu, corr != 1.f)) {
-                // S(i) was issued after PV(i - 2), so of the products only PV(i - 1) can be outstanding
-                if (!(ok = warp_wait(&o_full[(i - 1) & 1], ((i - 1) >> 1) & 1))) break;
-                fence_after_sync();
-#pragma unroll 1
-                for (int c = 0; c < DH / 32; ++c) {
-                    uint32_t o[32];
-                    tmem_ld32(t_o + c * 32, o);
-                    tmem_ld_wait();
-#pragma unroll
-                    for (int j = 0; j < 32; ++j) o[j] = __float_as_uint(__uint_as_float(o[j]) * corr);
-                    tmem_st16(t_o + c * 32, o);
-                    tmem_st16(t_o + c * 32 + 16, o + 16);
-                }
             }
             const float neg = ref == -INFINITY ? 0.f : -ref;
             float part[4] = {0.f, 0.f, 0.f, 0.f};
@@ -334,6 +318,21 @@ __global__ void __launch_bounds__(192, PrefillSmem<DH, BN, KS>::PER_SM) attn_pre
                 tmem_st16(t_s + c * 16, p);
             }
             sum += (part[0] + part[1]) + (part[2] + part[3]);
+            if (i > 0 && __any_sync(0xffffffffu, corr != 1.f)) {
+                // S(i) was issued after PV(i - 2), so of the products only PV(i - 1) can be outstanding
+                if (!(ok = warp_wait(&o_full[(i - 1) & 1], ((i - 1) >> 1) & 1))) break;
+                fence_after_sync();
+#pragma unroll 1
+                for (int c = 0; c < DH / 32; ++c) {
+                    uint32_t o[32];
+                    tmem_ld32(t_o + c * 32, o);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) o[j] = __float_as_uint(__uint_as_float(o[j]) * corr);
+                    tmem_st16(t_o + c * 32, o);
+                    tmem_st16(t_o + c * 32 + 16, o + 16);
+                }
+            }
             tmem_st_wait();
             fence_before_sync();
             __syncwarp();
