@@ -407,15 +407,25 @@ int launch(const AttnArgs& a, int G, int max_q, long q_rows, long cache_rows, in
 
 }  // namespace
 
-// Prompt attention on tcgen05.  `q_rows`: packed query rows of q and out; `cache_rows`: slots of the K and V caches, whose pages
-// hold a multiple of 64 slots; `status`: device word that a bounded wait which gave up sets.  Everything else as tsb_attn_prefill.
+// Whether tsb_attn_prefill_tc takes these arguments: one head size of 64, 128 or 256 and no form beyond window, sinks, soft cap
+// and a gate per head; pages of a multiple of 64 slots, which the 64-row loads never straddle; and q, the caches and out on
+// 16 bytes, which tensor maps and the 16-byte stores ask for (tsb_attn_prefill stores four bytes at a time).
+extern "C" int tsb_attn_prefill_tc_takes(const AttnArgs* args, long cache_rows) {
+    const AttnArgs& a = *args;
+    const uintptr_t all = reinterpret_cast<uintptr_t>(a.q) | reinterpret_cast<uintptr_t>(a.k_cache) | reinterpret_cast<uintptr_t>(a.v_cache) |
+                          reinterpret_cast<uintptr_t>(a.out);
+    return !attn_needs_vd(a) && (a.Dh == 64 || a.Dh == 128 || a.Dh == 256) && a.q_pos0 == nullptr && a.lse_out == nullptr && a.page_size > 0 &&
+           a.page_size % 64 == 0 && cache_rows >= 64 && (all & 15) == 0;
+}
+
+// Prompt attention on tcgen05.  `q_rows`: packed query rows of q and out; `cache_rows`: slots of the K and V caches;
+// `status`: device word that a bounded wait which gave up sets.  Everything else as tsb_attn_prefill.
 extern "C" int tsb_attn_prefill_tc(const AttnArgs* args, int max_q_len, long q_rows, long cache_rows, int* status, void* stream) {
     const AttnArgs& a = *args;
     TSB_CHECK_ARG(a.Hkv > 0 && a.Hq % a.Hkv == 0, "attn_prefill_tc: Hq=%d not a multiple of Hkv=%d", a.Hq, a.Hkv);
     TSB_CHECK_ARG(a.cu_q != nullptr && status != nullptr, "attn_prefill_tc: cu_q and the status word are required");
-    TSB_CHECK_ARG(!attn_needs_vd(a) && (a.Dh == 64 || a.Dh == 128 || a.Dh == 256) && a.q_pos0 == nullptr && a.lse_out == nullptr,
-                  "attn_prefill_tc: head size %d or a form that tsb_attn_prefill serves", a.Dh);
-    TSB_CHECK_ARG(a.page_size > 0 && a.page_size % 64 == 0 && cache_rows >= 64, "attn_prefill_tc: pages of %d slots in a cache of %ld", a.page_size, cache_rows);
+    TSB_CHECK_ARG(tsb_attn_prefill_tc_takes(args, cache_rows), "attn_prefill_tc: head size %d, pages of %d slots in a cache of %ld, a form or an alignment that tsb_attn_prefill serves",
+                  a.Dh, a.page_size, cache_rows);
     if (a.B == 0 || max_q_len == 0 || q_rows == 0) return TSB_OK;
     cudaStream_t s = (cudaStream_t)stream;
     int G = 1;

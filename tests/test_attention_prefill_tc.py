@@ -91,3 +91,16 @@ def test_as_exact_as_the_mma_kernel(Hq, Hkv, Dh, ql, n, peak):
         got = K.attn_prefill(q, kc, vc, table, kl, cu, ql, scale=Dh ** -0.5, Hq=Hq, Hkv=Hkv, Dh=Dh, page_size=64, q_pos0=pos0)
         err.append(((got.double() - want).norm() / want.norm()).item())
     assert err[0] < 1.03 * err[1], err
+
+
+def test_output_off_sixteen_bytes():
+    """A caller's output that starts on 8 bytes only: 16-byte stores may not reach it."""
+    from tensorsharp_b200.ops import kernels as K
+    torch.manual_seed(6)
+    kc, vc, table, (r,) = _paged([200], 2, 128, 64)
+    q = torch.randn(70, 8, 128, device=DEV).bfloat16()
+    cu, kl = torch.tensor([0, 70], dtype=torch.int32, device=DEV), torch.tensor([200], dtype=torch.int32, device=DEV)
+    buf = torch.zeros(4 + 70 * 8 * 128 + 4, dtype=torch.bfloat16, device=DEV)
+    K.attn_prefill(q, kc, vc, table, kl, cu, 70, scale=0.1, Hq=8, Hkv=2, Dh=128, page_size=64, out=buf[4:-4].view(70, 8, 128))
+    want = ref.attention(q, kc[r], vc[r], torch.arange(130, 200, device=DEV), scale=0.1)
+    assert ((buf[4:-4].view(70, 8, 128).float() - want).norm() / want.norm()).item() < 6e-3 and not buf[:4].any() and not buf[-4:].any()

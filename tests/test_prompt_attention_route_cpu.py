@@ -1,0 +1,36 @@
+"""Which prompts the tcgen05 attention kernel takes: the library's own answer, a host function that follows no pointer."""
+import ctypes as C
+
+import pytest
+
+from tensorsharp_b200.ops import kernels as K
+from tensorsharp_b200.ops import native
+
+pytestmark = pytest.mark.skipif(not native.available(), reason="the kernel library is not built here")
+
+
+def takes(cache_rows=4096, **kw):
+    a = K.AttnArgs()
+    plain = dict(q=1 << 20, k_cache=2 << 20, v_cache=3 << 20, out=4 << 20, block_table=5 << 20, kv_lens=6 << 20, cu_q=7 << 20, scale=0.1, B=2, Hq=8,
+                 Hkv=2, Dh=128, Dv=128, page_size=64, max_pages=40, splits=1)
+    for k, v in {**plain, **kw}.items():
+        setattr(a, k, v)
+    return bool(K._lib().tsb_attn_prefill_tc_takes(C.byref(a), C.c_long(cache_rows)))
+
+
+@pytest.mark.parametrize("Dh", [64, 128, 256])
+def test_plain_forms(Dh):
+    assert takes(Dh=Dh, Dv=Dh) and takes(Dh=Dh, Dv=0, page_size=256, window=100, sinks=1 << 22, softcap=30.0) and takes(Dh=Dh, Dv=Dh, gate=1 << 22, gate_tok=8)
+
+
+@pytest.mark.parametrize("name", ["q", "k_cache", "v_cache", "out"])
+@pytest.mark.parametrize("off", [2, 4, 8])
+def test_every_pointer_on_sixteen_bytes(name, off):
+    assert not takes(**{name: (1 << 20) + off}) and takes(**{name: (1 << 20) + 16})
+
+
+@pytest.mark.parametrize("kw", [dict(Dh=512, Dv=512), dict(Dh=96, Dv=96), dict(Dv=64), dict(page_size=16), dict(page_size=96), dict(cache_rows=32), dict(k_ld=2048),
+                                dict(v_ld=2048), dict(q_pos0=64), dict(lse_out=64), dict(keep_first=4), dict(slopes=64), dict(gate=64, gate_cols=1),
+                                dict(kv_scale=256), dict(log_r1=64), dict(sig_bias=64)])
+def test_what_stays_with_the_other_kernels(kw):
+    assert not takes(**kw)
