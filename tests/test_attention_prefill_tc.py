@@ -104,3 +104,21 @@ def test_output_off_sixteen_bytes():
     K.attn_prefill(q, kc, vc, table, kl, cu, 70, scale=0.1, Hq=8, Hkv=2, Dh=128, page_size=64, out=buf[4:-4].view(70, 8, 128))
     want = ref.attention(q, kc[r], vc[r], torch.arange(130, 200, device=DEV), scale=0.1)
     assert ((buf[4:-4].view(70, 8, 128).float() - want).norm() / want.norm()).item() < 6e-3 and not buf[:4].any() and not buf[-4:].any()
+
+
+def test_gate_through_the_public_call():
+    """F.attention names every form, at its neutral value: the route follows the values, and the bits those of the plain call."""
+    from tensorsharp_b200.ops import functional as F
+    from tensorsharp_b200.ops import kernels as K
+    torch.manual_seed(7)
+    T, n, Hq, Hkv, Dh = 90, 300, 8, 2, 128
+    kc, vc, table, (r,) = _paged([n], Hkv, Dh, 64)
+    q, gate = torch.randn(T, Hq, Dh, device=DEV).bfloat16(), torch.randn(T, Hq, device=DEV)
+    cu, kl = torch.tensor([0, T], dtype=torch.int32, device=DEV), torch.tensor([n], dtype=torch.int32, device=DEV)
+    pos = torch.arange(n - T, n, device=DEV, dtype=torch.int32)
+    batch = F.Batch(tokens=pos, positions=pos, slots=pos.long(), cu_q=cu, kv_lens=kl, block_table=table, last_idx=None, seq_slots=None, max_q_len=T,
+                    max_kv_len=n, is_decode=False, page_size=64, h_cu_q=(0, T), h_kv_lens=(n,))
+    got = F.attention(q, kc, vc, batch, scale=0.1, Hq=Hq, Hkv=Hkv, Dh=Dh, gate=gate)
+    plain = K.attn_prefill(q, kc, vc, table, kl, cu, T, scale=0.1, Hq=Hq, Hkv=Hkv, Dh=Dh, page_size=64, gate=gate)
+    want = ref.attention(q, kc[r], vc[r], pos, scale=0.1) * torch.sigmoid(gate)[..., None]
+    assert ((plain.float() - want).norm() / want.norm()).item() < 6e-3 and torch.equal(got.view_as(plain), plain)
