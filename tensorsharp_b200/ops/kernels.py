@@ -86,6 +86,7 @@ class AttnArgs(C.Structure):
 
 
 _configured = False
+_prefill_tc = False   # whether the library has the tcgen05 prompt attention
 LAUNCHES = 0          # kernels launched through this module (eager mode; graph replays add theirs)
 
 
@@ -95,9 +96,13 @@ def _count(n: int = 1) -> None:
 
 
 def _lib():
-    global _configured
+    global _configured, _prefill_tc
     lib = native.lib()
     if not _configured:
+        # a library linked from a selection of sources may do without it; in the whole one it can only be missing from an old build
+        _prefill_tc = hasattr(lib, "tsb_attn_prefill_tc_takes")
+        if not _prefill_tc and native.is_whole(lib):
+            raise native.NativeLibraryError(f"{native.LIB_PATH} has no tsb_attn_prefill_tc_takes: it is older than this package, build it again")
         for name in ("tsb_quantize_q8", "tsb_gemv", "tsb_rmsnorm", "tsb_qkv_rope", "tsb_glu", "tsb_gather_rows",
                      "tsb_argmax", "tsb_rope_table", "tsb_fused_gemv", "tsb_gemv_push", "tsb_tp_reduce_norm", "tsb_tpseq_push_rows", "tsb_decode_advance", "tsb_attn_decode", "tsb_attn_prefill", "tsb_gemm_bf16", "tsb_causal_conv1d", "tsb_gdn_recurrent",
                      "tsb_mamba2_recurrent"):
@@ -619,13 +624,13 @@ def attn_prefill(q, k_cache, v_cache, block_table, kv_lens, cu_q, max_q_len, *, 
                    page_size, B, Dv, gate, **forms)
     a.q_pos0 = q_pos0.data_ptr() if q_pos0 is not None else None
     a.lse_out = lse_out.data_ptr() if lse_out is not None else None
-    tc = getattr(_lib(), "tsb_attn_prefill_tc", None)          # absent from a library linked from a selection of sources
-    if (tc is not None and _lib().tsb_attn_prefill_tc_takes(C.byref(a), C.c_long(k_cache.shape[0])) and q.is_contiguous()
+    lib = _lib()
+    if (_prefill_tc and lib.tsb_attn_prefill_tc_takes(C.byref(a), C.c_long(k_cache.shape[0])) and q.is_contiguous()
             and k_cache.is_contiguous() and v_cache.is_contiguous() and k_cache.shape[0] == v_cache.shape[0]):
-        native.check(tc(C.byref(a), C.c_int(max_q_len), C.c_long(q.shape[0]), C.c_long(k_cache.shape[0]), _p(gemm_status(q.device)), _stream()),
-                     "attn_prefill_tc")
+        native.check(lib.tsb_attn_prefill_tc(C.byref(a), C.c_int(max_q_len), C.c_long(q.shape[0]), C.c_long(k_cache.shape[0]),
+                                             _p(gemm_status(q.device)), _stream()), "attn_prefill_tc")
     else:
-        native.check(_lib().tsb_attn_prefill(C.byref(a), C.c_int(max_q_len), _stream()), "attn_prefill")
+        native.check(lib.tsb_attn_prefill(C.byref(a), C.c_int(max_q_len), _stream()), "attn_prefill")
     _count(1)
     return out
 

@@ -169,6 +169,11 @@ def _open(path: Path) -> ctypes.CDLL:
     return handle
 
 
+def is_whole(handle: ctypes.CDLL) -> bool:
+    """Whether this is the library of all sources, not one linked from a selection of them."""
+    return Path(handle._name) == LIB_PATH
+
+
 def available() -> bool:
     return LIB_PATH.exists()
 

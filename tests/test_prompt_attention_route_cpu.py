@@ -34,3 +34,18 @@ def test_every_pointer_on_sixteen_bytes(name, off):
                                 dict(kv_scale=256), dict(log_r1=64), dict(sig_bias=64)])
 def test_what_stays_with_the_other_kernels(kw):
     assert not takes(**kw)
+
+
+def test_a_whole_library_without_the_kernel_is_refused(monkeypatch):
+    """An old build is an error, not the slower kernel; a library of selected sources may lack it."""
+    class Old:
+        pass
+    old = Old()
+    monkeypatch.setattr(K, "_configured", False)
+    monkeypatch.setattr(K, "_prefill_tc", True)
+    monkeypatch.setattr(native, "lib", lambda: old)
+    old._name = str(native.LIB_PATH)
+    with pytest.raises(native.NativeLibraryError, match="build it again"):
+        K._lib()
+    old._name = str(native.OUT_DIR / "libtsb200-part-0.so")
+    assert K._lib() is old and K._prefill_tc is False
