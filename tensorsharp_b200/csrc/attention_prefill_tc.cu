@@ -405,17 +405,38 @@ int launch(const AttnArgs& a, int G, int max_q, long q_rows, long cache_rows, in
     return TSB_OK;
 }
 
+// Heads packed into a row tile: the largest power of two that divides Hq / Hkv, at most 16.
+int packed_heads(const AttnArgs& a) {
+    int G = 1;
+    while (G < 16 && (a.Hq / a.Hkv) % (2 * G) == 0) G *= 2;
+    return G;
+}
+long prefill_ctas(const AttnArgs& a, int max_q_len) {
+    const int G = packed_heads(a);
+    return (long)((max_q_len + 128 / G - 1) / (128 / G)) * (a.Hq / G) * a.B;
+}
+
 }  // namespace
 
 // Whether tsb_attn_prefill_tc takes these arguments: one head size of 64, 128 or 256 and no form beyond window, sinks, soft cap
 // and a gate per head; pages of a multiple of 64 slots, which the 64-row loads never straddle; and q, the caches and out on
 // 16 bytes, which tensor maps and the 16-byte stores ask for (tsb_attn_prefill stores four bytes at a time).
-extern "C" int tsb_attn_prefill_tc_takes(const AttnArgs* args, long cache_rows) {
+// Left to tsb_attn_prefill are also the smallest prompts, whose time is a CTA's start and end (barriers and tensor memory here),
+// and small grids with a soft cap at head size 64, where its CTAs of 64 rows spread the tanh over more SMs.  Measured (us,
+// mma.sync / here): head size 64, up to 64 slots: 8 / 1 heads, 1 to 16 prompts 4.1 .. 5.0 / 5.1 .. 5.5, 32 prompts 5.7 .. 6.8 /
+// 5.1 .. 5.5; one KV head per query head, 6 or 16 of them, 1 to 32 prompts 4.1 .. 9.9 / 5.0 .. 10.6; 64 / 8 heads, 4 prompts 5.6 .. 6.8 /
+// 5.2 .. 5.5.  Soft cap, head size 64: 38 CTAs 22.0 / 25.5, 64 CTAs 34 / 41, 72 CTAs 10.7 / 10.7, 80 CTAs 27.6 / 26.0, 128 CTAs
+// 50 / 41; head size 128, 64 slots 7.9 / 8.2.
+extern "C" int tsb_attn_prefill_tc_takes(const AttnArgs* args, int max_q_len, long cache_rows) {
     const AttnArgs& a = *args;
     const uintptr_t all = reinterpret_cast<uintptr_t>(a.q) | reinterpret_cast<uintptr_t>(a.k_cache) | reinterpret_cast<uintptr_t>(a.v_cache) |
                           reinterpret_cast<uintptr_t>(a.out);
-    return !attn_needs_vd(a) && (a.Dh == 64 || a.Dh == 128 || a.Dh == 256) && a.q_pos0 == nullptr && a.lse_out == nullptr && a.page_size > 0 &&
-           a.page_size % 64 == 0 && cache_rows >= 64 && (all & 15) == 0;
+    if (attn_needs_vd(a) || (a.Dh != 64 && a.Dh != 128 && a.Dh != 256) || a.q_pos0 != nullptr || a.lse_out != nullptr || a.page_size <= 0 ||
+        a.page_size % 64 != 0 || cache_rows < 64 || (all & 15) != 0 || a.Hkv <= 0 || a.Hq % a.Hkv != 0)
+        return 0;
+    const bool tiny = (long)a.max_pages * a.page_size <= 64, few = (long)a.Hq * a.B < 256;
+    if (a.Dh == 64 && ((tiny && (few || packed_heads(a) == 1)) || (a.softcap > 0.f && prefill_ctas(a, max_q_len) < 72))) return 0;
+    return !(a.Dh == 128 && a.softcap > 0.f && tiny && few);
 }
 
 // Prompt attention on tcgen05.  `q_rows`: packed query rows of q and out; `cache_rows`: slots of the K and V caches;
@@ -424,20 +445,23 @@ extern "C" int tsb_attn_prefill_tc(const AttnArgs* args, int max_q_len, long q_r
     const AttnArgs& a = *args;
     TSB_CHECK_ARG(a.Hkv > 0 && a.Hq % a.Hkv == 0, "attn_prefill_tc: Hq=%d not a multiple of Hkv=%d", a.Hq, a.Hkv);
     TSB_CHECK_ARG(a.cu_q != nullptr && status != nullptr, "attn_prefill_tc: cu_q and the status word are required");
-    TSB_CHECK_ARG(tsb_attn_prefill_tc_takes(args, cache_rows), "attn_prefill_tc: head size %d, pages of %d slots in a cache of %ld, a form or an alignment that tsb_attn_prefill serves",
+    TSB_CHECK_ARG(tsb_attn_prefill_tc_takes(args, max_q_len, cache_rows), "attn_prefill_tc: head size %d, pages of %d slots in a cache of %ld, a form or an alignment that tsb_attn_prefill serves",
                   a.Dh, a.page_size, cache_rows);
     if (a.B == 0 || max_q_len == 0 || q_rows == 0) return TSB_OK;
     cudaStream_t s = (cudaStream_t)stream;
-    int G = 1;
-    while (G < 16 && (a.Hq / a.Hkv) % (2 * G) == 0) G *= 2;
+    const int G = packed_heads(a);
     int dev = 0, sms = 148;
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     // 64-key tiles and two CTAs per SM once there are CTAs for that, else 128-key tiles (times of both at the top); at head
-    // size 64 the smaller tiles are ahead down to one CTA per SM
-    const long ctas = (long)((max_q_len + 128 / G - 1) / (128 / G)) * (a.Hq / G) * a.B;
+    // size 64 the smaller tiles are ahead down to one CTA per SM.  They are also ahead where a row sees few keys, so that half
+    // of a larger tile would lie behind the mask, and with a soft cap, whose tanh two CTAs overlap with the products (us, 128 /
+    // 64): 32 / 8 heads of 128, 130 tokens 7.9 / 7.2, 1024 tokens in a window of 128 18.8 / 11.8, 1024 tokens capped 54 / 49; 8 / 1
+    // heads of 64, 130 tokens 7.4 / 6.8; equal at 300 keys (10.3 / 10.4).
+    const long ctas = prefill_ctas(a, max_q_len), slots = (long)a.max_pages * a.page_size;
+    const bool small = a.softcap > 0.f || (a.window > 0 && a.window < slots ? a.window : slots) <= 256;
     switch (a.Dh) {
-    case 64: return ctas > sms ? launch<64, 64, 4>(a, G, max_q_len, q_rows, cache_rows, status, s) : launch<64, 128, 4>(a, G, max_q_len, q_rows, cache_rows, status, s);
-    case 128: return ctas > 2 * sms ? launch<128, 64, 2>(a, G, max_q_len, q_rows, cache_rows, status, s) : launch<128, 128, 2>(a, G, max_q_len, q_rows, cache_rows, status, s);
+    case 64: return small || ctas > sms ? launch<64, 64, 4>(a, G, max_q_len, q_rows, cache_rows, status, s) : launch<64, 128, 4>(a, G, max_q_len, q_rows, cache_rows, status, s);
+    case 128: return small || ctas > 2 * sms ? launch<128, 64, 2>(a, G, max_q_len, q_rows, cache_rows, status, s) : launch<128, 128, 2>(a, G, max_q_len, q_rows, cache_rows, status, s);
     default: return launch<256, 64, 2>(a, G, max_q_len, q_rows, cache_rows, status, s);
     }
 }

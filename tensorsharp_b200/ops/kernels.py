@@ -625,7 +625,7 @@ def attn_prefill(q, k_cache, v_cache, block_table, kv_lens, cu_q, max_q_len, *, 
     a.q_pos0 = q_pos0.data_ptr() if q_pos0 is not None else None
     a.lse_out = lse_out.data_ptr() if lse_out is not None else None
     lib = _lib()
-    if (_prefill_tc and lib.tsb_attn_prefill_tc_takes(C.byref(a), C.c_long(k_cache.shape[0])) and q.is_contiguous()
+    if (_prefill_tc and lib.tsb_attn_prefill_tc_takes(C.byref(a), C.c_int(max_q_len), C.c_long(k_cache.shape[0])) and q.is_contiguous()
             and k_cache.is_contiguous() and v_cache.is_contiguous() and k_cache.shape[0] == v_cache.shape[0]):
         native.check(lib.tsb_attn_prefill_tc(C.byref(a), C.c_int(max_q_len), C.c_long(q.shape[0]), C.c_long(k_cache.shape[0]),
                                              _p(gemm_status(q.device)), _stream()), "attn_prefill_tc")

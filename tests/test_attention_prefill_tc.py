@@ -74,6 +74,14 @@ def test_forms(Hq, Hkv, Dh):
     _check(Hq, Hkv, Dh, [2300], [2300])                                  # more than one wave, two row tiles per CTA
 
 
+@pytest.mark.parametrize("Hq,Hkv,Dh", [(16, 2, 64), (8, 2, 128)])
+@pytest.mark.parametrize("qlens,lens,window,softcap", [([600], [700], 0, 20.0), ([256, 255, 3], [256, 256, 250], 0, 0.0), ([400, 257], [900, 257], 256, 0.0),
+                                                      ([400, 257], [900, 257], 257, 0.0), ([600, 9], [700, 9], 100, 20.0)])
+def test_both_sides_of_the_tile_rule(Hq, Hkv, Dh, qlens, lens, window, softcap):
+    # grids below one CTA per SM: 64-key tiles with a soft cap and where a row sees at most 256 keys, 128-key tiles otherwise
+    _check(Hq, Hkv, Dh, qlens, lens, window=window, softcap=softcap, gate=softcap > 0 and window > 0)
+
+
 @pytest.mark.parametrize("Hq,Hkv,Dh,ql,n,peak", [(32, 8, 128, 300, 2000, 3.0), (32, 8, 128, 1100, 1100, 6.0), (16, 2, 64, 1024, 1024, 4.0), (16, 2, 256, 200, 900, 3.0)])
 def test_as_exact_as_the_mma_kernel(Hq, Hkv, Dh, ql, n, peak):
     """Both kernels round each weight, taken relative to the running maximum, and the result to bf16 and keep the rest in f32, so

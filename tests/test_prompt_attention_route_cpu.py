@@ -9,13 +9,13 @@ from tensorsharp_b200.ops import native
 pytestmark = pytest.mark.skipif(not native.available(), reason="the kernel library is not built here")
 
 
-def takes(cache_rows=4096, **kw):
+def takes(cache_rows=4096, max_q=1000, **kw):
     a = K.AttnArgs()
     plain = dict(q=1 << 20, k_cache=2 << 20, v_cache=3 << 20, out=4 << 20, block_table=5 << 20, kv_lens=6 << 20, cu_q=7 << 20, scale=0.1, B=2, Hq=8,
                  Hkv=2, Dh=128, Dv=128, page_size=64, max_pages=40, splits=1)
     for k, v in {**plain, **kw}.items():
         setattr(a, k, v)
-    return bool(K._lib().tsb_attn_prefill_tc_takes(C.byref(a), C.c_long(cache_rows)))
+    return bool(K._lib().tsb_attn_prefill_tc_takes(C.byref(a), C.c_int(max_q), C.c_long(cache_rows)))
 
 
 @pytest.mark.parametrize("Dh", [64, 128, 256])
@@ -34,6 +34,16 @@ def test_every_pointer_on_sixteen_bytes(name, off):
                                 dict(kv_scale=256), dict(log_r1=64), dict(sig_bias=64)])
 def test_what_stays_with_the_other_kernels(kw):
     assert not takes(**kw)
+
+
+def test_smallest_prompts_and_small_capped_grids():
+    """The lines of the rule: 64 slots, 256 heads of all prompts together, 72 CTAs (at two heads a tile 64 tokens each)."""
+    tiny = dict(Dh=64, Dv=64, max_pages=1, max_q=40)
+    assert not takes(**tiny) and takes(**{**tiny, "max_pages": 2}) and takes(**{**tiny, "B": 32}) and not takes(**{**tiny, "B": 31})
+    assert not takes(**{**tiny, "B": 32, "Hkv": 8}) and takes(**{**tiny, "Dh": 128, "Dv": 128}) and takes(**{**tiny, "Dh": 256, "Dv": 256})
+    cap = dict(Dh=64, Dv=64, softcap=30.0, Hq=4, Hkv=2, B=1)
+    assert not takes(max_q=35 * 64, **cap) and takes(max_q=35 * 64 + 1, **cap) and takes(max_q=64, **{**cap, "softcap": 0.0})
+    assert not takes(Dh=128, softcap=30.0, max_pages=1) and takes(Dh=128, softcap=30.0, max_pages=2)
 
 
 def test_a_whole_library_without_the_kernel_is_refused(monkeypatch):
