@@ -127,8 +127,9 @@ extern "C" int tsb_causal_conv1d(const ConvArgs* args, int max_q, void* stream) 
     TSB_CHECK_ARG(a.K >= 1 && a.K <= 9, "conv1d: kernel size %d out of range (1..9)", a.K);
     if (a.B == 0 || max_q == 0) return TSB_OK;
     cudaStream_t s = (cudaStream_t)stream;
-    // prompts whose rows can be read in 16-byte pieces; single tokens and other tap counts take the general kernel
-    const bool vec = a.K == 4 && max_q >= 16 && a.C % 4 == 0 && a.xs % 4 == 0 && a.os % 4 == 0 && a.B <= 65535 &&
+    // prompts whose rows can be read in 16-byte pieces; single tokens and other tap counts take the general kernel, and so does a
+    // prompt beyond the 65535 token groups of gridDim.y
+    const bool vec = a.K == 4 && max_q >= 16 && a.C % 4 == 0 && a.xs % 4 == 0 && a.os % 4 == 0 && a.B <= 65535 && (max_q + 7) / 8 <= 65535 &&
                      ((reinterpret_cast<uintptr_t>(a.x) | reinterpret_cast<uintptr_t>(a.out)) & 15) == 0;
     const long per = (long)max_q * a.C;
     if (vec) {

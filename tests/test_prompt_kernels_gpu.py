@@ -191,6 +191,17 @@ def test_conv_over_prompts(C, f32):
     assert rel(got, torch.cat(want)) < 1e-5 and torch.equal(state, tail)
 
 
+@pytest.mark.parametrize("n", [65535 * 8, 65535 * 8 + 1])
+def test_conv_over_the_longest_prompts(n):
+    """Either side of the 65535 groups of eight tokens that a grid dimension takes."""
+    torch.manual_seed(9)
+    cu = torch.tensor([0, n], dtype=torch.int32, device=DEV)
+    x, w, state = torch.randn(n, 4, device=DEV), torch.randn(4, 4, device=DEV), torch.randn(1, 3, 4, device=DEV)
+    want, tail = (t.to(DEV) for t in ref.causal_conv1d(x.cpu(), w.cpu(), None, state[0].cpu(), True))
+    got = K().causal_conv1d(x, w, None, state, cu, torch.zeros(1, dtype=torch.int64, device=DEV), n)
+    assert rel(got, want) < 1e-5 and torch.equal(state[0], tail)
+
+
 @pytest.mark.parametrize("D", [32, 2048, 5376, 8192])
 @pytest.mark.parametrize("rows", [1, 16, 300])
 def test_rms_seam(D, rows):
