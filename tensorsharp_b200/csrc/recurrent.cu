@@ -127,11 +127,14 @@ extern "C" int tsb_causal_conv1d(const ConvArgs* args, int max_q, void* stream) 
     TSB_CHECK_ARG(a.K >= 1 && a.K <= 9, "conv1d: kernel size %d out of range (1..9)", a.K);
     if (a.B == 0 || max_q == 0) return TSB_OK;
     cudaStream_t s = (cudaStream_t)stream;
-    // prompts whose rows can be read in 16-byte pieces; single tokens and other tap counts take the general kernel, and so does a
-    // prompt beyond the 65535 token groups of gridDim.y
-    const bool vec = a.K == 4 && max_q >= 16 && a.C % 4 == 0 && a.xs % 4 == 0 && a.os % 4 == 0 && a.B <= 65535 && (max_q + 7) / 8 <= 65535 &&
-                     ((reinterpret_cast<uintptr_t>(a.x) | reinterpret_cast<uintptr_t>(a.out)) & 15) == 0;
     const long per = (long)max_q * a.C;
+    // Prompts whose rows can be read in 16-byte pieces, from 352 K outputs (counted over the longest prompt of each sequence, as the
+    // general kernel's grid is) on: below, that kernel's short chains end sooner than the loads, taps and eight tokens of a thread
+    // here.  Measured (us, f32 and bf16 input; general kernel / here): 131 K outputs 4.7 / 6.2 and 6.5, 262 K 5.5 / 6.1 and 6.5, 328 K
+    // 6.4 / 6.2 and 6.5, 410 K 6.9 / 6.2 and 6.5, 524 K 7.7 / 6.4 and 6.7.  Other tap counts take the general kernel, and so does a
+    // prompt beyond the 65535 token groups of gridDim.y.
+    const bool vec = a.K == 4 && max_q >= 16 && per * a.B >= (352 << 10) && a.C % 4 == 0 && a.xs % 4 == 0 && a.os % 4 == 0 && a.B <= 65535 &&
+                     (max_q + 7) / 8 <= 65535 && ((reinterpret_cast<uintptr_t>(a.x) | reinterpret_cast<uintptr_t>(a.out)) & 15) == 0;
     if (vec) {
         const dim3 g((unsigned)((a.C / 4 + 127) / 128), (unsigned)((max_q + 7) / 8), (unsigned)a.B);
         TSB_CHECK_CUDA(a.x_f32 ? tsb_launch(conv1d_vec_kernel<4, true, 8>, g, dim3(128), 0, s, a) : tsb_launch(conv1d_vec_kernel<4, false, 8>, g, dim3(128), 0, s, a));

@@ -173,7 +173,7 @@ def test_rope_rows(Hq, Hkv, Dh, rot, T, f32):
         assert rel(got, want) < 3e-3
 
 
-@pytest.mark.parametrize("C", [4, 132, 1024])
+@pytest.mark.parametrize("C", [4, 132, 1024, 1124, 1128, 2052])           # five prompts of at most 64 tokens: from 1128 channels on the kernel for prompts
 @pytest.mark.parametrize("f32", [False, True])
 def test_conv_over_prompts(C, f32):
     torch.manual_seed(7)
