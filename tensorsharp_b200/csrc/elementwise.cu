@@ -626,6 +626,19 @@ static bool qkv_rope_vec_ok(const QkvArgs& a) {
     return true;
 }
 
+// Whether it is the faster one.  While all warps of the kernel above fit on the GPU at once it ends after one row's chain of
+// latencies; a thread here has up to four rows in turn.  So the lines lie by the rows of a thread and the head size.  Measured
+// (us, above / here, tokens x (query heads + 2 x KV heads) of the head size): four rows: 100 x 80 of 64 5.1 / 6.2, 170 x 80 6.9 / 6.3, 64 x 48
+// of 128 3.8 / 5.8, 130 x 48 5.5 / 6.0, 170 x 48 6.5 / 6.1, 130 x 20 of 256 4.3 / 5.3, 170 x 20 5.6 / 5.4; two rows: 170 x 18 of 64 3.1 / 3.3, 300 x
+// 18 4.8 / 3.4, 300 x 10 of 128 3.7 / 4.1, 400 x 10 5.3 / 4.2, 64 x 6 of 256 4.1 / 3.5; one row: 64 x 10 of 64 2.9 / 2.9, 64 x 6 of 128 3.2 / 2.9.
+static bool qkv_rope_vec_pays(const QkvArgs& a) {
+    const int H = a.Hq + 2 * a.Hkv, lanes = H * (a.Dh / 8);               // lanes of a token; 128 in a pass over the block
+    const long values = (long)a.T * H * a.Dh;
+    if (lanes > 256) return values >= (a.Dh == 256 ? 690000 : 850000);
+    if (a.Dh == 64) return values >= 288000;
+    return a.Dh == 256 || lanes <= 128 || values >= 400000;
+}
+
 extern "C" int tsb_qkv_rope(const QkvArgs* args, void* stream) {
     const QkvArgs& a = *args;
     TSB_CHECK_ARG(a.Dh > 0 && a.Dh <= 512, "qkv_rope: head dim %d out of range (1..512)", a.Dh);
@@ -636,8 +649,7 @@ extern "C" int tsb_qkv_rope(const QkvArgs* args, void* stream) {
     const long warps = (long)a.T * (a.Hq + 2 * a.Hkv);
     if (warps == 0) return TSB_OK;
     cudaStream_t st = (cudaStream_t)stream;
-    // (a decode batch is a few microseconds of latency either way, the kernel above spreads a token's heads over more blocks)
-    if (a.T >= 64 && qkv_rope_vec_ok(a)) {
+    if (a.T >= 64 && qkv_rope_vec_ok(a) && qkv_rope_vec_pays(a)) {
         const int rows = 4 * 128 / (a.Dh / 8);                         // of a block: four passes over its threads
         const dim3 g((unsigned)a.T, (unsigned)((a.Hq + 2 * a.Hkv + rows - 1) / rows)), b(128);
         if (a.Dh == 64) TSB_CHECK_CUDA(a.in_f32 ? tsb_launch(qkv_rope_vec_kernel<8, true>, g, b, 0, st, a) : tsb_launch(qkv_rope_vec_kernel<8, false>, g, b, 0, st, a));

@@ -147,8 +147,8 @@ def test_moe_tile_height_is_checked():
     assert call(8) == 0 and call(16) != 0 and call(0) != 0
 
 
-@pytest.mark.parametrize("Hq,Hkv,Dh,rot", [(8, 2, 64, 64), (5, 1, 128, 128), (4, 2, 256, 64), (3, 3, 128, 32), (16, 8, 128, 0)])
-@pytest.mark.parametrize("T", [64, 65, 700])
+@pytest.mark.parametrize("Hq,Hkv,Dh,rot", [(8, 2, 64, 64), (5, 1, 128, 128), (4, 2, 256, 64), (3, 3, 128, 32), (16, 8, 128, 0), (14, 2, 256, 128)])
+@pytest.mark.parametrize("T", [64, 65, 374, 375, 700])             # 374 / 375: either side of the line of the first heads
 @pytest.mark.parametrize("f32", [False, True])
 def test_rope_rows(Hq, Hkv, Dh, rot, T, f32):
     from tensorsharp_b200.ops import functional as F
