@@ -287,7 +287,7 @@ __device__ __forceinline__ void comp_q4_32(const QW& w, const WQ432& t, int u, c
 // Q8_0 planes, the gate and up rows of a pair, in groups of U half blocks per lane, all of a group's loads issued before any is
 // used (the first group's before `pre`).  A lane takes 16 codes: neighbouring lanes read neighbouring 16 bytes, so a request covers
 // whole sectors.  (With 32 codes a lane, as two 16-byte loads 32 bytes apart, every sector came from L2 twice: 60 us for the
-// 43008 x 5376 pair of a single-token step, 4.1 TB/s; in this form 49 us.  Single rows lose with eight loads ahead what they gain, 17.5
+// 43008 x 5376 pair of a single-token step, 4.1 TB/s; in this form 43 us.  Single rows lose with eight loads ahead what they gain, 17.5
 // against 22 us on average over a Gemma-31B layer's other products, and keep the two-deep loop of whole blocks.)
 template <int M, class Pre>
 __device__ __forceinline__ void dot_q8_pair(const QW& w, const long (&rows)[2], int lane, const int8_t* xq, const float2* xds, float* const (&acc)[2],
@@ -311,6 +311,32 @@ __device__ __forceinline__ void dot_q8_pair(const QW& w, const long (&rows)[2], 
     pre();
     for (; u0 < units; u0 += U * step) {
         if (u0 != lane) fetch(u0);
+        if (M <= 2) {
+            // the group's activations, too, all requested before any is used; units past the end count zero
+#pragma unroll
+            for (int m = 0; m < M; ++m) {
+                const int mr = m < mv ? m : 0;
+                int4 x[U];
+                float xd[U];
+#pragma unroll
+                for (int i = 0; i < U; ++i) {
+                    const int u = min(u0 + i * step, units - 1);
+                    x[i] = *reinterpret_cast<const int4*>(xq + (long)mr * K + u * 16);
+                    xd[i] = u0 + i * step < units ? xds[(long)mr * kb + (u >> 1)].x : 0.f;
+                }
+#pragma unroll
+                for (int i = 0; i < U; ++i)
+#pragma unroll
+                    for (int r = 0; r < R; ++r) {
+                        int s = __dp4a((int)q[r][i].x, x[i].x, 0);
+                        s = __dp4a((int)q[r][i].y, x[i].y, s);
+                        s = __dp4a((int)q[r][i].z, x[i].z, s);
+                        s = __dp4a((int)q[r][i].w, x[i].w, s);
+                        acc[r][m] += d[r][i] * xd[i] * (float)s;
+                    }
+            }
+            continue;
+        }
 #pragma unroll
         for (int i = 0; i < U; ++i) {
             const int u = u0 + i * step;
@@ -474,12 +500,17 @@ __device__ __forceinline__ void dot_row2(const QW& w, long row_a, long row_b, in
     case TSB_Q4_K: TSB_ROW_LOOP2(WQ4K, load_q45k<false>, (comp_q45k<M, false>), (w.K >> 8) << 3) break;
     case TSB_Q5_K: TSB_ROW_LOOP2(WQ4K, load_q45k<true>, (comp_q45k<M, true>), (w.K >> 8) << 3) break;
     case TSB_Q6_K: TSB_ROW_LOOP2(WQ6K, load_q6k, comp_q6k<M>, (w.K >> 8) << 2) break;
-    case TSB_Q8_0: {
-        const long rows[2] = {row_a, row_b};
-        float* const a[2] = {acc_a, acc_b};
-        dot_q8_pair<M>(w, rows, lane, xq, xds, a, mv, pre);
+    case TSB_Q8_0:
+        // Groups of four half blocks a lane, unless a row is half a group or less, or three or four activation rows share a matrix
+        // whose rows are soon dealt out, where the shorter chain of the two-deep loop ends first.  Measured (us, two-deep loop / here), one
+        // row: 8192 x 1024 4.1 / 4.3, 13824 x 1152 7.3 / 6.5, 1024 x 2048 2.3 / 2.2, 43008 x 5376 58.5 / 43.3; two rows: 8192 x 1024 6.0 / 6.5, 8192 x 2048
+        // 7.3 / 6.5, 43008 x 5376 74 / 58; three rows: 8192 x 1024 7.7 / 8.2, 4096 x 4096 9.3 / 9.8, 13824 x 1152 12.8 / 11.9, 43008 x 5376 87 / 74.
+        if (w.K > 1024 && (M <= 2 || w.N > 8192)) {
+            const long rows[2] = {row_a, row_b};
+            float* const a[2] = {acc_a, acc_b};
+            dot_q8_pair<M>(w, rows, lane, xq, xds, a, mv, pre);
+        } else TSB_ROW_LOOP2(WQ80, load_q8_0, comp_q8_0<M>, w.K >> 5)
         break;
-    }
     case TSB_MXFP4: TSB_ROW_LOOP2(WQ432, load_q4_32<true>, (comp_q4_32<M, true>), w.K >> 5) break;
     case TSB_Q4_0: TSB_ROW_LOOP2(WQ432, load_q4_32<false>, (comp_q4_32<M, false>), w.K >> 5) break;
     case TSB_BF16: {

@@ -214,3 +214,16 @@ def test_rms_seam(D, rows):
     assert rel(a, ref.rmsnorm(want.float(), pre, 1e-6)) < 3e-3
     wq, wds = K().quantize_q8(ref.rmsnorm(want.float(), pre, 1e-6).contiguous())
     assert (q.int() - wq.int()).abs().max() <= 1 and rel(ds[..., 0], wds[..., 0]) < 1e-5
+
+
+# either side of the lines of the Q8_0 pair loop (K 1024, and 8192 rows for several activation rows), K with a group that ends early
+@pytest.mark.parametrize("N,Kd", [(8192, 1024), (8192, 1056), (8196, 1056), (8196, 2080), (6, 1056), (6, 32)])
+@pytest.mark.parametrize("M", [1, 2, 3, 4])
+def test_q8_pairs(N, Kd, M):
+    torch.manual_seed(10)
+    w = QuantWeight.from_float(torch.randn(N, Kd, device=DEV) * 0.1, GGMLType.Q8_0)
+    xq, xds = K().quantize_q8(torch.randn(M, Kd, device=DEV))
+    got = K().gemv(w, xq=xq, xds=xds, M=M, act="swiglu")
+    y = (xq.view(M, -1, 32).double() * xds[..., :1].double()).view(M, Kd) @ w.dequantize().double().t()
+    # whole-number products of blocks, scaled and added in f32
+    assert rel(got, torch.nn.functional.silu(y[:, :N // 2]) * y[:, N // 2:]) < 1e-5
