@@ -828,8 +828,119 @@ __global__ void __launch_bounds__(128) gemv_tiles_mma_kernel(TileArgs a) {
     }
 }
 
-// The same tile GEMV with the weights on their way through shared memory, for tiles of up to 16 rows.  The kernel above has about
-// 1 KB of weights in flight per warp and stops for each of them; here every warp keeps STG stages of its own 16 (gated: 32)
+// The same tile GEMV with 8-byte weight loads.  In the kernel above a lane reads 4 bytes per block and row, so a warp
+// has about 1 KB of weights in flight and every request uses half a sector; at four CTAs per SM that is a third of the
+// bytes in flight the memory system needs.  Here lane t of a row's four lanes reads half (t & 1) of block ub + (t >> 1):
+// one request covers two whole blocks (a full sector), twice the bytes in flight for the same registers, and the word a
+// lane needs for a block's MMA fragment (word t) comes from lane 2q + (t >> 1) by shuffle.  The scales of a block pair
+// are one 2-byte (MXFP4) or 4-byte (Q4_0) load.  Needs an even number of blocks per row.  Serves what the ring kernel below
+// does not (moe_ring_pays).
+template <bool GLU, bool MX>
+__global__ void __launch_bounds__(128) gemv_tiles_mma_wide_kernel(TileArgs a) {
+    constexpr int S = GLU ? 2 : 1;
+    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const int r0 = (blockIdx.x * 4 + (threadIdx.x >> 5)) * 16;
+    pdl_wait();
+    pdl_trigger();
+    if ((int)blockIdx.y >= a.meta[0] || r0 >= a.n_out) return;
+    const int4 tile = a.tiles[blockIdx.y];
+    const int expert = tile.x, row0 = tile.y, mv = tile.z;
+    const int K = a.w.K, kb = K >> 5;
+    long wr[S][2];
+#pragma unroll
+    for (int s = 0; s < S; ++s) {
+        wr[s][0] = (long)expert * a.w.N + s * a.n_out + min(r0 + g, a.n_out - 1);
+        wr[s][1] = (long)expert * a.w.N + s * a.n_out + min(r0 + g + 8, a.n_out - 1);
+    }
+    const bool bact = g < mv;
+    const int8_t* xrow = a.xq + (long)(row0 + (bact ? g : 0)) * K + 4 * t;
+    const int c0 = 2 * t, c1 = 2 * t + 1;
+    const float2* xs0 = a.xds + (long)(row0 + (c0 < mv ? c0 : 0)) * kb;
+    const float2* xs1 = a.xds + (long)(row0 + (c1 < mv ? c1 : 0)) * kb;
+    const int src_base = lane & ~3;
+    float acc[S][4];
+#pragma unroll
+    for (int s = 0; s < S; ++s)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc[s][i] = 0.f;
+    for (int u0 = 0; u0 < kb; u0 += 4) {
+        uint2 wv[2][S][2];
+        uint32_t sc[2][S][2];
+        int b0[4], b1[4];
+        float xd0[4], xd1[4];
+#pragma unroll
+        for (int P = 0; P < 2; ++P) {
+            const int ub = min(u0 + 2 * P, kb - 2);                 // (a pair past the end re-reads the last one; not used)
+#pragma unroll
+            for (int s = 0; s < S; ++s)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    wv[P][s][h] = __ldg(reinterpret_cast<const uint2*>(a.w.p0 + wr[s][h] * (K >> 1) + (ub + (t >> 1)) * 16 + (t & 1) * 8));
+                    if (MX) sc[P][s][h] = __ldg(reinterpret_cast<const unsigned short*>(a.w.p1 + wr[s][h] * kb + ub));
+                    else sc[P][s][h] = __ldg(reinterpret_cast<const uint32_t*>(a.w.p1 + 2 * (wr[s][h] * kb + ub)));
+                }
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int u = min(u0 + j, kb - 1);
+            b0[j] = bact ? *reinterpret_cast<const int*>(xrow + u * 32) : 0;
+            b1[j] = bact ? *reinterpret_cast<const int*>(xrow + u * 32 + 16) : 0;
+            xd0[j] = xs0[u].x;
+            xd1[j] = xs1[u].x;
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int P = j >> 1, q = j & 1;
+            const bool live = u0 + j < kb;                          // uniform over the warp
+            const int src = src_base | (2 * q + (t >> 1));
+#pragma unroll
+            for (int s = 0; s < S; ++s) {
+                uint32_t wd[2];
+                float ws[2];
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const uint32_t x = __shfl_sync(0xffffffffu, wv[P][s][h].x, src), y = __shfl_sync(0xffffffffu, wv[P][s][h].y, src);
+                    wd[h] = (t & 1) ? y : x;
+                    if (MX) ws[h] = e8m0_half_scale((uint8_t)(sc[P][s][h] >> (8 * q)));
+                    else ws[h] = __half2float(__ushort_as_half((unsigned short)(sc[P][s][h] >> (16 * q))));
+                }
+                if (live) {
+                    int af[4], c[4] = {0, 0, 0, 0};
+                    decode_q4_words<MX>(wd[0], wd[1], af);
+                    mma_s8_16x8x32(c, af, b0[j], b1[j]);
+                    acc[s][0] += ws[0] * xd0[j] * (float)c[0];
+                    acc[s][1] += ws[0] * xd1[j] * (float)c[1];
+                    acc[s][2] += ws[1] * xd0[j] * (float)c[2];
+                    acc[s][3] += ws[1] * xd1[j] * (float)c[3];
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int r = r0 + g + (i >> 1) * 8, col = 2 * t + (i & 1);
+        if (r >= a.n_out || col >= mv) continue;
+        float v = acc[0][i];
+        if (a.bias) v += a.bias[(long)expert * a.w.N + r];
+        if (GLU) {
+            float up = acc[S - 1][i];
+            if (a.bias) up += a.bias[(long)expert * a.w.N + r + a.n_out];
+            v = act_glu(a.act, v, up);
+        } else if (a.act == ACT_RELU2) {
+            v = fmaxf(v, 0.f);
+            v = v * v;
+        } else if (a.act == ACT_SILU) {
+            v = v / (1.f + __expf(-v));
+        }
+        if (a.row_scale) v *= a.row_scale[row0 + col];
+        const long o = (long)(row0 + col) * a.n_out + r;
+        if (a.out_f32) reinterpret_cast<float*>(a.out)[o] = v;
+        else reinterpret_cast<bf16*>(a.out)[o] = f2bf(v);
+    }
+}
+
+// The same tile GEMV with the weights on their way through shared memory, for tiles of up to 16 rows.  The kernels above have 1 to
+// 2 KB of weights in flight per warp and stop for each of them; here every warp keeps STG stages of its own 16 (gated: 32)
 // weight rows x 64 bytes in flight with cp.async, two sets of four warps take a half of K each, the tile's activations and the rows' scales are staged once, and a weight
 // word is decoded once for up to 16 rows, so an expert with 9 to 16 pairs no longer streams its matrix twice.
 // The 16-byte block of a row's stage sits at place (block ^ (row / 2 & 3)), so that the eight rows of a fragment load differ in
@@ -1003,23 +1114,38 @@ static bool moe_mma_on() {
     return on;
 }
 
-// Whether the ring kernel takes a projection: 4-bit blocks of 32 with their scales in a plane whose 64-row pieces start on 16
-// bytes, and a K whose activations fit beside the ring.  Both the height of the tiles and the kernel that serves them follow from
-// this one answer.
-static bool moe_ring_ok(int type, int N, int K, bool glu) {
-    if (!moe_mma_on() || (type != TSB_MXFP4 && type != TSB_Q4_0) || K % 32 != 0 || N <= 0) return false;
-    const bool mx = type == TSB_MXFP4;
-    const long n_out = glu ? N / 2 : N, sb = mx ? 1 : 2;
-    if ((n_out * (K / 32) * sb) % 16 != 0) return false;
-    const size_t smem = glu ? (mx ? RingSmem<true, true>::total(K) : RingSmem<true, false>::total(K))
-                            : (mx ? RingSmem<false, true>::total(K) : RingSmem<false, false>::total(K));
-    return smem <= 226 * 1024;
+static size_t moe_ring_smem(int type, int K, bool glu) {
+    if (type == TSB_MXFP4) return glu ? RingSmem<true, true>::total(K) : RingSmem<false, true>::total(K);
+    return glu ? RingSmem<true, false>::total(K) : RingSmem<false, false>::total(K);
 }
 
-// Most rows of a tile that both projections of a layer take (see tsb_moe_group_rows).
-extern "C" int tsb_moe_tile_rows(int up_type, int up_N, int up_K, int act, int down_type, int down_N, int down_K) {
+// Whether the ring kernel takes a projection: 4-bit blocks of 32 with their scales in a plane whose 64-row pieces start on 16
+// bytes, and a K whose activations fit beside the ring.
+static bool moe_ring_ok(int type, int N, int K, bool glu) {
+    if (!moe_mma_on() || (type != TSB_MXFP4 && type != TSB_Q4_0) || K % 32 != 0 || N <= 0) return false;
+    const long n_out = glu ? N / 2 : N, sb = type == TSB_MXFP4 ? 1 : 2;
+    return (n_out * (K / 32) * sb) % 16 == 0 && moe_ring_smem(type, K, glu) <= 226 * 1024;
+}
+static bool moe_ring_twice(int type, int K, bool glu) { return moe_ring_smem(type, K, glu) <= 113 * 1024; }
+
+// Whether it is the faster one for tiles of at most `tile_rows`: with two CTAs on an SM always; with one (eight warps, too few to
+// decode the words as fast as they arrive) only where its tiles of sixteen spare half of the passes over the weights.
+static bool moe_ring_pays(int type, int N, int K, bool glu, int tile_rows) {
+    return moe_ring_ok(type, N, K, glu) && (tile_rows > MOE_TILE_ROWS || moe_ring_twice(type, K, glu));
+}
+
+// Most rows of a tile of a layer (see tsb_moe_group_rows): sixteen where the ring kernel takes both projections and either has them
+// twice on an SM or P pairs make eight for every one of the E experts; else each projection takes its better kernel for eight.
+// Measured, a layer of P pairs, us (both projections: 8-byte loads / ring, tiles of sixteen / each its better one, tiles of eight):
+// MXFP4, 32 experts of 3072 x 3072: 128 pairs 267 / 321 / 261, 192 pairs 305 / 335 / 302, 256 pairs 361 / 348 / 350, 512 pairs 575 / 510 / 569;
+// 128 of 4096 x 1536: 512 pairs 661 / 771 / 645, 1024 pairs 928 / 856 / 905; 8 of 4096 x 14336 (down beyond the ring's K): 128 pairs
+// 1003 / - / 1003.  Q4_0, 32 of 2880 x 2880: 128 pairs 187 / 240 / 185, 256 pairs 242 / 270 / 237, 512 pairs 389 / 381 / 393; 16 of 12288 x 1024 (gate
+// and up beyond it): 128 pairs 282 / - / 267.  Twice on an SM: MXFP4, 32 of 2880 x 2880, 128 pairs 239 / 228, 512 pairs 505 / 360.
+extern "C" int tsb_moe_tile_rows(int up_type, int up_N, int up_K, int act, int down_type, int down_N, int down_K, int P, int E) {
     const bool glu = act >= ACT_SWIGLU && act <= ACT_SWIGLU_OAI;
-    return moe_ring_ok(up_type, up_N, up_K, glu) && moe_ring_ok(down_type, down_N, down_K, false) ? MOE_RING_ROWS : MOE_TILE_ROWS;
+    if (!moe_ring_ok(up_type, up_N, up_K, glu) || !moe_ring_ok(down_type, down_N, down_K, false)) return MOE_TILE_ROWS;
+    const bool twice = moe_ring_twice(up_type, up_K, glu) && moe_ring_twice(down_type, down_K, false);
+    return twice || P >= 8L * E ? MOE_RING_ROWS : MOE_TILE_ROWS;
 }
 
 template <bool GLU, bool MX>
@@ -1049,7 +1175,7 @@ extern "C" int tsb_moe_gemv_tiles(const void* p0, const void* p1, const void* p2
     const bool glu = act >= ACT_SWIGLU && act <= ACT_SWIGLU_OAI;
     TSB_CHECK_ARG(!glu || N % 2 == 0, "moe_gemv_tiles: GLU needs an even row count, got %d", N);
     TSB_CHECK_ARG(max_tiles <= 65535, "moe_gemv_tiles: %d tiles exceed the grid limit", max_tiles);
-    const bool ring = moe_ring_ok(type, N, K, glu);
+    const bool ring = moe_ring_pays(type, N, K, glu, tile_rows);
     TSB_CHECK_ARG(tile_rows > 0 && tile_rows <= (ring ? MOE_RING_ROWS : MOE_TILE_ROWS), "moe_gemv_tiles: tiles of %d rows of weight type %d, K=%d",
                   tile_rows, type, K);
     if (max_tiles == 0) return TSB_OK;
@@ -1064,6 +1190,17 @@ extern "C" int tsb_moe_gemv_tiles(const void* p0, const void* p1, const void* p2
         if (ring) {
             if (type == TSB_MXFP4) return glu ? launch_ring<true, true>(a, max_tiles, st) : launch_ring<false, true>(a, max_tiles, st);
             return glu ? launch_ring<true, false>(a, max_tiles, st) : launch_ring<false, false>(a, max_tiles, st);
+        }
+        if ((K >> 5) % 2 == 0) {
+            if (type == TSB_MXFP4) {
+                if (glu) TSB_CHECK_CUDA(tsb_launch(gemv_tiles_mma_wide_kernel<true, true>, grid, block, 0, st, a));
+                else TSB_CHECK_CUDA(tsb_launch(gemv_tiles_mma_wide_kernel<false, true>, grid, block, 0, st, a));
+            } else {
+                if (glu) TSB_CHECK_CUDA(tsb_launch(gemv_tiles_mma_wide_kernel<true, false>, grid, block, 0, st, a));
+                else TSB_CHECK_CUDA(tsb_launch(gemv_tiles_mma_wide_kernel<false, false>, grid, block, 0, st, a));
+            }
+            TSB_CHECK_LAUNCH();
+            return TSB_OK;
         }
         if (type == TSB_MXFP4) {
             if (glu) TSB_CHECK_CUDA(tsb_launch(gemv_tiles_mma_kernel<true, true>, grid, block, 0, st, a));

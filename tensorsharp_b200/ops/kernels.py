@@ -249,7 +249,7 @@ def moe_grouped(*, xq=None, xds=None, xb=None, ids: torch.Tensor, weights: torch
     ids = ids.contiguous()
     pos = torch.empty((P,), dtype=torch.int32, device=dev)
     rows = int(lib.tsb_moe_tile_rows(C.c_int(int(gate_up.ggml_type)), C.c_int(gate_up.N), C.c_int(K), C.c_int(a), C.c_int(int(down.ggml_type)),
-                                     C.c_int(D), C.c_int(F_out)))
+                                     C.c_int(D), C.c_int(F_out), C.c_int(P), C.c_int(E_local)))
     max_tiles = int(lib.tsb_moe_max_tiles_rows(C.c_int(P), C.c_int(E_local), C.c_int(rows)))
     tiles = torch.empty((max_tiles, 4), dtype=torch.int32, device=dev)
     meta = torch.empty((2,), dtype=torch.int32, device=dev)

@@ -103,7 +103,9 @@ def test_moe_spread_and_grouped(T, E, k, bn, e0):
 
 # tiles of 1 .. 16 pairs, rows that end inside a 64-row block, 9 blocks of K (one stage and a bit), both 4-bit types
 @pytest.mark.parametrize("t", [GGMLType.MXFP4, GGMLType.Q4_0])
-@pytest.mark.parametrize("T,k,E,Kd,Fd", [(40, 2, 3, 288, 160), (70, 1, 4, 2880, 96), (33, 4, 9, 64, 256)])
+@pytest.mark.parametrize("T,k,E,Kd,Fd", [(40, 2, 3, 288, 160), (70, 1, 4, 2880, 96), (33, 4, 9, 64, 256),
+                                           # gate and up once on an SM: 255 pairs tiles of eight, 256 pairs of sixteen; beyond the ring's K; an odd number of blocks there
+                                           (255, 1, 32, 4096, 64), (256, 1, 32, 4096, 64), (40, 2, 3, 12288, 64), (40, 2, 3, 12320, 32)])
 def test_moe_tiles_of_sixteen(t, T, k, E, Kd, Fd):
     torch.manual_seed(5)
     gu = QuantWeight.from_float(torch.randn(E, 2 * Fd, Kd, device=DEV) * 0.1, t)
