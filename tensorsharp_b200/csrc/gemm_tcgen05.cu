@@ -491,6 +491,14 @@ constexpr int PAIR_STAGE_BYTES = 2 * 128 * 128;                  // 128 features
 constexpr int PAIR_SMEM = PAIR_STAGES * PAIR_STAGE_BYTES + 256 + 1024;
 constexpr int PAIR_GLU_SMEM = 4 * 2 * 16 * 32 * 4;               // two chunks of 16 tokens for each of four pairs of epilogue warps
 
+// A barrier of the 64 threads that name `id`, which also tells each whether the predicate held for all of them.
+__device__ __forceinline__ bool bar_all64(int id, bool ok) {
+    uint32_t r;
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.and.pred q, %2, 64, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+                 : "=r"(r) : "r"((uint32_t)ok), "r"(id) : "memory");
+    return r != 0;
+}
+
 // GLU: the rows of a CTA's tile are 64 gate rows and the 64 up rows of the same features.  A warp that reads up values hands them
 // through shared memory to the one that reads the gates of the same features and tokens, so the gated activation leaves the kernel
 // and its two inputs, rounded to bf16 as a kernel of its own would have read them, never reach memory.
@@ -620,7 +628,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(320) gemm_bf16_pair_
             const int cols = min(bn, t_end - n0);                  // tokens of this tile that exist
             if (GLU) {
                 const int pr = turn * 2 + (q & 1);
-                if (!tc::warp_wait(&acc_full[buf], (j >> 1) & 1)) { atomicExch(status, 3); break; }
+                // Both warps of the pair go on, or both leave: one that gave up alone would leave the other at the barriers below.
+                // The barrier also says that the place where this tile starts, which the tile before may have read last, was read.
+                if (!bar_all64(pr + 1, tc::warp_wait(&acc_full[buf], (j >> 1) & 1))) { atomicExch(status, 3); break; }
                 tc::fence_after_sync();
                 int side = 0;
 #pragma unroll 1
@@ -646,8 +656,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(320) gemm_bf16_pair_
                     }
                 }
                 tc::fence_before_sync();
-                // the next tile starts with the place that this one may just have read
-                asm volatile("bar.sync %0, 64;" ::"r"(pr + 1) : "memory");
+                __syncwarp();
                 if (lane == 0) tc::mbar_arrive_cluster(tc::map_to_rank(&acc_empty[buf], 0));
                 ++j;
                 continue;

@@ -53,7 +53,7 @@ def test_gemm_pairs_launched_back_to_back():
 
 # each of gate and up is rounded to bf16 ahead of the activation and the result once more; swiglu's slope is at most about 1.1
 @pytest.mark.parametrize("act", ["swiglu", "geglu", "geglu_erf", "swiglu_oai"])
-@pytest.mark.parametrize("T,F,Kd", [(65, 40, 64), (300, 129, 200), (1000, 576, 512)])
+@pytest.mark.parametrize("T,F,Kd", [(65, 40, 64), (300, 129, 200), (1000, 576, 512), (2050, 4104, 72)])      # the last: several tiles a pair
 def test_gemm_glu(act, T, F, Kd):
     torch.manual_seed(3)
     W, X, b = (torch.randn(2 * F, Kd, device=DEV) * 0.1).bfloat16(), torch.randn(T, Kd, device=DEV).bfloat16(), torch.randn(2 * F, device=DEV)
