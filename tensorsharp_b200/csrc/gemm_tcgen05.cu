@@ -663,38 +663,46 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(320) gemm_bf16_pair_
             }
             // the residual does not depend on the products: a chunk's values are requested one chunk ahead, the first
             // one's before the wait for the accumulator
-            auto residual = [&](int c, float (&res)[16]) {
+            const long at = (long)n0 * ep.ldo + f;
+            float res[16], next[16];
 #pragma unroll
-                for (int i = 0; i < 16; ++i) {
-                    const int t = n0 + c * 16 + i;
-                    res[i] = 0.f;
-                    if (ep.residual != nullptr && mine && c * 16 < cols && t < t_end) {
-                        const long o = (long)t * ep.ldo + f;
-                        res[i] = ep.out_f32 ? reinterpret_cast<const float*>(ep.residual)[o] : bf2f(reinterpret_cast<const bf16*>(ep.residual)[o]);
-                    }
+            for (int i = 0; i < 16; ++i) res[i] = next[i] = 0.f;
+            auto residual = [&](int c, float (&v)[16]) {
+                const int left = cols - c * 16;
+                if (ep.residual == nullptr || !mine || left <= 0) return;
+                if (ep.out_f32) {
+                    const float* p = reinterpret_cast<const float*>(ep.residual) + at + (long)(c * 16) * ep.ldo;
+#pragma unroll
+                    for (int i = 0; i < 16; ++i, p += ep.ldo)
+                        if (i < left) v[i] = *p;
+                } else {
+                    const bf16* p = reinterpret_cast<const bf16*>(ep.residual) + at + (long)(c * 16) * ep.ldo;
+#pragma unroll
+                    for (int i = 0; i < 16; ++i, p += ep.ldo)
+                        if (i < left) v[i] = bf2f(*p);
                 }
             };
-            float res[16];
             residual(turn, res);
             if (!tc::warp_wait(&acc_full[buf], (j >> 1) & 1)) { atomicExch(status, 3); break; }
             tc::fence_after_sync();
 #pragma unroll 1
             for (int c = turn; c * 16 < cols; c += 2) {
-                float next[16];
                 residual(c + 2, next);
                 uint32_t r[16];
                 tc::tmem_ld16(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)buf * 256 + c * 16, r);
                 tc::tmem_ld_wait();
                 if (mine) {
+                    const int left = cols - c * 16;
+                    if (ep.out_f32) {
+                        float* p = reinterpret_cast<float*>(ep.out) + at + (long)(c * 16) * ep.ldo;
 #pragma unroll
-                    for (int i = 0; i < 16; ++i) {
-                        const int t = n0 + c * 16 + i;
-                        if (t < t_end) {
-                            const float v = __uint_as_float(r[i]) + bias + res[i];
-                            const long o = (long)t * ep.ldo + f;
-                            if (ep.out_f32) reinterpret_cast<float*>(ep.out)[o] = v;
-                            else reinterpret_cast<bf16*>(ep.out)[o] = f2bf(v);
-                        }
+                        for (int i = 0; i < 16; ++i, p += ep.ldo)
+                            if (i < left) *p = __uint_as_float(r[i]) + bias + res[i];
+                    } else {
+                        bf16* p = reinterpret_cast<bf16*>(ep.out) + at + (long)(c * 16) * ep.ldo;
+#pragma unroll
+                        for (int i = 0; i < 16; ++i, p += ep.ldo)
+                            if (i < left) *p = f2bf(__uint_as_float(r[i]) + bias + res[i]);
                     }
                 }
 #pragma unroll
