@@ -20,6 +20,7 @@
 #include <cudaTypedefs.h>
 #include <mutex>
 #include <cstdlib>
+#include <type_traits>
 #include "glu.cuh"
 #include "tcgen05.cuh"
 #include "tp_fused.cuh"
@@ -499,9 +500,10 @@ __device__ __forceinline__ bool bar_all64(int id, bool ok) {
     return r != 0;
 }
 
-// GLU: the rows of a CTA's tile are 64 gate rows and the 64 up rows of the same features.  A warp that reads up values hands them
-// through shared memory to the one that reads the gates of the same features and tokens, so the gated activation leaves the kernel
-// and its two inputs, rounded to bf16 as a kernel of its own would have read them, never reach memory.
+// GLU: the rows of a CTA's tile are 64 gate rows and the 64 up rows of the same features.  The warp that reads the gates of some
+// features and tokens and the one that reads their up values give one another half of a chunk through shared memory and form the
+// activation of eight tokens each, so the gated activation leaves the kernel and its two inputs, rounded to bf16 as a kernel of
+// its own would have read them, never reach memory.
 template <bool GLU>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(320) gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmW,
                                                                                        const __grid_constant__ CUtensorMap tmX, GemmEpi ep, int K,
@@ -632,28 +634,37 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(320) gemm_bf16_pair_
                 // The barrier also says that the place where this tile starts, which the tile before may have read last, was read.
                 if (!bar_all64(pr + 1, tc::warp_wait(&acc_full[buf], (j >> 1) & 1))) { atomicExch(status, 3); break; }
                 tc::fence_after_sync();
-                int side = 0;
+                auto chunks = [&](auto act) {
+                    int side = 0;
 #pragma unroll 1
-                for (int c = turn; c * 16 < cols; c += 2, side ^= 1) {
-                    uint32_t r[16];
-                    tc::tmem_ld16(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)buf * 256 + c * 16, r);
-                    tc::tmem_ld_wait();
-                    float* st = up_stage + (pr * 2 + side) * (16 * 32) + lane;
-                    if (q >= 2) {
+                    for (int c = turn; c * 16 < cols; c += 2, side ^= 1) {
+                        uint32_t r[16];
+                        tc::tmem_ld16(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)buf * 256 + c * 16, r);
+                        tc::tmem_ld_wait();
+                        float v[16];
 #pragma unroll
-                        for (int i = 0; i < 16; ++i) st[i * 32] = bf2f(f2bf(__uint_as_float(r[i]) + bias));
-                    }
-                    // both warps of the pair: the up values are there; and those of two chunks ago, in the same place, were read
-                    asm volatile("bar.sync %0, 64;" ::"r"(pr + 1) : "memory");
-                    if (q < 2 && mine) {
+                        for (int i = 0; i < 16; ++i) v[i] = bf2f(f2bf(__uint_as_float(r[i]) + bias));
+                        float* st = up_stage + (pr * 2 + side) * (16 * 32) + lane;
 #pragma unroll
-                        for (int i = 0; i < 16; ++i) {
-                            const int t = n0 + c * 16 + i;
-                            if (t < t_end)
-                                reinterpret_cast<bf16*>(ep.out)[(long)t * ep.ldo + f] =
-                                    f2bf(act_glu(ep.act, bf2f(f2bf(__uint_as_float(r[i]) + bias)), st[i * 32]));
+                        for (int i = 0; i < 8; ++i) st[q < 2 ? (i + 8) * 32 : i * 32] = q < 2 ? v[i + 8] : v[i];
+                        // both warps of the pair: the other half is there; and that of two chunks ago, in the same place, was read
+                        asm volatile("bar.sync %0, 64;" ::"r"(pr + 1) : "memory");
+                        const int left = cols - c * 16;
+                        bf16* p = reinterpret_cast<bf16*>(ep.out) + (long)(n0 + c * 16 + (q < 2 ? 0 : 8)) * ep.ldo + f;
+                        if (mine) {
+#pragma unroll
+                            for (int i = 0; i < 8; ++i, p += ep.ldo) {
+                                const float other = st[q < 2 ? i * 32 : (i + 8) * 32], g = q < 2 ? v[i] : other, u = q < 2 ? other : v[i + 8];
+                                if ((q < 2 ? i : i + 8) < left) *p = f2bf(act_glu(decltype(act)::value, g, u));
+                            }
                         }
                     }
+                };
+                switch (ep.act) {
+                case ACT_SWIGLU: chunks(std::integral_constant<int, ACT_SWIGLU>{}); break;
+                case ACT_GEGLU_TANH: chunks(std::integral_constant<int, ACT_GEGLU_TANH>{}); break;
+                case ACT_GEGLU_ERF: chunks(std::integral_constant<int, ACT_GEGLU_ERF>{}); break;
+                default: chunks(std::integral_constant<int, ACT_SWIGLU_OAI>{}); break;
                 }
                 tc::fence_before_sync();
                 __syncwarp();
