@@ -168,6 +168,7 @@ __global__ void __launch_bounds__(192, PrefillSmem<DH, BN, KS>::PER_SM) attn_pre
             const int* table = a.block_table + (long)b * a.max_pages;
             const int n_sub = (j_hi + 63) / 64;                                     // 64-slot runs that exist
             int base = -64, slot_of = 0;                                             // lane i: first slot of run base + i
+            int loaded[2] = {0, 0};                                                  // tiles of K and of V requested
             bool ok = true;
             // K runs one tile ahead of V: two score tiles are computed before the first PV
             for (int i = 0; i <= nt && ok; ++i) {
@@ -189,6 +190,8 @@ __global__ void __launch_bounds__(192, PrefillSmem<DH, BN, KS>::PER_SM) attn_pre
                     uint64_t* bar = kv ? &v_full[s] : &k_full[s];
                     unsigned char* dst = (kv ? sV : sK) + s * L::KV_BYTES;
                     if (lane == 0) mbar_expect_tx(bar, valid * CH * 8192);
+                    if (kv) loaded[1] = t + 1;
+                    else loaded[0] = t + 1;
 #pragma unroll
                     for (int r = 0; r < SUB; ++r) {
                         const int row = __shfl_sync(0xffffffffu, slot_of, run + r - base);
@@ -197,9 +200,12 @@ __global__ void __launch_bounds__(192, PrefillSmem<DH, BN, KS>::PER_SM) attn_pre
                     }
                 }
             }
-            if (!ok && lane == 0) {
-                // give up only with no copy in flight: wait for whatever was issued and not consumed
+            // The CTA leaves with no copy in flight, whichever warp gave up: the last tile of every stage has arrived (where nothing
+            // went wrong the products read it already).
+            if (lane == 0) {
                 mbar_wait(q_full, 0);
+                for (int t = max(0, loaded[0] - KS); t < loaded[0]; ++t) mbar_wait(&k_full[t % KS], (t / KS) & 1);
+                for (int t = max(0, loaded[1] - KS); t < loaded[1]; ++t) mbar_wait(&v_full[t % KS], (t / KS) & 1);
             }
         }
         __syncwarp();

@@ -579,6 +579,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(320) gemm_bf16_pair_
                     tc::tma_load_2d_pair(a + 128 * 128, &tmX, bar, kb * 64, n0 + rank * (int)half);
                 }
             }
+            // The pair leaves with no copy in flight, whichever wait gave up: the last slab of every stage, of both CTAs, has arrived.
+            if (rank == 0)
+                for (int i = max(0, it - PAIR_STAGES); i < it; ++i) tc::mbar_wait(&full_bar[i % PAIR_STAGES], (i / PAIR_STAGES) & 1);
         }
         __syncwarp();
     } else if (warp == 1) {
