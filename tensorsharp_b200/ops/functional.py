@@ -148,7 +148,8 @@ def norm_add(x: torch.Tensor, w: Optional[torch.Tensor], eps: float, h: torch.Te
 def norm_add_norm(x: torch.Tensor, post: torch.Tensor, h: torch.Tensor, pre: torch.Tensor, eps: float, *, want_q8: bool = False):
     """:func:`norm_add` and the :func:`norm` of the next block: (h + RMSNorm(x) * post, RMSNorm of that * pre as an ``Act``)."""
     D = h.shape[-1]
-    if x.is_cuda and D % 32 == 0 and D <= 8192 and h.dtype == torch.float32 and h.is_contiguous():
+    if (x.is_cuda and D % 32 == 0 and D <= 8192 and x.dtype == h.dtype == torch.float32 and x.shape == h.shape and h.is_contiguous()
+            and all(w is not None and w.dtype == torch.float32 and w.is_contiguous() for w in (post, pre))):
         out, yb, yq, yds = _k().rms_seam(x.contiguous(), post, h, pre, eps, want_q8)
         return out, Act(yb, yq, yds)
     h = norm_add(x, post, eps, h)

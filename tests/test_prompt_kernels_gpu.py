@@ -229,3 +229,16 @@ def test_q8_pairs(N, Kd, M):
     y = (xq.view(M, -1, 32).double() * xds[..., :1].double()).view(M, Kd) @ w.dequantize().double().t()
     # whole-number products of blocks, scaled and added in f32
     assert rel(got, torch.nn.functional.silu(y[:, :N // 2]) * y[:, N // 2:]) < 1e-5
+
+
+@pytest.mark.parametrize("D,dtype,plain", [(2048, torch.float32, False), (2048, torch.bfloat16, False), (8224, torch.float32, False), (2056, torch.float32, False),
+                                           (2048, torch.float32, True)])
+def test_norm_add_norm(D, dtype, plain):
+    """The seam of two norms in one kernel and, for a bf16 sublayer, wide or odd rows or a missing weight, as two."""
+    from tensorsharp_b200.ops import functional as F
+    torch.manual_seed(11)
+    y, h, post, pre = torch.randn(20, D, device=DEV).to(dtype), torch.randn(20, D, device=DEV), torch.rand(D, device=DEV) + 0.5, torch.rand(D, device=DEV) + 0.5
+    post = None if plain else post
+    out, a = F.norm_add_norm(y, post, h, pre, 1e-6)
+    want = h.double() + ref.rmsnorm(y.double(), post, 1e-6).double()
+    assert rel(out, want) < 1e-6 and rel(a.b, ref.rmsnorm(want.float(), pre, 1e-6)) < 3e-3
