@@ -482,13 +482,8 @@ extern "C" int tsb_moe_group_rows(const int* ids, int P, int e0, int E_local, in
     return TSB_OK;
 }
 
-extern "C" int tsb_moe_group(const int* ids, int P, int e0, int E_local, int* pos, void* tiles, int* meta, void* stream) {
-    return tsb_moe_group_rows(ids, P, e0, E_local, MOE_TILE_ROWS, pos, tiles, meta, stream);
-}
-
 // Upper bound on the tile count for P routed pairs over E_local experts (the grid.y of the tile GEMV).
 extern "C" int tsb_moe_max_tiles_rows(int P, int E_local, int tile_rows) { return P / tile_rows + (E_local < P ? E_local : P); }
-extern "C" int tsb_moe_max_tiles(int P, int E_local) { return tsb_moe_max_tiles_rows(P, E_local, MOE_TILE_ROWS); }
 
 // ---------------------------------------------------------------------------------------------
 // Gather into sorted order.  One warp per routed pair; 16-byte copies.
@@ -1259,14 +1254,4 @@ extern "C" int tsb_moe_combine_seam(const float* y, const int* pos, const float*
     TSB_CHECK_CUDA(tsb_launch(moe_combine_kernel, dim3(T), dim3(256), 0, (cudaStream_t)stream, y, pos, w, shared, gate, res, k, D, out));
     TSB_CHECK_LAUNCH();
     return TSB_OK;
-}
-
-extern "C" int tsb_moe_combine(const float* y, const int* pos, int T, int k, int D, float* out, void* stream) {
-    return tsb_moe_combine_seam(y, pos, nullptr, nullptr, nullptr, nullptr, T, k, D, out, stream);
-}
-
-// The same with a weight per (token, slot), for projections that did not scale their rows themselves.
-extern "C" int tsb_moe_combine_weighted(const float* y, const int* pos, const float* w, int T, int k, int D, float* out, void* stream) {
-    TSB_CHECK_ARG(w != nullptr, "moe_combine_weighted: null weights");
-    return tsb_moe_combine_seam(y, pos, w, nullptr, nullptr, nullptr, T, k, D, out, stream);
 }

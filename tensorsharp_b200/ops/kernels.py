@@ -326,11 +326,6 @@ def moe_combine(y: torch.Tensor, pos: torch.Tensor, w: Optional[torch.Tensor], T
     return out
 
 
-def moe_combine_weighted(y: torch.Tensor, pos: torch.Tensor, w: torch.Tensor, T: int, k: int) -> torch.Tensor:
-    """:func:`moe_combine` with a weight for every slot."""
-    return moe_combine(y, pos, w, T, k)
-
-
 def sample(logits: torch.Tensor, ngen: torch.Tensor, *, temperature: float, top_k: int, top_p: float, min_p: float,
            repetition_penalty: float = 1.0, presence_penalty: float = 0.0, frequency_penalty: float = 0.0, seed: int = 0,
            counts: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None) -> torch.Tensor:
