@@ -71,7 +71,33 @@ def test_windows(Hq, Hkv, Dh, window):
 def test_forms(Hq, Hkv, Dh):
     _check(Hq, Hkv, Dh, [70, 9], [70, 333], ps=128, softcap=20.0, gate=True)
     _check(Hq, Hkv, Dh, [257], [1000], sinks=True, peak=30.0)            # row maxima that grow: O is rescaled
-    _check(Hq, Hkv, Dh, [2300], [2300])                                  # more than one wave, two row tiles per CTA
+    _check(Hq, Hkv, Dh, [2300], [2300])                                  # 144 CTAs: just below one per SM at head sizes 64 and 128
+
+
+# on the GPU's 148 SMs: grids on either side of one CTA per SM (head size 64) and two (128), where the tiles change from 128 to 64 keys
+@pytest.mark.parametrize("Hq,Hkv,Dh,qlens,lens", [
+    (64, 8, 64, [288], [700]), (64, 8, 64, [304], [700]), (64, 8, 64, [1000, 17, 333], [1000, 500, 333]),
+    (32, 8, 128, [1184], [1500]), (32, 8, 128, [1185], [1500]), (32, 8, 128, [2048], [2048]), (32, 8, 128, [900, 5, 700], [2000, 400, 700])])
+@pytest.mark.parametrize("window,sinks,peak", [(0, False, 1.0), (300, True, 1.0), (0, True, 20.0)])
+def test_grids_of_one_and_two_blocks_per_sm(Hq, Hkv, Dh, qlens, lens, window, sinks, peak):
+    _check(Hq, Hkv, Dh, qlens, lens, window=window, sinks=sinks, peak=peak)
+
+
+def test_window_over_a_ring_of_pages():
+    """A table whose pages come round again: only the pages that the window reaches hold their own keys."""
+    from tensorsharp_b200.ops import kernels as K
+    torch.manual_seed(8)
+    Hq, Hkv, Dh, window, n, ql, ring = 8, 2, 128, 200, 1500, 180, 7
+    k, v = (torch.randn(n, Hkv, Dh, device=DEV).bfloat16() for _ in range(2))
+    kc, vc = (torch.zeros(ring * 64, Hkv, Dh, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+    for j in range(n):                                                       # the newest keys stay, as a ring keeps them
+        kc[j % (ring * 64)], vc[j % (ring * 64)] = k[j], v[j]
+    table = (torch.arange((n + 63) // 64, dtype=torch.int32, device=DEV) % ring)[None].contiguous()
+    q = torch.randn(ql, Hq, Dh, device=DEV).bfloat16()
+    cu, kl = torch.tensor([0, ql], dtype=torch.int32, device=DEV), torch.tensor([n], dtype=torch.int32, device=DEV)
+    got = K.attn_prefill(q, kc, vc, table, kl, cu, ql, scale=0.1, Hq=Hq, Hkv=Hkv, Dh=Dh, page_size=64, window=window)
+    want = ref.attention(q, k, v, torch.arange(n - ql, n, device=DEV), scale=0.1, window=window)
+    assert ((got.float() - want).norm() / want.norm()).item() < 6e-3
 
 
 @pytest.mark.parametrize("Hq,Hkv,Dh", [(16, 2, 64), (8, 2, 128)])

@@ -279,8 +279,7 @@ def test_attn_prefill(Hq, Hkv, Dh, window, sinks, softcap):
         o += ql
 
 
-# the last four shapes have more tiles than SMs and take the persistent kernel (two accumulators in tensor memory, the
-# epilogue of a tile under the next tile's main loop): 256- and 128-token tiles, ragged edges, a single k-block
+# more than 64 tokens: pairs of CTAs (several tiles a pair in the large ones), ragged edges, a single k-block
 @pytest.mark.parametrize("T,N,Kd", [(5, 128, 64), (33, 200, 320), (100, 384, 2560), (300, 1000, 512), (2048, 256, 1024),
                                     (3900, 7744, 320), (4096, 7680, 64), (100, 20480, 256), (520, 19400, 192),
                                     (16, 2560, 9728), (33, 640, 4096), (9, 256, 8192)])     # the last three: split-K

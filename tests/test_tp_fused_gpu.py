@@ -126,6 +126,39 @@ def test_single_rank_push_then_reduce_round_trip():
     tpx.close()
 
 
+@pytest.mark.parametrize("T", [3000, 2900, 300])
+def test_sequence_parallel_gemms_of_a_single_rank(T):
+    """Gather, gather -> GEMM, GEMM -> reduce-scatter and the reducing norm with one rank, every wait already met by the launch before it.
+    3000 tokens: a shard of 3072 rows, the persistent kernel with tiles of 256 rows; 2900: of 2944 and 128; 300: one tile per CTA."""
+    from tensorsharp_b200.gguf.constants import GGMLType
+    from tensorsharp_b200.ops import reference as ref
+    from tensorsharp_b200.parallel.dist import Communicator
+    from tensorsharp_b200.parallel.fused import TpSeqParallel
+    from tensorsharp_b200.quant.qweight import QuantWeight
+    dev = torch.device("cuda", 0)
+    torch.manual_seed(1)
+    hidden, N, K = 2048, 2568, 328
+    sp = TpSeqParallel(Communicator(0, 1, dev), T, hidden)
+    wq = QuantWeight.from_float(torch.randn(N, hidden, device=dev) * 0.02, GGMLType.BF16)
+    wo = QuantWeight.from_float(torch.randn(hidden, K, device=dev) * 0.05, GGMLType.BF16)
+    nw, bias = torch.rand(hidden, device=dev) + 0.5, torch.randn(N, device=dev)
+    h = torch.zeros(sp.shard, hidden, device=dev)
+    h[:T] = torch.randn(T, hidden, device=dev)
+    x = torch.randn(T, K, device=dev).bfloat16()
+    rel = lambda a, b: ((a.double() - b.double()).norm() / b.double().norm()).item()               # noqa: E731
+    sp.norm_gather(h, nw, 1e-6, False)
+    for rep in range(3):                            # counters and accumulators of several exchanges
+        a = ref.rmsnorm(h[:T], nw, 1e-6).bfloat16()
+        # the gathered rows are rounded to bf16 once, as those are: a value on an edge may fall the other way
+        assert rel(sp.gemm_ag(wq, T, bias=bias, out_dtype=torch.float32), a.double() @ wq.dequantize().double().t() + bias) < 2e-3
+        want = h[:T].double() + (x.double() @ wo.dequantize().double().t()).float().bfloat16().double()
+        sp.gemm_rs(x, wo)
+        sp.norm_gather(h, nw, 1e-6, True)
+        assert rel(h[:T], want) < 2e-4 and not h[T:].any()
+    assert sp.status() == 0
+    sp.close()
+
+
 def test_pipeline_stages_over_nccl(kv8_model_path):
     """Two pipeline stages on two GPUs (NCCL send / recv of the residual stream, token broadcast back)
     generate what one GPU generates."""
