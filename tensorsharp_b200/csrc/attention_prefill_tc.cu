@@ -433,6 +433,10 @@ long prefill_ctas(const AttnArgs& a, int max_q_len) {
 // 5.1 .. 5.5; one KV head per query head, 6 or 16 of them, 1 to 32 prompts 4.1 .. 9.9 / 5.0 .. 10.6; 64 / 8 heads, 4 prompts 5.6 .. 6.8 /
 // 5.2 .. 5.5.  Soft cap, head size 64: 38 CTAs 22.0 / 25.5, 64 CTAs 34 / 41, 72 CTAs 10.7 / 10.7, 80 CTAs 27.6 / 26.0, 128 CTAs
 // 50 / 41; head size 128, 64 slots 7.9 / 8.2.
+// And at head size 64 with one head per row tile, up to 128 slots, where a tile of 128 rows stands against tiles of 64: prompts of 65 to
+// 128 tokens while those smaller tiles still have an SM each (6, 10, 14, 16 or 32 heads, 65 tokens, up to 64 CTAs here 5.1 .. 5.3 /
+// 5.5 .. 5.9, 128 tokens 5.8 .. 6.0 / 5.7 .. 6.4; 80 CTAs 6.3 / 5.9, 112 CTAs 7.3 / 6.1), and more than two CTAs per SM of at most 64 tokens, half
+// of each tile empty (10 tokens on 90: 256 CTAs 7.9 / 6.4, 320 CTAs 8.1 / 10.6, 448 CTAs 11.4 / 11.6, 1024 CTAs 18.1 / 22.1).
 extern "C" int tsb_attn_prefill_tc_takes(const AttnArgs* args, int max_q_len, long cache_rows) {
     const AttnArgs& a = *args;
     const uintptr_t all = reinterpret_cast<uintptr_t>(a.q) | reinterpret_cast<uintptr_t>(a.k_cache) | reinterpret_cast<uintptr_t>(a.v_cache) |
@@ -441,7 +445,12 @@ extern "C" int tsb_attn_prefill_tc_takes(const AttnArgs* args, int max_q_len, lo
         a.page_size % 64 != 0 || cache_rows < 64 || (all & 15) != 0 || a.Hkv <= 0 || a.Hq % a.Hkv != 0)
         return 0;
     const bool tiny = (long)a.max_pages * a.page_size <= 64, few = (long)a.Hq * a.B < 256;
-    if (a.Dh == 64 && ((tiny && (few || packed_heads(a) == 1)) || (a.softcap > 0.f && prefill_ctas(a, max_q_len) < 72))) return 0;
+    if (a.Dh == 64) {
+        const long ctas = prefill_ctas(a, max_q_len);
+        const bool single = packed_heads(a) == 1, two_pages = (long)a.max_pages * a.page_size <= 128;
+        if ((tiny && (few || single)) || (a.softcap > 0.f && ctas < 72)) return 0;
+        if (single && two_pages && (max_q_len > 64 ? ctas <= 74 : ctas > 296)) return 0;
+    }
     return !(a.Dh == 128 && a.softcap > 0.f && tiny && few);
 }
 

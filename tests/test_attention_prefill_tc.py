@@ -108,6 +108,13 @@ def test_both_sides_of_the_tile_rule(Hq, Hkv, Dh, qlens, lens, window, softcap):
     _check(Hq, Hkv, Dh, qlens, lens, window=window, softcap=softcap, gate=softcap > 0 and window > 0)
 
 
+@pytest.mark.parametrize("qlens,lens", [([64], [128]), ([65], [65]), ([128, 3], [128, 120]), ([65] * 7, [70] * 7), ([65] * 8, [70] * 8), ([10] * 29, [100] * 29),
+                                        ([64] * 30, [128] * 30), ([10] * 30, [129] * 30)])
+def test_both_sides_of_the_rule_for_single_heads(qlens, lens):
+    # ten heads in groups of five: one head per row tile
+    _check(10, 2, 64, qlens, lens, sinks=True)
+
+
 @pytest.mark.parametrize("Hq,Hkv,Dh,ql,n,peak", [(32, 8, 128, 300, 2000, 3.0), (32, 8, 128, 1100, 1100, 6.0), (16, 2, 64, 1024, 1024, 4.0), (16, 2, 256, 200, 900, 3.0)])
 def test_as_exact_as_the_mma_kernel(Hq, Hkv, Dh, ql, n, peak):
     """Both kernels round each weight, taken relative to the running maximum, and the result to bf16 and keep the rest in f32, so

@@ -46,6 +46,14 @@ def test_smallest_prompts_and_small_capped_grids():
     assert not takes(Dh=128, softcap=30.0, max_pages=1) and takes(Dh=128, softcap=30.0, max_pages=2)
 
 
+def test_single_heads_of_64_on_two_pages():
+    """One head per row tile: 65 to 128 tokens up to 74 CTAs, at most 64 tokens beyond 296, both up to 128 slots."""
+    one = dict(Dh=64, Dv=64, Hq=10, Hkv=2, max_pages=2)
+    assert not takes(max_q=65, **one, B=7) and takes(max_q=64, **one, B=7) and takes(max_q=65, **one, B=8) and takes(max_q=65, **{**one, "max_pages": 3}, B=7)
+    assert not takes(max_q=64, **one, B=30) and takes(max_q=64, **one, B=29) and takes(max_q=65, **one, B=30) and takes(max_q=64, **{**one, "max_pages": 3}, B=30)
+    assert takes(max_q=65, **{**one, "Hq": 8}, B=7) and takes(max_q=65, **{**one, "Dh": 128, "Dv": 128}, B=7)
+
+
 def test_a_whole_library_without_the_kernel_is_refused(monkeypatch):
     """An old build is an error, not the slower kernel; a library of selected sources may lack it."""
     class Old:
