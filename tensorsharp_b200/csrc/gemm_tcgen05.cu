@@ -485,7 +485,10 @@ static int launch_gemm_persistent(const CUtensorMap& tw, const CUtensorMap& tx, 
 // cycle at bn = 256.  Each CTA loads its 128 features and its half of the tokens, the even CTA issues the products, each
 // CTA keeps the accumulators of its own features in its own tensor memory (two buffers, epilogue under the next tile as
 // above).  bn is any multiple of 16, so that the last wave can be filled (choose_pair_bn).
-// Measured (us; kernel above / this one): see choose_pair_bn.
+// Bound by the tensor pipe (busy 90 % of the time that an SM has work at 2048 x 19456 x 2560), on narrow shapes by the last wave.
+// Measured (us; one CTA per SM as above, one-tile or persistent / this one): 65 x 2560 x 4096 21.1 / 19.2, 512 x 6144 x 2560 24.2 /
+// 17.5, 2048 x 2560 x 4096 63.7 / 41.9, 2048 x 2560 x 9728 134 / 91, 4096 x 37984 x 2560 636 / 572; 2048 x (2 x 9728) x 2560 with
+// SwiGLU 187 (and a kernel of its own for it) / 149.
 // ------------------------------------------------------------------------------------------
 constexpr int PAIR_STAGES = 6;
 constexpr int PAIR_STAGE_BYTES = 2 * 128 * 128;                  // 128 features and up to 128 tokens, 64 bf16 each

@@ -940,10 +940,10 @@ __global__ void __launch_bounds__(128) gemv_tiles_mma_wide_kernel(TileArgs a) {
 // word is decoded once for up to 16 rows, so an expert with 9 to 16 pairs no longer streams its matrix twice.
 // The 16-byte block of a row's stage sits at place (block ^ (row / 2 & 3)), so that the eight rows of a fragment load differ in
 // their banks.  Products are those of the kernel above; each half of K is summed in its order and the second joins the first.
-// Bound by memory (the weights of the experts that were chosen), next to it by the decode of the 4-bit words.
+// Bound by issue slots (63 % busy: the decode of the 4-bit words, a scale and conversions per block of 32); the weights of the chosen
+// experts come from DRAM once, at a quarter of its rate.
 // Measured, 32 experts of 2880 x 2880, top 4 of 64 tokens, us per launch (8-byte-load version of the kernel above / this
-// one): gate and up 194 / 148, down 113 / 90 (four warps a CTA over the
-// whole of K: 157 and 102).
+// one): gate and up 194 / 148, down 113 / 90 (four warps a CTA over the whole of K: 157 and 102).
 template <bool GLU, bool MX>
 struct RingSmem {
     static constexpr int S = GLU ? 2 : 1, STG = 3, SB = MX ? 1 : 2;     // weight row sets; ring stages; bytes of a block scale
