@@ -829,6 +829,28 @@ int tsb_make_tmap_2d_bf16(CUtensorMap* out, const void* base, uint64_t rows, uin
     return tsb_make_tmap_bf16(out, base, 2, dims, &row_stride_elems, box);
 }
 
+// A map over rows of bytes.  Boxes of 128 and of 64 bytes take the swizzle of their width, others none.
+int tsb_make_tmap_bytes(CUtensorMap* out, const void* base, uint64_t rows, uint64_t row_bytes, uint32_t box_rows, uint32_t box_bytes) {
+    std::call_once(g_encode_once, resolve_encode);
+    if (!g_encode) {
+        tsb_set_error("cuTensorMapEncodeTiled is not available from the driver");
+        return TSB_ERR_CUDA;
+    }
+    TSB_CHECK_ARG((reinterpret_cast<uintptr_t>(base) & 15) == 0, "tensor map base %p is not 16-byte aligned", base);
+    TSB_CHECK_ARG(row_bytes % 16 == 0 && box_bytes % 16 == 0 && box_bytes <= 256 && box_rows <= 256, "tensor map of rows of %llu bytes, box %u x %u",
+                  (unsigned long long)row_bytes, box_rows, box_bytes);
+    const cuuint64_t gdim[2] = {row_bytes, rows}, gstride[1] = {row_bytes};
+    const cuuint32_t gbox[2] = {box_bytes, box_rows}, estr[2] = {1, 1};
+    const CUtensorMapSwizzle sw = box_bytes == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : box_bytes == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_NONE;
+    CUresult r = g_encode(out, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), gdim, gstride, gbox, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, sw,
+                          CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) {
+        tsb_set_error("cuTensorMapEncodeTiled failed with CUresult %d (rows of %llu bytes, box %u x %u)", (int)r, (unsigned long long)row_bytes, box_rows, box_bytes);
+        return TSB_ERR_CUDA;
+    }
+    return TSB_OK;
+}
+
 template <int BN, int STAGES>
 static int launch_gemm(const CUtensorMap& tw, const CUtensorMap& tx, const GemmEpi& ep, int K, int* status,
                        cudaStream_t s) {

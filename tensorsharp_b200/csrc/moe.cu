@@ -466,7 +466,7 @@ __global__ void __launch_bounds__(1024) moe_group_kernel(const int* __restrict__
 
 // `tile_rows`: most rows of a tile (what the tile kernels that follow take: MOE_TILE_ROWS, or tsb_moe_tile_rows()).
 extern "C" int tsb_moe_group_rows(const int* ids, int P, int e0, int E_local, int tile_rows, int* pos, void* tiles, int* meta, void* stream) {
-    TSB_CHECK_ARG(tile_rows == MOE_TILE_ROWS || tile_rows == MOE_RING_ROWS, "moe_group: tiles of %d rows", tile_rows);
+    TSB_CHECK_ARG(tile_rows == MOE_TILE_ROWS || tile_rows == MOE_RING_ROWS || tile_rows == 32 || tile_rows == 64, "moe_group: tiles of %d rows", tile_rows);
     TSB_CHECK_ARG(E_local > 0 && E_local <= 1024, "moe_group: %d local experts (limit 1024)", E_local);
     const size_t smem = sizeof(int) * ((size_t)P + 2 * (E_local + 1));
     TSB_CHECK_ARG(smem <= 200 * 1024, "moe_group: %d routed pairs do not fit one CTA's shared memory", P);

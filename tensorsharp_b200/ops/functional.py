@@ -23,6 +23,7 @@ import torch
 from ..quant.qweight import QuantWeight
 from . import reference as ref
 
+BLOCK_GEMM_MAX_M = 64  # up to this many rows the weights' bytes are the bound, and the tensor cores read the GGUF blocks themselves
 PAIR_GEMM_MIN_M = 64  # above this many rows the tensor-core GEMM is the one that can end with the gated activation
 GATED_ACTS = ("swiglu", "geglu", "geglu_tanh", "geglu_erf", "swiglu_oai")
 GEMV_MAX_M = 16   # "small batch": token count up to which the models take their decode-style paths (int8 activations, mailbox exchanges)
@@ -450,6 +451,8 @@ def linear(a: Act, w: QuantWeight, *, bias: Optional[torch.Tensor] = None, resid
             _ensure_q8(a)
             return k.gemv(w, xq=a.q, xds=a.ds, M=T, out_dtype=out_dtype, bias=bias, residual=residual, act=act)
         return k.gemv(w, xb=a.b.contiguous(), M=T, out_dtype=out_dtype, bias=bias, residual=residual, act=act)
+    if T <= BLOCK_GEMM_MAX_M and k.gemm_blocks_takes(w, act) and (residual is None or (residual.dtype == out_dtype and residual.is_contiguous())):
+        return k.gemm_blocks(w, a.b, out_dtype=out_dtype, bias=bias, residual=residual, act=act)
     wb = _dequant_scratch(w)
     if act is None:
         return k.gemm_bf16(wb, a.b, out_dtype=out_dtype, bias=bias, residual=residual)
@@ -1137,8 +1140,10 @@ def moe_experts(a: Act, ids: torch.Tensor, weights: torch.Tensor, gate_up: Quant
         if down_scale is not None:
             wts = wts * down_scale[ids.reshape(-1).long()]
         if gate_up.uses_q8_activations:
-            _ensure_q8(a)
-            return kk.moe_grouped(xq=a.q, xds=a.ds, ids=ids, weights=wts, gate_up=gate_up, down=down, act=act,
+            blocks = a.b is not None and a.b.dtype == torch.bfloat16 and kk.gemm_experts_takes(gate_up, act) and kk.gemm_experts_takes(down)
+            if not blocks:
+                _ensure_q8(a)
+            return kk.moe_grouped(xq=a.q, xds=a.ds, xb=a.b.contiguous() if blocks else None, ids=ids, weights=wts, gate_up=gate_up, down=down, act=act,
                                   gate_up_bias=gate_up_bias, down_bias=down_bias, expert_offset=expert_offset, shared=shared, residual=residual)
         return kk.moe_grouped(xb=a.b.contiguous(), ids=ids, weights=wts, gate_up=gate_up, down=down, act=act,
                               gate_up_bias=gate_up_bias, down_bias=down_bias, expert_offset=expert_offset, shared=shared, residual=residual)

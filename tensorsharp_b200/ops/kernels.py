@@ -13,6 +13,7 @@ from typing import Optional
 
 import torch
 
+from ..gguf.constants import GGMLType
 from ..quant.qweight import QuantWeight
 from . import native
 
@@ -230,11 +231,19 @@ def gather_bf16_rows(x: torch.Tensor, order: torch.Tensor, div: int) -> torch.Te
     return out
 
 
+def expert_tile_rows(most: int, P: int, E: int) -> int:
+    """Rows of a tile of :func:`gemm_experts` for P pairs over E experts: twice the average and more, so that most experts' weights are
+    decoded once.  Measured, a layer of 32 experts of 2880 x 2880 (us; tiles of 16 / 32 / 64): 256 pairs 194 / 194 / 201, 512 280 / 200 / 211, 768
+    342 / 224 / 225, 1024 433 / 305 / 237."""
+    return min(most, 32 if P <= 16 * E else 64)
+
+
 def moe_grouped(*, xq=None, xds=None, xb=None, ids: torch.Tensor, weights: torch.Tensor, gate_up: QuantWeight,
                 down: QuantWeight, act, gate_up_bias=None, down_bias=None, expert_offset: int = 0, shared=None, residual=None) -> torch.Tensor:
     """Grouped expert projections with the routing kept on the device (no host read-back, fixed launch
     sequence): group the (token, slot) pairs by local expert, gather activations into that order, run
-    gate/up and down as tile GEMVs (each tile streams its expert's rows once for up to 8 pairs, 16 in 4-bit blocks), and
+    gate/up and down as tile GEMVs (each tile streams its expert's rows once for up to 8 pairs, 16 in 4-bit blocks) or, where
+    the experts are MXFP4 and bf16 rows are given, as tensor-core products of tiles of 16 to 64 pairs, and
     sum every token's slots.  ``ids`` are global expert ids [T, k]; pairs whose expert is not in
     ``[expert_offset, expert_offset + gate_up.experts)`` contribute nothing.  Returns f32 [T, D]."""
     lib = _lib()
@@ -248,7 +257,11 @@ def moe_grouped(*, xq=None, xds=None, xb=None, ids: torch.Tensor, weights: torch
     D, K = down.N, gate_up.K
     ids = ids.contiguous()
     pos = torch.empty((P,), dtype=torch.int32, device=dev)
-    rows = int(lib.tsb_moe_tile_rows(C.c_int(int(gate_up.ggml_type)), C.c_int(gate_up.N), C.c_int(K), C.c_int(a), C.c_int(int(down.ggml_type)),
+    tc_rows = min(gemm_experts_takes(gate_up, act), gemm_experts_takes(down)) if xb is not None else 0
+    if tc_rows:
+        tc_rows = expert_tile_rows(tc_rows, P, E_local)
+        xq = xds = None
+    rows = tc_rows or int(lib.tsb_moe_tile_rows(C.c_int(int(gate_up.ggml_type)), C.c_int(gate_up.N), C.c_int(K), C.c_int(a), C.c_int(int(down.ggml_type)),
                                      C.c_int(D), C.c_int(F_out), C.c_int(P), C.c_int(E_local)))
     max_tiles = int(lib.tsb_moe_max_tiles_rows(C.c_int(P), C.c_int(E_local), C.c_int(rows)))
     tiles = torch.empty((max_tiles, 4), dtype=torch.int32, device=dev)
@@ -266,6 +279,11 @@ def moe_grouped(*, xq=None, xds=None, xb=None, ids: torch.Tensor, weights: torch
     wflat = weights.reshape(-1).float().contiguous()
     native.check(lib.tsb_moe_gather(_p(pos), C.c_int(P), C.c_int(k), C.c_int(K), _p(xq), _p(xds), _p(xb), _p(wflat), _p(sq),
                                     _p(sds), _p(sb), _p(sw), _stream()), "moe_gather")
+    if tc_rows:
+        gu = gemm_experts(gate_up, sb, tiles, meta, rows, out_dtype=torch.bfloat16, bias=gate_up_bias, act=act)
+        y = gemm_experts(down, gu, tiles, meta, rows, out_dtype=torch.float32, bias=down_bias, row_scale=sw)
+        _count(2)
+        return moe_combine(y, pos, None, T, k, shared, residual)
     gu = torch.zeros((P, F_out), dtype=torch.bfloat16, device=dev)
     ps = _planes(gate_up)
     native.check(lib.tsb_moe_gemv_tiles(ps[0], ps[1], ps[2], ps[3], C.c_int(int(gate_up.ggml_type)), C.c_int(gate_up.N), C.c_int(K),
@@ -1316,6 +1334,53 @@ def gemm_bf16_glu(W: torch.Tensor, X: torch.Tensor, act: str, *, bias=None, E: i
                                        C.c_int(T), C.c_int(N), C.c_int(K), C.c_int(ACT[act]), _p(tiles),
                                        C.c_int(tiles.shape[0] if tiles is not None else 0), C.c_int(bn), _p(gemm_status(X.device)), _stream()),
                  "gemm_bf16_glu")
+    _count(1)
+    return out
+
+
+def gemm_blocks_takes(w: QuantWeight, act=None) -> bool:
+    """Whether :func:`gemm_blocks` takes the matrix (csrc/gemm_blocks.cu: tsb_gemm_blocks_takes)."""
+    return (w.experts == 1 and w.ggml_type in (GGMLType.Q4_K, GGMLType.Q6_K, GGMLType.Q8_0) and w.K % 256 == 0
+            and (not 1 <= ACT[act] <= 4 or w.N % 2 == 0) and all(p.data_ptr() % 16 == 0 for p in w.planes[:3]))
+
+
+def gemm_blocks(w: QuantWeight, X: torch.Tensor, *, out_dtype=torch.float32, bias=None, residual=None, act=None) -> torch.Tensor:
+    """act(X [T, K] @ w^T + bias) (+ residual in ``out_dtype``) for up to 64 bf16 rows, the weight read as GGUF blocks."""
+    assert X.dtype == torch.bfloat16 and X.stride(1) == 1 and (residual is None or (residual.dtype == out_dtype and residual.is_contiguous()))
+    T, a = X.shape[0], ACT[act]
+    n_out = w.N // 2 if 1 <= a <= 4 else w.N
+    out = torch.empty((T, n_out), dtype=out_dtype, device=X.device)
+    lib = _lib()
+    lib.tsb_gemm_blocks.restype = C.c_int
+    ps = _planes(w)
+    native.check(lib.tsb_gemm_blocks(ps[0], ps[1], ps[2], ps[3], C.c_int(int(w.ggml_type)), C.c_int(w.N), C.c_int(w.K), _p(X), C.c_long(X.stride(0)),
+                                     C.c_int(T), _p(out), C.c_long(n_out), C.c_int(out_dtype == torch.float32), _p(bias), _p(residual), C.c_int(a),
+                                     _p(gemm_status(X.device)), _stream()), "gemm_blocks")
+    _count(1)
+    return out
+
+
+def gemm_experts_takes(w: QuantWeight, act=None) -> int:
+    """Most rows of a tile with which :func:`gemm_experts` takes the stack; 0: not at all."""
+    if w.ggml_type != GGMLType.MXFP4 or any(p.data_ptr() % 16 for p in w.planes):
+        return 0
+    return _lib().tsb_gemm_experts_takes(C.c_int(int(w.ggml_type)), C.c_int(w.N), C.c_int(w.K), C.c_int(ACT[act]))
+
+
+def gemm_experts(w: QuantWeight, X: torch.Tensor, tiles: torch.Tensor, meta: torch.Tensor, tile_rows: int, *, out_dtype, bias=None, row_scale=None,
+                 act=None, out: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """The same for the matrices of a stack: bf16 rows in expert order [P, K], ``tiles`` int32 [n, 4] {expert, first row, rows, -} of at most
+    ``tile_rows`` rows, ``meta[0]`` of them; rows that no tile covers are not written."""
+    a = ACT[act]
+    n_out = w.N // 2 if 1 <= a <= 4 else w.N
+    if out is None:
+        out = torch.empty((X.shape[0], n_out), dtype=out_dtype, device=X.device)
+    lib = _lib()
+    lib.tsb_gemm_experts.restype = C.c_int
+    ps = _planes(w)
+    native.check(lib.tsb_gemm_experts(ps[0], ps[1], C.c_int(int(w.ggml_type)), C.c_int(w.N), C.c_int(w.K), C.c_int(w.experts), _p(X), C.c_int(X.shape[0]),
+                                      _p(out), C.c_long(n_out), C.c_int(out_dtype == torch.float32), _p(bias), _p(row_scale), _p(tiles), _p(meta),
+                                      C.c_int(tiles.shape[0]), C.c_int(tile_rows), C.c_int(a), _p(gemm_status(X.device)), _stream()), "gemm_experts")
     _count(1)
     return out
 
