@@ -104,7 +104,7 @@ def recurrent(args):
 
         def kern3():
             s3.zero_()
-            return kernels.gdn_chunked(qkv, z, beta, alpha, dt_bias, a_log, norm_w, s3, cu_q, [0, T], [0], **kw)
+            return kernels.gdn_chunked(qkv, z, beta, alpha, dt_bias, a_log, norm_w, s3, cu_q, [0, T], torch.zeros(1, dtype=torch.int64, device=dev), **kw)
     if args.op == "mamba2":
         s3 = torch.zeros(1, H, P, N, device=dev)
 

@@ -1311,7 +1311,7 @@ def gdn(qkv: torch.Tensor, z: torch.Tensor, beta: torch.Tensor, alpha: torch.Ten
     slots = batch.host_slots()
     if chunked and qkv.is_cuda and os.environ.get("TSB_GDN_CHUNK_KERNELS", "1") != "0" and _k().gdn_chunked_supported(Dk, Dv) \
             and qkv.dtype == torch.float32 and beta.dtype == alpha.dtype and beta.stride(0) == alpha.stride(0):
-        return _k().gdn_chunked(qkv, z, beta, alpha, dt_bias, a_log, norm_w, state, batch.cu_q, list(batch.h_cu_q), slots,
+        return _k().gdn_chunked(qkv, z, beta, alpha, dt_bias, a_log, norm_w, state, batch.cu_q, list(batch.h_cu_q), batch.seq_slots,
                                 Hk=Hk, Hv=Hv, Dk=Dk, Dv=Dv, eps=eps)
     if chunked:                                 # every sequence of a batch that took this route, short ones included
         carry = None

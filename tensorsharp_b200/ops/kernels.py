@@ -1427,8 +1427,8 @@ class GdnCarryArgs(C.Structure):
 
 class GdnPrepArgs(C.Structure):
     _fields_ = [("qkv", _vp), ("qkv_s", C.c_long), ("beta", _vp), ("alpha", _vp), ("ba_s", C.c_long), ("ba_f32", C.c_int),
-                ("dt_bias", _vp), ("a_log", _vp), ("cu_q", _vp),
-                ("U0", _vp), ("W", _vp), ("Qd", _vp), ("Kd", _vp), ("P", _vp), ("gamma", _vp),
+                ("dt_bias", _vp), ("a_log", _vp), ("cu_q", _vp), ("K", _vp), ("Q", _vp), ("T", _vp), ("P", _vp), ("scale", _vp), ("gamma", _vp),
+                ("state", _vp), ("slots", _vp), ("out", _vp), ("status", _vp),
                 ("Hk", C.c_int), ("Hv", C.c_int), ("Dk", C.c_int), ("Dv", C.c_int), ("B", C.c_int), ("nc", C.c_int),
                 ("eps", C.c_float)]
 
@@ -1487,39 +1487,40 @@ def gdn_chunked_supported(Dk: int, Dv: int) -> bool:
     return Dk in (64, 128) and Dv % 32 == 0 and Dv <= 128
 
 
-def gdn_chunked(qkv, z, beta, alpha, dt_bias, a_log, norm_w, state, cu_q, h_cu_q, slots, *, Hk, Hv, Dk, Dv, eps) -> torch.Tensor:
+def gdn_chunked(qkv, z, beta, alpha, dt_bias, a_log, norm_w, state, cu_q, h_cu_q, seq_slots, *, Hk, Hv, Dk, Dv, eps) -> torch.Tensor:
     """Chunked GatedDeltaNet prefill of a packed batch in three kernels (csrc/gdn_chunk.cu): the chunk-parallel algebra
-    (normalisation, decay, Gram products, the triangular solve) per (sequence, head, chunk); the state carried chunk
-    after chunk per (sequence, head, value slice); the gated output norm.  ``state`` [slots, Hv, Dv, Dk] f32 is updated
-    for the sequences' slots (host list ``slots``); ``cu_q`` int32 [B + 1] on the device, ``h_cu_q`` its host copy.
+    (normalisation, decay, Gram products, the triangular inverse) per (sequence, key head, chunk); the state carried chunk
+    after chunk per (sequence, value head, value slice); the gated output norm.  ``state`` [slots, Hv, Dv, Dk] f32 is updated
+    for the sequences' slots (``seq_slots`` int64 [B] on the device); ``cu_q`` int32 [B + 1] on the device, ``h_cu_q`` its host copy.
     Returns bf16 [T, Hv * Dv]."""
     T = qkv.shape[0]
     B = len(h_cu_q) - 1
     nc = (max(h_cu_q[i + 1] - h_cu_q[i] for i in range(B)) + 63) // 64
     dev = qkv.device
-    assert qkv.dtype == torch.float32 and qkv.stride(1) == 1 and beta.dtype == alpha.dtype and beta.stride(0) == alpha.stride(0)
+    assert qkv.dtype == torch.float32 and beta.dtype == alpha.dtype and beta.stride(0) == alpha.stride(0)
+    assert state.dtype == torch.float32 and state.is_contiguous() and seq_slots.dtype == torch.int64
+    check_index("gdn_chunked", "state slot", seq_slots, state.shape[0])
+    check_index("gdn_chunked", "row offset", cu_q, T + 1)
+    if qkv.stride(1) != 1 or qkv.stride(0) % 4 or qkv.data_ptr() % 16:
+        qkv = qkv.contiguous()
     BH = B * Hv
     f32 = dict(dtype=torch.float32, device=dev)
-    U0, W = torch.empty((BH, nc, 64, Dv), **f32), torch.empty((BH, nc, 64, Dk), **f32)
-    Qd, Kd = torch.empty((BH, nc, 64, Dk), **f32), torch.empty((BH, nc, 64, Dk), **f32)
-    P, gamma = torch.empty((BH, nc, 64, 64), **f32), torch.empty((BH, nc), **f32)
+    Ks, Qs = torch.empty((B * Hk, nc, 64 * Dk), **f32), torch.empty((B * Hk, nc, 64 * Dk), **f32)
+    Ti, P = torch.empty((BH, nc, 2 * 2560), **f32), torch.empty((BH, nc, 2560), **f32)
+    scale, gamma = torch.empty((BH, nc, 64, 4), **f32), torch.empty((BH, nc), **f32)
+    core = torch.empty((BH, nc, 64, Dv), **f32)
     a = GdnPrepArgs()
     a.qkv, a.qkv_s = _p(qkv), qkv.stride(0)
     a.beta, a.alpha, a.ba_s, a.ba_f32 = _p(beta), _p(alpha), beta.stride(0), int(beta.dtype == torch.float32)
     a.dt_bias, a.a_log, a.cu_q = _p(dt_bias), _p(a_log), _p(cu_q)
-    a.U0, a.W, a.Qd, a.Kd, a.P, a.gamma = _p(U0), _p(W), _p(Qd), _p(Kd), _p(P), _p(gamma)
+    seq_slots = seq_slots.contiguous()
+    a.K, a.Q, a.T, a.P, a.scale, a.gamma = _p(Ks), _p(Qs), _p(Ti), _p(P), _p(scale), _p(gamma)
+    a.state, a.slots, a.out, a.status = _p(state), _p(seq_slots), _p(core), _p(gemm_status(dev))
     a.Hk, a.Hv, a.Dk, a.Dv, a.B, a.nc, a.eps = Hk, Hv, Dk, Dv, B, nc, eps
     lib = _lib()
-    native.check(lib.tsb_gdn_chunk_prep(C.byref(a), _stream()), "gdn_chunk_prep")
-    _count(1)
-    if B == 1:
-        S = state[slots[0]]
-    else:
-        idx = torch.tensor(slots, dtype=torch.long, device=dev)
-        S = state[idx].reshape(BH, Dv, Dk)
-    core = gdn_chunk_carry(U0, W, Qd, Kd, P, gamma, S)
-    if B > 1:
-        state[idx] = S.view(B, Hv, Dv, Dk)
+    lib.tsb_gdn_chunks.restype = C.c_int
+    native.check(lib.tsb_gdn_chunks(C.byref(a), _stream()), "gdn_chunks")
+    _count(2)
     out = torch.empty((T, Hv * Dv), dtype=torch.bfloat16, device=dev)
     f = GdnFinishArgs()
     f.core, f.z, f.z_s, f.z_f32 = _p(core), _p(z), z.stride(0), int(z.dtype == torch.float32)

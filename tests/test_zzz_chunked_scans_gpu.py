@@ -92,6 +92,45 @@ def test_chunk_carry_kernel_matches_the_scan_across_chunk_and_call_boundaries(mo
     assert _rel(kern[0], scan[0]) < 2e-2 and _rel(kern[1], scan[1]) < 3e-3, (_rel(kern[0], scan[0]), _rel(kern[1], scan[1]))
 
 
+# The delta rule in 64 bits, token by token: tf32 factors are rounded by 2^-12 each (four products from a chunk's keys to the state: below 1e-3),
+# the bf16 output by 2^-9 once more.  One to five value heads per key head, chunks of one to 64 tokens at a sequence's
+# end, a sequence that is shorter than a chunk, slots in any order.
+@pytest.mark.parametrize("Hk,Hv,Dk,Dv", [(2, 4, 128, 128), (1, 5, 64, 32), (3, 3, 128, 64)])
+@pytest.mark.parametrize("lens", [[64], [65, 1, 200], [7], [128, 127]])
+def test_chunk_kernels_against_64_bits(monkeypatch, Hk, Hv, Dk, Dv, lens):
+    monkeypatch.setenv("TSB_GDN_CHUNKED", "1")
+    monkeypatch.setenv("GDN_CHUNK_PREFILL_MIN_SEQ_LEN", "2")
+    torch.manual_seed(3)
+    dev, T, B = "cuda", sum(lens), len(lens)
+    dtb, a_log, nw = torch.randn(Hv, device=dev) * 0.5, -torch.rand(Hv, device=dev), torch.rand(Dv, device=dev) + 0.5
+    state = torch.randn(B + 1, Hv, Dv, Dk, device=dev) * 0.1
+    qkv = torch.randn(T, 2 * Hk * Dk + Hv * Dv, device=dev)
+    z, beta, alpha = torch.randn(T, Hv * Dv, device=dev), torch.randn(T, Hv, device=dev), torch.randn(T, Hv, device=dev)
+    b = _batch(lens, dev)
+    slots = list(range(B, 0, -1))
+    b.seq_slots, b.h_seq_slots = torch.tensor(slots, device=dev), tuple(slots)
+    want_s = state.double().clone()
+    outs = []
+    for i, n in enumerate(lens):
+        r0 = sum(lens[:i])
+        S = want_s[slots[i]]
+        for t in range(r0, r0 + n):
+            row = qkv[t].double()
+            q, k = (row[j * Hk * Dk:(j + 1) * Hk * Dk].view(Hk, Dk) for j in range(2))
+            q, k = q * torch.rsqrt((q * q).sum(-1, keepdim=True) + 1e-6) * Dv ** -0.5, k * torch.rsqrt((k * k).sum(-1, keepdim=True) + 1e-6)
+            heads = torch.arange(Hv, device=dev) % Hk
+            q, k, v = q[heads], k[heads], row[2 * Hk * Dk:].view(Hv, Dv)
+            g = torch.exp(torch.nn.functional.softplus(alpha[t].double() + dtb.double()) * a_log.double())
+            S.mul_(g.view(-1, 1, 1))
+            S.add_((torch.sigmoid(beta[t].double()).view(-1, 1) * (v - torch.einsum("hvk,hk->hv", S, k))).unsqueeze(-1) * k.unsqueeze(1))
+            o = torch.einsum("hvk,hk->hv", S, q)
+            o = o * torch.rsqrt((o * o).mean(-1, keepdim=True) + 1e-6) * nw.double()
+            outs.append((o * torch.nn.functional.silu(z[t].double().view(Hv, Dv))).reshape(-1))
+    got = F.gdn(qkv, z, beta, alpha, dtb, a_log, nw, state, b, Hk=Hk, Hv=Hv, Dk=Dk, Dv=Dv, eps=1e-6)
+    assert _rel(got.double(), torch.stack(outs)) < 1e-2 and _rel(state.double(), want_s) < 3e-3
+    assert torch.equal(state[0].double(), want_s[0])
+
+
 @pytest.mark.parametrize("H,P,G,N", [(4, 64, 2, 128), (6, 32, 1, 64), (8, 64, 8, 128)])
 def test_mamba2_chunk_kernels_match_the_scan_across_chunk_and_call_boundaries(monkeypatch, H, P, G, N):
     """csrc/gdn_chunk.cu: mamba2_chunk_prep_kernel + the chunk-carry kernel against the token-by-token scan kernel and
