@@ -111,9 +111,15 @@ class Batch:
         return self.tokens.shape[0]
 
 
+_kernels = None
+
+
 def _k():
-    from . import kernels
-    return kernels
+    global _kernels
+    if _kernels is None:
+        from . import kernels
+        _kernels = kernels
+    return _kernels
 
 
 # --------------------------------------------------------------------------------------------

@@ -27,8 +27,15 @@ def _p(t: Optional[torch.Tensor]):
     return _vp(t.data_ptr()) if t is not None else _vp(0)
 
 
+def _ptr(t: Optional[torch.Tensor]):
+    """The address for a function with declared argument types (``_ARGS``)."""
+    return t.data_ptr() if t is not None else None
+
+
 def _stream():
-    return _vp(torch.cuda.current_stream().cuda_stream)
+    """The current stream's handle.  A prompt makes this call for every one of its launches, and the Stream object that
+    torch.cuda.current_stream() builds costs ten times what the handle does."""
+    return _vp(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
 
 
 # Debug mode TSB_CHECK_INDICES=1: before a launch, every index tensor that the kernel will use to address memory (token
@@ -86,6 +93,10 @@ class AttnArgs(C.Structure):
                 ("kv_scale", C.c_int), ("log_r1", _vp), ("log_r2", _vp), ("sig_bias", _vp)]
 
 
+_KIND = {"p": _vp, "i": C.c_int, "l": C.c_long, "f": C.c_float}
+_ARGS = {"tsb_gemm_blocks": "ppppiiipliplipp" "ipp", "tsb_gemm_bf16_ws": "plplplippiiipppl", "tsb_gemm_bf16_glu": "plipl" "plp" "iii" "ip" "ii" "pp",
+         "tsb_rmsnorm": "pippflipppppip"}
+
 _configured = False
 _prefill_tc = False   # whether the library has the tcgen05 prompt attention
 LAUNCHES = 0          # kernels launched through this module (eager mode; graph replays add theirs)
@@ -110,6 +121,11 @@ def _lib():
             fn = getattr(lib, name, None)             # a library linked from a selection of sources lacks some
             if fn is not None:
                 fn.restype = C.c_int
+        # the launches of a prompt's layers: plain ints, floats and None go through without a ctypes object for each argument
+        for name, kinds in _ARGS.items():
+            fn = getattr(lib, name, None)
+            if fn is not None:
+                fn.restype, fn.argtypes = C.c_int, [_KIND[k] for k in kinds]
         _configured = True
     return lib
 
@@ -407,9 +423,8 @@ def rmsnorm(x: torch.Tensor, w: Optional[torch.Tensor], eps: float, *, delta=Non
     if want_q8:
         yq = torch.empty((rows, D), dtype=torch.int8, device=dev)
         yds = torch.empty((rows, D // 32, 2), dtype=torch.float32, device=dev)
-    native.check(_lib().tsb_rmsnorm(_p(x), C.c_int(x.dtype == torch.float32), _p(delta), _p(w), C.c_float(eps),
-                                    C.c_long(rows), C.c_int(D), _p(yb), _p(yf), _p(add), _p(yq), _p(yds),
-                                    C.c_int(1 if l2 else 0), _stream()), "rmsnorm")
+    native.check(_lib().tsb_rmsnorm(x.data_ptr(), x.dtype == torch.float32, _ptr(delta), _ptr(w), eps, rows, D, _ptr(yb), _ptr(yf), _ptr(add), _ptr(yq),
+                                    _ptr(yds), l2, _stream()), "rmsnorm")
     _count(1)
     return yb, yf, yq, yds
 
@@ -1312,12 +1327,9 @@ def gemm_bf16(W: torch.Tensor, X: torch.Tensor, *, out_dtype=torch.bfloat16, bia
     if out is None:
         out = torch.empty((T, N), dtype=out_dtype, device=X.device)
     ws = _splitk_workspace(X.device) if T <= 64 else None       # few tiles, long K: the library may split K over CTAs
-    lib = _lib()
-    lib.tsb_gemm_bf16_ws.restype = C.c_int
-    native.check(lib.tsb_gemm_bf16_ws(_p(W), C.c_long(W.stride(0)), _p(X), C.c_long(X.stride(0)), _p(out),
-                                      C.c_long(out.stride(0)), C.c_int(out.dtype == torch.float32), _p(bias),
-                                      _p(residual), C.c_int(T), C.c_int(N), C.c_int(K), _p(gemm_status(X.device)),
-                                      _stream(), _p(ws), C.c_long(ws.numel() * 4 if ws is not None else 0)), "gemm_bf16")
+    native.check(_lib().tsb_gemm_bf16_ws(W.data_ptr(), W.stride(0), X.data_ptr(), X.stride(0), out.data_ptr(), out.stride(0), out.dtype == torch.float32,
+                                         _ptr(bias), _ptr(residual), T, N, K, gemm_status(X.device).data_ptr(), _stream(), _ptr(ws),
+                                         ws.numel() * 4 if ws is not None else 0), "gemm_bf16")
     _count(1)
     return out
 
@@ -1328,11 +1340,8 @@ def gemm_bf16_glu(W: torch.Tensor, X: torch.Tensor, act: str, *, bias=None, E: i
     assert W.dtype == torch.bfloat16 and X.dtype == torch.bfloat16 and W.stride(1) == 1 and X.stride(1) == 1
     N, K, T = W.shape[0] // E, W.shape[1], X.shape[0]
     out = torch.empty((T, N // 2), dtype=torch.bfloat16, device=X.device)
-    lib = _lib()
-    lib.tsb_gemm_bf16_glu.restype = C.c_int
-    native.check(lib.tsb_gemm_bf16_glu(_p(W), C.c_long(W.stride(0)), C.c_int(E), _p(X), C.c_long(X.stride(0)), _p(out), C.c_long(N // 2), _p(bias),
-                                       C.c_int(T), C.c_int(N), C.c_int(K), C.c_int(ACT[act]), _p(tiles),
-                                       C.c_int(tiles.shape[0] if tiles is not None else 0), C.c_int(bn), _p(gemm_status(X.device)), _stream()),
+    native.check(_lib().tsb_gemm_bf16_glu(W.data_ptr(), W.stride(0), E, X.data_ptr(), X.stride(0), out.data_ptr(), N // 2, _ptr(bias), T, N, K, ACT[act],
+                                          _ptr(tiles), tiles.shape[0] if tiles is not None else 0, bn, gemm_status(X.device).data_ptr(), _stream()),
                  "gemm_bf16_glu")
     _count(1)
     return out
@@ -1350,12 +1359,9 @@ def gemm_blocks(w: QuantWeight, X: torch.Tensor, *, out_dtype=torch.float32, bia
     T, a = X.shape[0], ACT[act]
     n_out = w.N // 2 if 1 <= a <= 4 else w.N
     out = torch.empty((T, n_out), dtype=out_dtype, device=X.device)
-    lib = _lib()
-    lib.tsb_gemm_blocks.restype = C.c_int
-    ps = _planes(w)
-    native.check(lib.tsb_gemm_blocks(ps[0], ps[1], ps[2], ps[3], C.c_int(int(w.ggml_type)), C.c_int(w.N), C.c_int(w.K), _p(X), C.c_long(X.stride(0)),
-                                     C.c_int(T), _p(out), C.c_long(n_out), C.c_int(out_dtype == torch.float32), _p(bias), _p(residual), C.c_int(a),
-                                     _p(gemm_status(X.device)), _stream()), "gemm_blocks")
+    p = [t.data_ptr() for t in w.planes] + [None, None, None]
+    native.check(_lib().tsb_gemm_blocks(p[0], p[1], p[2], p[3], w.ggml_type, w.N, w.K, X.data_ptr(), X.stride(0), T, out.data_ptr(), n_out,
+                                        out_dtype == torch.float32, _ptr(bias), _ptr(residual), a, gemm_status(X.device).data_ptr(), _stream()), "gemm_blocks")
     _count(1)
     return out
 
