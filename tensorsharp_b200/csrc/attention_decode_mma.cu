@@ -330,6 +330,232 @@ __global__ void __launch_bounds__(128) attn_decode_mma_kernel(AttnArgs a) {
     }
 }
 
+// The same for bf16 pages of whole 16-key chunks without a cluster (every decode step of the models takes it), with the keys on their way
+// while others are multiplied: a warp walks chunks of 16 keys (stride 64) through a ring of three of its own, two of them asked for ahead.
+// A chunk lies in one page, so a lane's pieces are one pointer and a stride; fragment addresses are one XOR each; masks and the
+// rescaling of the sums run only for chunks that need them.  (With an address per piece and all of that on every chunk the
+// kernel issued 990 instructions a chunk, and that bound it: 41 % of the issue slots with two warps per scheduler, HBM at 38 %.)
+// The chunks are asked for before the wait for the kernel ahead, except the one that holds the newest key: the kernel ahead writes the
+// rows of this step's tokens, and the lengths, the block table and all earlier rows are older than that.
+// Measured with the merge kernel, us (the kernel above with its own splits / this one): 16 sequences of 2048 down to 1088 31.4 / 27.1,
+// 32 of them 50.8 / 42.8, 4 of 4096 down to 2560 21.6 / 16.5 (32 query, 8 key heads of 128); 64 of 1024 down to 520, 64 query, 8 key heads of 64 36.5 / 22.1, with a window of
+// 128 15.2 / 5.9; one of 131 7.1 / 5.1, one of 8111 14.3 / 13.7.
+template <int DH>
+__global__ void __launch_bounds__(128) attn_decode_ring_kernel(AttnArgs a) {
+    constexpr int CH = DH / 8, KT = 16, STG = 3, TILE = KT * DH * 2;                       // bytes of a K or V tile
+    constexpr float LOG2E = 1.4426950408889634f;
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    bf16* sQ = reinterpret_cast<bf16*>(smem_raw);                          // [16][DH]
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t ring = (uint32_t)__cvta_generic_to_shared(smem_raw) + 16 * DH * 2 + warp * (STG * 2 * TILE);      // [STG][K, V][16][DH]
+    const int split = blockIdx.x, hk = blockIdx.y, b = blockIdx.z;
+    const int G = a.Hq / a.Hkv, h0 = hk * G;
+    const int len = a.kv_lens[b];
+    const int lo = (a.window > 0 && len > a.window) ? len - a.window : 0;
+    const int span = len - lo;
+    const int per = a.split_len > 0 ? a.split_len : ((((span + a.splits - 1) / a.splits) + 31) & ~31);
+    const int s0 = lo + split * per, s1 = min(len, s0 + per), w0 = (s0 & ~(KT - 1)) + warp * KT;      // this warp's first chunk
+    const int n = max(0, (s1 - w0 + 4 * KT - 1) / (4 * KT));                // and how many it has
+    const int* table = a.block_table + (long)b * a.max_pages;
+    auto slot_of = [&](int i) {
+        const int j = w0 + i * 4 * KT;
+        return i < n ? table[j / a.page_size] * a.page_size + j % a.page_size : 0;
+    };
+    // a lane copies the pieces of column chunk lane % CH of every (32 / CH)-th key: their places in a tile are swizzled by the key's low bits
+    constexpr int KEYS = 32 / CH, IT = KT / KEYS;
+    const int c = lane % CH, key0 = lane / CH;
+    const long stride = (long)a.Hkv * DH;
+    const bf16* kp = a.k_cache + (long)hk * DH + c * 8 + key0 * stride;
+    const bf16* vp = a.v_cache + (long)hk * DH + c * 8 + key0 * stride;
+    bool waited = false;
+    auto fetch = [&](int i, int slot) {
+        if (i < n) {
+            const int base = w0 + i * 4 * KT;
+            if (!waited && base + KT >= len) {
+                pdl_wait();
+                waited = true;
+            }
+            const uint32_t dst = ring + (i % STG) * (2 * TILE) + key0 * DH * 2;
+            const bf16 *k = kp + (long)slot * stride, *v = vp + (long)slot * stride;
+            const bool whole = base >= s0 && base + KT <= s1;
+#pragma unroll
+            for (int r = 0; r < IT; ++r, k += KEYS * stride, v += KEYS * stride) {
+                const int key = base + key0 + r * KEYS;
+                const uint32_t at = dst + r * (KEYS * DH * 2) + ((c ^ ((key0 + r * KEYS) & 7)) << 4);
+                if (whole || (key >= s0 && key < s1)) {
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(at), "l"(k));
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(at + TILE), "l"(v));
+                } else {                                                    // 0 x garbage would poison P V
+                    asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(at), "r"(0u) : "memory");
+                    asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(at + TILE), "r"(0u) : "memory");
+                }
+            }
+        }
+        cp_async_commit();
+    };
+    const int first = slot_of(0), second = slot_of(1);
+    fetch(0, first);
+    fetch(1, second);
+    int next = slot_of(2);
+    if (!waited) pdl_wait();
+    waited = true;
+    pdl_trigger();
+    for (int i = threadIdx.x; i < 16 * CH; i += 128) {                      // rows past the group are zero
+        const int r = i / CH, cc = i % CH;
+        uint4 v = make_uint4(0u, 0u, 0u, 0u);
+        if (r < G) v = *reinterpret_cast<const uint4*>(a.q + ((long)b * a.Hq + h0 + r) * DH + cc * 8);
+        *reinterpret_cast<uint4*>(tile_ptr<DH>(sQ, r, cc)) = v;
+    }
+    __syncthreads();
+    uint32_t qa[DH / 16][4];
+#pragma unroll
+    for (int kk = 0; kk < DH / 16; ++kk) ldsm_x4(qa[kk], tile_ptr<DH>(sQ, lane & 15, kk * 2 + (lane >> 4)));
+    float o[DH / 8][4];
+#pragma unroll
+    for (int i = 0; i < DH / 8; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
+    float mrow[2] = {-INFINITY, -INFINITY}, lrow[2] = {0.f, 0.f};          // rows lane / 4 and lane / 4 + 8
+    // fragment addresses in a tile: a row of DH * 2 bytes is a power of two, so the column chunk 2 kk joins by an XOR
+    const int kt = ((lane >> 4) << 3) + (lane & 7), vt = (((lane >> 3) & 1) << 3) + (lane & 7);
+    const uint32_t kfrag = kt * DH * 2 + ((((lane >> 3) & 1) ^ (kt & 7)) << 4), vfrag = TILE + vt * DH * 2 + (((lane >> 4) ^ (vt & 7)) << 4);
+
+    for (int i = 0; i < n; ++i) {
+        fetch(i + 2, next);
+        next = slot_of(i + 3);
+        cp_async_wait<2>();
+        __syncwarp();
+        const uint32_t tile = ring + (i % STG) * (2 * TILE);
+        const int base = w0 + i * 4 * KT;
+        float s[2][4] = {};
+#pragma unroll
+        for (int kk = 0; kk < DH / 16; ++kk) {
+            uint32_t kb[4];
+            asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+                         : "=r"(kb[0]), "=r"(kb[1]), "=r"(kb[2]), "=r"(kb[3]) : "r"((tile + kfrag) ^ (kk << 5)) : "memory");
+            mma_bf16(s[0], qa[kk], kb[0], kb[1]);
+            mma_bf16(s[1], qa[kk], kb[2], kb[3]);
+        }
+        // scale, soft cap, mask, online softmax (scores in natural-log units, as the combine expects)
+        float mx[2] = {-INFINITY, -INFINITY};
+#pragma unroll
+        for (int e = 0; e < 8; ++e) s[e >> 2][e & 3] *= a.scale;
+        if (a.softcap > 0.f) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) s[e >> 2][e & 3] = a.softcap * tanhf(s[e >> 2][e & 3] / a.softcap);
+        }
+        if (base < s0 || base + KT > s1) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                const int key = base + (e >> 2) * 8 + (lane & 3) * 2 + (e & 1);
+                if (key < s0 || key >= s1) s[e >> 2][e & 3] = -INFINITY;
+            }
+        }
+#pragma unroll
+        for (int e = 0; e < 8; ++e) mx[(e >> 1) & 1] = fmaxf(mx[(e >> 1) & 1], s[e >> 2][e & 3]);
+        float corr[2], mneg[2];
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 1));
+            mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 2));
+            mx[r] = fmaxf(mrow[r], mx[r]);
+        }
+        if (__any_sync(0xffffffffu, mx[0] > mrow[0] || mx[1] > mrow[1])) {  // a new maximum: what there is belongs to the old one
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+                corr[r] = (mrow[r] == -INFINITY) ? 0.f : exp2f((mrow[r] - mx[r]) * LOG2E);
+                lrow[r] *= corr[r];
+                mrow[r] = mx[r];
+            }
+#pragma unroll
+            for (int d = 0; d < DH / 8; ++d) {
+                o[d][0] *= corr[0]; o[d][1] *= corr[0];
+                o[d][2] *= corr[1]; o[d][3] *= corr[1];
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < 2; ++r) mneg[r] = (mrow[r] == -INFINITY) ? 0.f : -mrow[r] * LOG2E;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            const int r = (e >> 1) & 1;
+            s[e >> 2][e & 3] = exp2f(fmaf(s[e >> 2][e & 3], LOG2E, mneg[r]));
+            lrow[r] += s[e >> 2][e & 3];
+        }
+        const uint32_t pa[4] = {pack_bf16(s[0][0], s[0][1]), pack_bf16(s[0][2], s[0][3]), pack_bf16(s[1][0], s[1][1]), pack_bf16(s[1][2], s[1][3])};
+#pragma unroll
+        for (int dt = 0; dt < DH / 16; ++dt) {
+            uint32_t vb[4];
+            asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                         : "=r"(vb[0]), "=r"(vb[1]), "=r"(vb[2]), "=r"(vb[3]) : "r"((tile + vfrag) ^ (dt << 5)) : "memory");
+            mma_bf16(o[2 * dt], pa, vb[0], vb[1]);
+            mma_bf16(o[2 * dt + 1], pa, vb[2], vb[3]);
+        }
+        __syncwarp();                                                       // the chunk's place is free
+    }
+    cp_async_wait<0>();
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+        lrow[r] += __shfl_xor_sync(0xffffffffu, lrow[r], 1);
+        lrow[r] += __shfl_xor_sync(0xffffffffu, lrow[r], 2);
+    }
+    // merge the four warps through shared memory, over the rings
+    __syncthreads();
+    float* red_m = reinterpret_cast<float*>(smem_raw);                      // [4][16]
+    float* red_l = red_m + 64;                                              // [4][16]
+    float* red_o = red_l + 64;                                              // [4][G][DH]
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+        const int row = (lane >> 2) + 8 * r;
+        if (row < G) {
+            if ((lane & 3) == 0) { red_m[warp * 16 + row] = mrow[r]; red_l[warp * 16 + row] = lrow[r]; }
+#pragma unroll
+            for (int i = 0; i < DH / 8; ++i)
+                *reinterpret_cast<float2*>(red_o + (warp * G + row) * DH + i * 8 + (lane & 3) * 2) = make_float2(o[i][2 * r], o[i][2 * r + 1]);
+        }
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < G * DH; i += 128) {
+        const int g = i / DH, d = i % DH;
+        float mm = -INFINITY;
+#pragma unroll
+        for (int w = 0; w < 4; ++w) mm = fmaxf(mm, red_m[w * 16 + g]);
+        float ll = 0.f, ov = 0.f;
+#pragma unroll
+        for (int w = 0; w < 4; ++w) {
+            const float c = (red_m[w * 16 + g] == -INFINITY) ? 0.f : __expf(red_m[w * 16 + g] - mm);
+            ll += red_l[w * 16 + g] * c;
+            ov += red_o[(w * G + g) * DH + d] * c;
+        }
+        if (a.splits > 1 || a.gate != nullptr) {
+            const long pi = ((long)b * a.Hq + h0 + g) * a.splits + split;
+            a.part_o[pi * DH + d] = ov;
+            if (d == 0) { a.part_ml[pi * 2] = mm; a.part_ml[pi * 2 + 1] = ll; }
+            continue;
+        }
+        // a single split is the result: the arithmetic of attn_combine_kernel
+        const float sink = a.sinks ? a.sinks[h0 + g] : -INFINITY, top = fmaxf(mm, sink), cf = mm == -INFINITY ? 0.f : __expf(mm - top);
+        const float sum = ll * cf + (a.sinks ? __expf(sink - top) : 0.f);
+        const bf16 ob = f2bf(sum > 0.f ? ov * cf / sum : 0.f);
+        const long e = ((long)b * a.Hq + h0 + g) * DH + d;
+        a.out[e] = ob;
+        if (a.out_q != nullptr) {                                           // a warp holds one group of 32 columns
+            const float v = bf2f(ob), amax = warp_max(fabsf(v)), vs = warp_sum(v), dq = amax / 127.f;
+            a.out_q[e] = (int8_t)__float2int_rn(amax > 0.f ? v / dq : 0.f);
+            if ((d & 31) == 0) a.out_ds[e >> 5] = make_float2(dq, vs);
+        }
+    }
+}
+
+template <int DH>
+static int launch_decode_ring(const AttnArgs& a, cudaStream_t s) {
+    constexpr size_t smem = (size_t)(16 + 4 * 3 * 2 * 16) * DH * sizeof(bf16);     // the merge needs 4 x 16 rows of floats and less
+    static bool configured = false;
+    if (!configured) {
+        TSB_CHECK_CUDA(cudaFuncSetAttribute(attn_decode_ring_kernel<DH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        configured = true;
+    }
+    TSB_CHECK_CUDA(tsb_launch(attn_decode_ring_kernel<DH>, dim3(a.splits, a.Hkv, a.B), dim3(128), smem, s, a));
+    return TSB_OK;
+}
+
 template <int DH, int CS, bool FP8 = false>
 static int launch_decode_mma(const AttnArgs& a, cudaStream_t s) {
     // the query tile, four warps' K and V tiles; the merge buffers reuse them (4 * 16 * DH floats, and with a cluster
@@ -382,13 +608,15 @@ bool tsb_attn_decode_mma_cluster(const AttnArgs& a) {
     return cols % (a.splits * 32) == 0;
 }
 
-// Returns TSB_OK; `*merged` tells whether the outputs are final (cluster form) or the caller has to launch the combine.
+// Returns TSB_OK; `*merged` tells whether the outputs are final (cluster form, a single split) or the caller has to launch the combine.
 int tsb_attn_decode_mma_launch(const AttnArgs& a, cudaStream_t s, bool* merged) {
     const bool cl = tsb_attn_decode_mma_cluster(a);
     *merged = cl;
     if (cl && a.splits == 8) return a.Dh == 64 ? launch_decode_mma<64, 8>(a, s) : launch_decode_mma<128, 8>(a, s);
     if (cl) return a.Dh == 64 ? launch_decode_mma<64, 16>(a, s) : launch_decode_mma<128, 16>(a, s);
-    return a.Dh == 64 ? launch_decode_mma<64, 0>(a, s) : launch_decode_mma<128, 0>(a, s);
+    if (a.page_size % 16 != 0) return a.Dh == 64 ? launch_decode_mma<64, 0>(a, s) : launch_decode_mma<128, 0>(a, s);
+    *merged = a.splits == 1 && a.gate == nullptr;
+    return a.Dh == 64 ? launch_decode_ring<64>(a, s) : launch_decode_ring<128>(a, s);
 }
 
 // The same split kernel on e4m3 pages (`k_cache` / `v_cache` point at bytes); the caller launches the combine.

@@ -637,12 +637,21 @@ def decode_split_len(batch: Batch, splits: int, window: int) -> int:
     return ((batch.max_kv_len + splits - 1) // splits + 31) & ~31
 
 
-def decode_splits(batch: Batch, Hkv: int, window: int) -> int:
-    """Split-KV factor for decode attention: enough CTAs to cover the GPU's 148 SMs."""
+def ring_attention(Hq: int, Hkv: int, Dh: int, page_size: int, fp8: bool) -> bool:
+    """Whether decode attention takes attn_decode_ring_kernel (csrc/attention_decode_mma.cu)."""
+    return Dh in (64, 128) and Hq % Hkv == 0 and Hq // Hkv <= 16 and page_size % 16 == 0 and not fp8
+
+
+def decode_splits(batch: Batch, Hkv: int, window: int, ring: bool = False) -> int:
+    """Split-KV factor for decode attention: enough CTAs to cover the GPU's 148 SMs.  ``ring``: the kernel that loads ahead, two CTAs an SM and
+    no more (with the merge, us for 1 / 2 / 3 / 4 / 9 splits: 16 sequences of about 1600 40.9 / 26.3 / 27.1 / 26.0 / 30.2, 32 46.3 / 42.8 / 45.6 / 47.8;
+    64 of about 800 29.7 / 31.4 / 33.2; 4 of about 3300 for 4 / 9 / 13 / 18 / 37 21.3 / 16.0 / 18.8 / 19.1 / 23.8)."""
     span = batch.max_kv_len if not window else min(batch.max_kv_len, window)
     # one sequence: about two CTAs per SM; batches: up to eight (a CTA is 128 threads and latency-bound, and with 16
     # sequences two splits per (sequence, KV head) left the kernel at a fifth of the memory rate)
     want = max(1, (148 * (2 if batch.B == 1 else 8)) // max(1, batch.B * Hkv))
+    if ring and batch.B > 1:
+        want = -(-296 // (batch.B * Hkv))
     per = int(os.environ.get("TSB_ATTN_SPLIT_LEN", "128"))
     n = int(max(1, min(want, (span + per - 1) // per, 64)))
     # TSB_ATTN_CLUSTER=1: 8 or 16 splits are merged inside the attention kernel by a thread-block cluster (no combine
@@ -678,9 +687,10 @@ def attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, bat
                                 kv_scale=Hkv * Dh if own_values else 0, log_bias=log_bias, sigmoid_bias=sigmoid_bias)
     if as_act:
         if q.is_cuda and batch.is_decode and Dh % 32 == 0:
-            sp = decode_splits(batch, Hkv, window)
+            ring = ring_attention(Hq, Hkv, Dh, batch.page_size, is_fp8(k_cache))
+            sp = decode_splits(batch, Hkv, window, ring)
             out, oq, ods = _k().attn_decode(q, k_cache, v_cache, batch.block_table, batch.kv_lens, scale=scale, Hq=Hq, Hkv=Hkv,
-                                            Dh=Dh, page_size=batch.page_size, splits=sp, split_len=decode_split_len(batch, sp, window),
+                                            Dh=Dh, page_size=batch.page_size, splits=sp, split_len=0 if ring else decode_split_len(batch, sp, window),
                                             sinks=sinks, softcap=softcap, window=window, want_q8=True)
             return Act(out.view(T, Hq * Dh), oq, ods)
         return as_act_of(attention(q, k_cache, v_cache, batch, scale=scale, Hq=Hq, Hkv=Hkv, Dh=Dh, window=window, sinks=sinks,
@@ -688,9 +698,10 @@ def attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, bat
     if q.is_cuda:
         kk = _k()
         if batch.is_decode:
-            sp = decode_splits(batch, Hkv, window)
+            ring = ring_attention(Hq, Hkv, Dh, batch.page_size, is_fp8(k_cache))
+            sp = decode_splits(batch, Hkv, window, ring)
             out = kk.attn_decode(q, k_cache, v_cache, batch.block_table, batch.kv_lens, scale=scale, Hq=Hq, Hkv=Hkv,
-                                 Dh=Dh, page_size=batch.page_size, splits=sp, split_len=decode_split_len(batch, sp, window),
+                                 Dh=Dh, page_size=batch.page_size, splits=sp, split_len=0 if ring else decode_split_len(batch, sp, window),
                                  sinks=sinks, softcap=softcap, window=window)
         else:
             table, ps = batch.block_table, batch.page_size
