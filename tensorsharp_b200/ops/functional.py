@@ -13,6 +13,7 @@ Data conventions
 """
 from __future__ import annotations
 
+import functools
 import math
 import os
 from dataclasses import dataclass, field
@@ -24,6 +25,9 @@ from ..quant.qweight import QuantWeight
 from . import reference as ref
 
 BLOCK_GEMM_MAX_M = 64  # up to this many rows the weights' bytes are the bound, and the tensor cores read the GGUF blocks themselves
+# Routed pairs up to which MXFP4 experts go to the GEMV of one pair each: measured, a layer of 32 experts of 2880 x 2880 (us, GEMV / tensor cores): 4 pairs
+# 46 / 53, 8 72 / 72, 12 97 / 85, 16 122 / 99, 32 220 / 131, 64 420 / 165
+EXPERT_GEMV_PAIRS = 8
 PAIR_GEMM_MIN_M = 64  # above this many rows the tensor-core GEMM is the one that can end with the gated activation
 GATED_ACTS = ("swiglu", "geglu", "geglu_tanh", "geglu_erf", "swiglu_oai")
 GEMV_MAX_M = 16   # "small batch": token count up to which the models take their decode-style paths (int8 activations, mailbox exchanges)
@@ -430,6 +434,22 @@ def _dequant_scratch(w: QuantWeight, holder: Optional[QuantWeight] = None, slot:
     return out
 
 
+def gemv_rows(w: QuantWeight, act: Optional[str] = None) -> int:
+    """Most rows of bf16 activations for which a product goes to the GEMV kernels: two (one where the matrix is large) where the tensor cores
+    take the weight as it is, which costs the same for one row as for sixteen.  Measured, us for 1 / 2 / 3 / 4 / 8 rows (GEMV; tensor cores):
+    Q4_K 1024 x 2560 2.6 / 2.6 / 4.7 / 5.6 / 5.9; 4.8, 2560 x 4096 3.4 / 4.1 / 7.2 / 7.7 / 10.5; 6.2, 6144 x 2560 4.4 / 7.8 / 13.0 / 14.5 / 8.7; 7.5, 2 x 9728 x
+    2560 10.9 / 23.3 / 30.1 / 31.6 / 18.7; 16.8; Q6_K 2560 x 9728 7.6 / 12.4 / 20.7 / 20.9 / 59.8; 11.5; Q8_0 5376 x 21504 26.9 / 29.5 / 43.8 / 44.0 / 90.2; 27; bf16 2880 x
+    4096 7.5 / 9.0 / 12.8 / 12.8 / 21.8; 9.2, 32768 x 2880 29.8 / 36.2 / 56.4 / 58.0 / 102.8; 35."""
+    from ..gguf.constants import GGMLType
+    if w.experts != 1:
+        return DENSE_GEMV_MAX_M
+    if w.ggml_type == GGMLType.BF16:
+        return min(DENSE_GEMV_MAX_M, 2) if w.N * w.K >= 4 << 20 and w.K % 8 == 0 and w.planes[0].data_ptr() % 16 == 0 else DENSE_GEMV_MAX_M
+    if not _k().gemm_blocks_takes(w, act):
+        return DENSE_GEMV_MAX_M
+    return min(DENSE_GEMV_MAX_M, 1 if w.N * w.K >= 20 << 20 else 2)
+
+
 def linear(a: Act, w: QuantWeight, *, bias: Optional[torch.Tensor] = None, residual: Optional[torch.Tensor] = None,
            out_dtype=torch.float32, act: Optional[str] = None) -> torch.Tensor:
     """y = a @ w^T (+ bias) (+ residual), optional GLU over the row halves of ``w``
@@ -452,7 +472,7 @@ def linear(a: Act, w: QuantWeight, *, bias: Optional[torch.Tensor] = None, resid
             y = y + residual.float()
         return y.to(out_dtype) if out_dtype != torch.float32 else y
     k = _k()
-    if T <= DENSE_GEMV_MAX_M or (T <= GEMV_MAX_M and (a.b is None or w.experts != 1 or w.K % 8)):
+    if T <= (DENSE_GEMV_MAX_M if a.b is None else 1) or (T <= GEMV_MAX_M and (a.b is None or w.experts != 1 or w.K % 8)) or T <= gemv_rows(w, act):
         if w.uses_q8_activations:
             _ensure_q8(a)
             return k.gemv(w, xq=a.q, xds=a.ds, M=T, out_dtype=out_dtype, bias=bias, residual=residual, act=act)
@@ -481,7 +501,7 @@ def linear_multi(a: Act, ws, *, out_dtype=torch.float32):
     type); anything else is the plain sequence of ``linear`` calls."""
     ws = list(ws)
     T = a.T
-    if (ws[0].device.type == "cuda" and T <= DENSE_GEMV_MAX_M and 2 <= len(ws) <= 3 and all(w.experts == 1 and w.K == ws[0].K for w in ws)
+    if (ws[0].device.type == "cuda" and T <= (1 if a.b is not None and T > 1 and all(T > gemv_rows(w) for w in ws) else DENSE_GEMV_MAX_M) and 2 <= len(ws) <= 3 and all(w.experts == 1 and w.K == ws[0].K for w in ws)
             and len({w.uses_q8_activations for w in ws}) == 1):
         if ws[0].uses_q8_activations:
             _ensure_q8(a)
@@ -629,12 +649,20 @@ def fp8_prefill_view(k_cache: torch.Tensor, v_cache: torch.Tensor, batch: Batch)
     return kd, vd, table, L
 
 
-def decode_split_len(batch: Batch, splits: int, window: int) -> int:
+def decode_split_len(batch: Batch, splits: int, window: int, ring: bool = False) -> int:
     """Positions per split fixed on the host from the reserved maximum length (0 with a sliding window, whose
-    start depends on the actual length): the kernel then knows its range before it has read the length."""
+    start depends on the actual length): the kernel then knows its range before it has read the length.  ``ring``: a sequence's own
+    length is shared out, which that kernel reads ahead of its wait, in parts of no less than decode_splits counts with (the negative
+    number): a captured step, whose splits go by its bucket, then cuts a sequence where an eager one does."""
+    if ring:
+        return -_split_positions()
     if window:
         return 0
     return ((batch.max_kv_len + splits - 1) // splits + 31) & ~31
+
+
+def _split_positions() -> int:
+    return int(os.environ.get("TSB_ATTN_SPLIT_LEN", "128"))
 
 
 def ring_attention(Hq: int, Hkv: int, Dh: int, page_size: int, fp8: bool) -> bool:
@@ -652,7 +680,7 @@ def decode_splits(batch: Batch, Hkv: int, window: int, ring: bool = False) -> in
     want = max(1, (148 * (2 if batch.B == 1 else 8)) // max(1, batch.B * Hkv))
     if ring and batch.B > 1:
         want = -(-296 // (batch.B * Hkv))
-    per = int(os.environ.get("TSB_ATTN_SPLIT_LEN", "128"))
+    per = _split_positions()
     n = int(max(1, min(want, (span + per - 1) // per, 64)))
     # TSB_ATTN_CLUSTER=1: 8 or 16 splits are merged inside the attention kernel by a thread-block cluster (no combine
     # launch), so take those counts when the natural one is close (measured slower than the combine launch: off by default)
@@ -690,7 +718,7 @@ def attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, bat
             ring = ring_attention(Hq, Hkv, Dh, batch.page_size, is_fp8(k_cache))
             sp = decode_splits(batch, Hkv, window, ring)
             out, oq, ods = _k().attn_decode(q, k_cache, v_cache, batch.block_table, batch.kv_lens, scale=scale, Hq=Hq, Hkv=Hkv,
-                                            Dh=Dh, page_size=batch.page_size, splits=sp, split_len=0 if ring else decode_split_len(batch, sp, window),
+                                            Dh=Dh, page_size=batch.page_size, splits=sp, split_len=decode_split_len(batch, sp, window, ring),
                                             sinks=sinks, softcap=softcap, window=window, want_q8=True)
             return Act(out.view(T, Hq * Dh), oq, ods)
         return as_act_of(attention(q, k_cache, v_cache, batch, scale=scale, Hq=Hq, Hkv=Hkv, Dh=Dh, window=window, sinks=sinks,
@@ -701,7 +729,7 @@ def attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, bat
             ring = ring_attention(Hq, Hkv, Dh, batch.page_size, is_fp8(k_cache))
             sp = decode_splits(batch, Hkv, window, ring)
             out = kk.attn_decode(q, k_cache, v_cache, batch.block_table, batch.kv_lens, scale=scale, Hq=Hq, Hkv=Hkv,
-                                 Dh=Dh, page_size=batch.page_size, splits=sp, split_len=0 if ring else decode_split_len(batch, sp, window),
+                                 Dh=Dh, page_size=batch.page_size, splits=sp, split_len=decode_split_len(batch, sp, window, ring),
                                  sinks=sinks, softcap=softcap, window=window)
         else:
             table, ps = batch.block_table, batch.page_size
@@ -1123,7 +1151,9 @@ def moe_experts(a: Act, ids: torch.Tensor, weights: torch.Tensor, gate_up: Quant
     local = ids - expert_offset
     if expert_offset != 0 or E_local != int(1e9):
         local = torch.where((local >= 0) & (local < E_local), local, torch.full_like(local, -1))
-    if dev.type == "cuda" and T * k <= 4 * GEMV_MAX_M:
+    blocks = (dev.type == "cuda" and push is None and a.b is not None and a.b.dtype == torch.bfloat16
+              and _k().gemm_experts_takes(gate_up, act if glu_act or act == "relu2" else "silu") > 0 and _k().gemm_experts_takes(down) > 0)
+    if dev.type == "cuda" and T * k <= (EXPERT_GEMV_PAIRS if blocks else 4 * GEMV_MAX_M):
         kk = _k()
         flat = local.reshape(-1).contiguous()
         if gate_up.uses_q8_activations:
@@ -1157,7 +1187,6 @@ def moe_experts(a: Act, ids: torch.Tensor, weights: torch.Tensor, gate_up: Quant
         if down_scale is not None:
             wts = wts * down_scale[ids.reshape(-1).long()]
         if gate_up.uses_q8_activations:
-            blocks = a.b is not None and a.b.dtype == torch.bfloat16 and kk.gemm_experts_takes(gate_up, act) and kk.gemm_experts_takes(down)
             if not blocks:
                 _ensure_q8(a)
             return kk.moe_grouped(xq=a.q, xds=a.ds, xb=a.b.contiguous() if blocks else None, ids=ids, weights=wts, gate_up=gate_up, down=down, act=act,
@@ -1216,14 +1245,18 @@ def moe_tile_list(flat: torch.Tensor, n_groups: int, bn: int):
     return order, tiles.contiguous()
 
 
+@functools.lru_cache(maxsize=1024)
 def _pair_tile(avg: int) -> int:
-    """Token tile of the grouped pair GEMM for groups of ``avg`` rows: the cost per useful row, from the kernel's cost of a tile
-    (csrc/gemm_tcgen05.cu: gemm_cost) and half an empty tile per group.
-    Measured, both products of an expert layer (us; the chosen tile / 128 / 256 rows): 32 experts of 2 x 2880 x 2880, groups of 70
-    rows 307 / 293 / 414, of 128 340 / 385 / 455, of 512 1031 / 1119 / 987; 128 of 2 x 512 x 2048, groups of 70 214 / 214 / 188, of 128
-    209 / 247 / 211, of 1024 1027 / 1229 / 1112."""
+    """Token tile of the grouped pair GEMM for groups of ``avg`` rows: the kernel's cost of a tile (csrc/gemm_tcgen05.cu: gemm_cost) times the
+    expected number of tiles of a group whose size spreads about the average by 1.8 times its root (what softmax routers of random rows show:
+    groups of 72 rows 11, 128 17, 256 30, 800 59).
+    Measured, a prompt through the layers around them (ms; the tile that half an empty tile per group would choose / this one): 256 experts of 2 x
+    512 x 2048, groups of 72 rows 3.85 / 3.68, of 128 5.50 / 5.37, of 256 9.96 / 9.81; 32 of 2 x 2880 x 2880, of 250 3.14 / 2.85, of 800 6.86 / 6.86."""
+    sd = 1.8 * math.sqrt(avg)
+
     def cost(bn):
-        return max(2.0 * bn, (128 + bn / 2) * 128 / 70) / bn * (1 + bn / (2 * avg))
+        tiles = sum(0.5 * math.erfc((j * bn - avg) / (sd * math.sqrt(2.0))) for j in range(1 + int((avg + 4 * sd) / bn)))
+        return max(2.0 * bn, (128 + bn / 2) * 128 / 70) * tiles
     return min(range(80, 257, 16), key=cost)
 
 

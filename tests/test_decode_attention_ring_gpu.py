@@ -33,9 +33,9 @@ def want(q, k, v, table, lens, page, scale, window, sinks, softcap):
 @pytest.mark.parametrize("Hq,Hkv,Dh", [(32, 8, 128), (64, 8, 64), (4, 4, 128), (16, 1, 64)])
 @pytest.mark.parametrize("page", [16, 64])
 @pytest.mark.parametrize("window,sink,softcap", [(0, False, 0.0), (50, True, 0.0), (128, False, 20.0)])
-@pytest.mark.parametrize("splits,split_len", [(1, 0), (3, 0), (5, 64)])
+@pytest.mark.parametrize("splits,split_len", [(1, 0), (3, 0), (5, 64), (7, -128)])
 def test_against_plain_attention(Hq, Hkv, Dh, page, window, sink, softcap, splits, split_len):
-    if window and split_len:
+    if window and split_len > 0:
         pytest.skip("a fixed split length goes with no window")
     torch.manual_seed(1)
     lens = [1, 15, 16, 17, 64, 65, 129, 300]
@@ -55,3 +55,14 @@ def test_against_plain_attention(Hq, Hkv, Dh, page, window, sink, softcap, split
     assert ((got.double() - ref).norm() / ref.norm()).item() < 5e-3
     back = gq.view(B, -1, 32).double() * gds.view(B, -1, 2)[..., :1].double()
     assert ((back.view_as(ref) - got.double()).norm() / ref.norm()).item() < 1e-2            # 8 bits of a group's largest value
+
+
+def test_a_sequence_is_cut_alike_whatever_the_bucket():
+    """A captured step has splits for its bucket, an eager one for the longest sequence: the same parts, the same bits."""
+    torch.manual_seed(2)
+    lens, page, Hq, Hkv, Dh = [70, 300, 129], 64, 8, 2, 128
+    table = torch.arange(15, device=DEV).int().view(3, 5)
+    k, v = (torch.randn(15 * page, Hkv, Dh, device=DEV).bfloat16() for _ in range(2))
+    q, kl = torch.randn(3, Hq, Dh, device=DEV).bfloat16(), torch.tensor(lens, dtype=torch.int32, device=DEV)
+    a, b = (K().attn_decode(q, k, v, table, kl, scale=0.1, Hq=Hq, Hkv=Hkv, Dh=Dh, page_size=page, splits=s, split_len=-128) for s in (3, 8))
+    assert torch.equal(a, b)
