@@ -203,17 +203,6 @@ __global__ void __launch_bounds__(128) gemv_split_kernel(GemvArgs a) {
 // because their quantisation types differ) in one launch: the rows of all matrices form one row
 // space, a warp looks up which matrix its row belongs to, and the results land side by side in one
 // [M, N0 + N1 + N2] output.  Saves two launches per layer in the latency-bound decode step.
-struct GemvMultiArgs {
-    QW w[3];
-    int n_w;
-    int row_end[3];          // cumulative row counts
-    const int8_t* xq;
-    const float2* xds;
-    const bf16* xb;
-    void* out;
-    int M, out_f32, n_total;
-};
-
 template <int M>
 __global__ void __launch_bounds__(128) gemv_multi_kernel(GemvMultiArgs a) {
     const int lane = threadIdx.x & 31;
@@ -283,6 +272,8 @@ extern "C" int tsb_quantize_q8(const void* x, int x_is_f32, void* xq, void* xds,
 
 bool tsb_gemv_stream_eligible(const GemvArgs& a);                     // gemv_stream.cu
 int tsb_gemv_stream_launch(const GemvArgs& a, bool glu, cudaStream_t s);
+bool tsb_gemv_rows_multi_eligible(const GemvMultiArgs& m);
+int tsb_gemv_rows_multi_launch(const GemvMultiArgs& m, cudaStream_t s);
 bool tsb_gemv_mma_eligible(const GemvArgs& a);                        // gemv_mma.cu
 int tsb_gemv_mma_launch(const GemvArgs& a, bool glu, cudaStream_t s);
 bool tsb_gemv_bf16_eligible(const GemvArgs& a);                       // gemv_bf16.cu
@@ -406,6 +397,7 @@ extern "C" int tsb_gemv_multi(const void* const* planes, const int* types, const
     a.M = M; a.out_f32 = out_f32; a.n_total = total;
     dim3 block(128);
     cudaStream_t s = (cudaStream_t)stream;
+    if (tsb_gemv_rows_multi_eligible(a)) return tsb_gemv_rows_multi_launch(a, s);
     if (M <= 1) TSB_CHECK_CUDA(tsb_launch(gemv_multi_kernel<1>, dim3((total + 3) / 4, 1), block, 0, s, a));
     else if (M <= 2) TSB_CHECK_CUDA(tsb_launch(gemv_multi_kernel<2>, dim3((total + 3) / 4, 1), block, 0, s, a));
     else if (M <= 4) TSB_CHECK_CUDA(tsb_launch(gemv_multi_kernel<4>, dim3((total + 3) / 4, 1), block, 0, s, a));

@@ -30,6 +30,17 @@ struct GemvArgs {
     int n_first = 0;
 };
 
+struct GemvMultiArgs {
+    QW w[3];
+    int n_w;
+    int row_end[3];          // cumulative row counts
+    const int8_t* xq;
+    const float2* xds;
+    const bf16* xb;
+    void* out;
+    int M, out_f32, n_total;
+};
+
 // Each quantised type is split into a weight *load* (global, streaming, independent of the
 // activations) and a *compute* step, so that a lane can have the loads of two units in
 // flight before it touches either, and so that the first loads can be issued before the
