@@ -128,7 +128,7 @@ __global__ void __launch_bounds__(128) gemv_stream_kernel(GemvArgs a, int ppw) {
 }
 
 // ---------------------------------------------------------------------------------------------
-// Single-token Q4_K and Q6_K: rows of a matrix in groups of R, 32 / R lanes to a row.
+// Single-token Q4_K, Q6_K and Q8_0: rows of a matrix in groups of R, 32 / R lanes to a row.
 //
 // At one activation row the bound is the bytes of the weights, and what kept the kernel from it was the
 // instruction issue: with a row per warp and units of 32 values the Q4_K form spent 4.2 thread instructions
@@ -147,7 +147,8 @@ __global__ void __launch_bounds__(128) gemv_stream_kernel(GemvArgs a, int ppw) {
 // when the kernel starts.  KS = 4 (rows longer than 6144 values): the four warps of a CTA split every row by
 // blocks and the partial sums meet in shared memory, one barrier per group.
 // Measured (us, weights of several matrices in turn, before / after): 2 x 9728 x 2560 10.5 / 6.8, 2560 x 9728 7.3 / 4.7, Q6_K 7.3 / 6.3, 32768 x 2560
-// Q6_K 24.0 / 13.4 (5.2 TB/s), 151936 x 2560 64.9 / 37.5, Q6_K 100 / 59.  What is left of the short ones is latency: activations through L2 after the
+// Q6_K 24.0 / 13.4 (5.2 TB/s), 151936 x 2560 64.9 / 36.5, Q6_K 100 / 56; Q8_0, which has little to decode but kept two 16-byte loads a lane in flight:
+// 2 x 21504 x 5376 44.7 / 40.1 (6.1 TB/s), 5376 x 21504 27.4 / 20.4, 5376 x 4096 7.0 / 5.3, 8192 x 5376 11.7 / 8.3.  What is left of the short ones is latency: activations through L2 after the
 // wait, one group's arithmetic, the tail.  Three stages or two CTAs an SM measured slower, 128 registers (four CTAs) too: the units no longer overlap.
 // ---------------------------------------------------------------------------------------------
 __device__ __forceinline__ int dp4a_us(unsigned a, int b, int c) {      // unsigned bytes of a times signed bytes of b
@@ -157,13 +158,15 @@ __device__ __forceinline__ int dp4a_us(unsigned a, int b, int c) {      // unsig
 }
 constexpr int MAGIC_I = 0x4B400000;                                      // as a float 1.5 * 2^23: integers below 2^22 in magnitude added to these bits
 constexpr float MAGIC_F = 12582912.f;                                    // are read back by one float subtraction
+enum { ROWS_Q4, ROWS_Q6, ROWS_Q8 };
+__host__ __device__ constexpr int rows_block_bytes(int ty) { return ty == ROWS_Q4 ? 144 : ty == ROWS_Q6 ? 210 : 272; }
 constexpr int ROWS_D = 2, ROWS_PER_SM = 3;                             // stages of a warp, CTAs of an SM
 
 // Blocks [first, end) of a row that a warp owns; even boundaries keep the 2-byte super-scales of Q6_K 4-byte aligned for cp.async
-template <bool Q6, int KS>
+template <int TY, int KS>
 __host__ __device__ __forceinline__ int rows_slice(int nb, int warp) {
     if (KS == 1) return warp ? nb : 0;
-    return warp >= KS ? nb : Q6 ? ((nb * warp) / KS) & ~1 : (nb * warp) / KS;
+    return warp >= KS ? nb : TY == ROWS_Q6 ? ((nb * warp) / KS) & ~1 : (nb * warp) / KS;
 }
 
 // n chunks of 16 bytes (at most MOST, so that the loop unrolls to a compare and a copy each), lane by lane
@@ -174,13 +177,14 @@ __device__ __forceinline__ void rows_copy(uint8_t* dst, const uint8_t* src, int 
         if (lane + 32 * i < n) cp_async16(dst + 512 * i, src + 512 * i);
 }
 
-template <bool Q6, bool GLU, int R, int J, int KS>
+template <int TY, bool GLU, int R, int J, int KS>
 __device__ __forceinline__ void rows_body(const GemvArgs& a, uint8_t* rows_smem, int stage_bytes, int n_groups, int block, int blocks) {
     __shared__ float part[2][4][R];
+    constexpr bool Q4 = TY == ROWS_Q4, Q6 = TY == ROWS_Q6;
     constexpr int L = 32 / R, H = R / 2, D = ROWS_D;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int nb = a.w.K >> 8;
-    const int bs = rows_slice<Q6, KS>(nb, KS == 1 ? 0 : warp), nblk = rows_slice<Q6, KS>(nb, KS == 1 ? 1 : warp + 1) - bs;
+    const int bs = rows_slice<TY, KS>(nb, KS == 1 ? 0 : warp), nblk = rows_slice<TY, KS>(nb, KS == 1 ? 1 : warp + 1) - bs;
     uint8_t* ring = rows_smem + (long)warp * D * stage_bytes;
     const int n_out = a.n_out;
     const int owner = KS == 1 ? block * 4 + warp : block, owners = KS == 1 ? blocks * 4 : blocks;
@@ -189,16 +193,21 @@ __device__ __forceinline__ void rows_body(const GemvArgs& a, uint8_t* rows_smem,
     // n blocks (at most MOST) from block `sb` of the matrix to block `db` of a stage
     constexpr int MOST = (KS == 1 ? (GLU ? H : R) : 1) * (L / 4) * J;
     const int o_qh = R * nblk * 128, o_sc = R * nblk * 192, o_d = R * nblk * 208;
-    const int swz = lane ^ ((lane >> 2) & 2);                           // low nibbles of Q6_K: chunks 2 and 3 of four exchanged in odd blocks (bank conflicts)
+    // against bank conflicts: the low nibbles of Q6_K lie with chunks 2 and 3 of four exchanged in odd blocks, the bytes of Q8_0 with the four chunks of
+    // a unit permuted by the unit's number
+    const int swz = Q6 ? lane ^ ((lane >> 2) & 2) : lane ^ ((lane >> 3) & 3);
     auto copy = [&](uint8_t* st, int db, long sb, int n) {
-        if (!Q6) {
+        if (Q4) {
             rows_copy<MOST * 9>(st + (db * 9 + lane) * 16, a.w.p0 + sb * 144 + lane * 16, n * 9, lane);
-        } else {
+        } else if (Q6) {
             rows_copy<MOST * 8>(st + (db * 8 + swz) * 16, a.w.p0 + sb * 128 + lane * 16, n * 8, lane);
             rows_copy<MOST * 4>(st + o_qh + (db * 4 + lane) * 16, a.w.p1 + sb * 64 + lane * 16, n * 4, lane);
             rows_copy<MOST>(st + o_sc + (db + lane) * 16, a.w.p2 + sb * 16 + lane * 16, n, lane);
             static_assert(MOST <= 64, "one word of super-scales a lane");
             if (lane < n / 2) cp_async4(st + o_d + db * 2 + lane * 4, a.w.p3 + sb * 2 + lane * 4);
+        } else {
+            rows_copy<MOST * 16>(st + (db * 16 + swz) * 16, a.w.p0 + sb * 256 + lane * 16, n * 16, lane);
+            rows_copy<MOST>(st + R * nblk * 256 + (db + lane) * 16, a.w.p1 + sb * 16 + lane * 16, n, lane);
         }
     };
     auto issue = [&](int t, int slot) {
@@ -265,8 +274,10 @@ __device__ __forceinline__ void rows_body(const GemvArgs& a, uint8_t* rows_smem,
     const uint32_t m_lo = hi ? 0x0F0Fu : 0x3F3Fu, m_hi = hi ? 0x3030u : 0u;
     const unsigned shq = sh + (hi ? 4u : 0u);
     const uint32_t sel0 = 0x7540u | hb, sel1 = 0x7542u | hb;             // Q6_K: bytes hb and hb + 2 of a word of scales
-    const int off0 = Q6 ? (i_row * nblk + bl0) * 128 + (((4 * (c4 >> 1) + hb) ^ (2 * (bl0 & 1))) << 4) : (i_row * nblk + bl0) * 144;
+    const int xr = ((l >> 1) + (KS == 1 ? 2 * ((GLU ? i_row % H : i_row) * nblk & 1) : 0)) & 3;   // Q8_0: what permutes the chunks of a lane's units (copies count rows of a run on)
+    const int off0 = !Q4 && !Q6 ? (i_row * nblk + bl0) * 256 + 64 * c4 : Q6 ? (i_row * nblk + bl0) * 128 + (((4 * (c4 >> 1) + hb) ^ (2 * (bl0 & 1))) << 4) : (i_row * nblk + bl0) * 144;
     const int off1 = Q6 ? off0 ^ 32 : off0 + 16 + 32 * c4;
+    const int off5 = R * nblk * 256 + (i_row * nblk + bl0) * 16 + 4 * c4;
     const int off2 = o_qh + (i_row * nblk + bl0) * 64 + 16 * c4, off3 = o_sc + (i_row * nblk + bl0) * 16 + 8 * (c4 >> 1), off4 = o_d + (i_row * nblk + bl0) * 2;
 
     int slot = 0, next = D - 1;
@@ -309,6 +320,18 @@ __device__ __forceinline__ void rows_body(const GemvArgs& a, uint8_t* rows_smem,
 #pragma unroll
                 for (int k = 0; k < 4; ++k) v += (__int_as_float(s[k]) - MAGIC_F) * (__uint_as_float(sb[k]) - 8388736.f) * f[j][k];
                 acc += d * v;
+            } else if (!Q4) {
+                int s[2] = {MAGIC_I, MAGIC_I};
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const uint4 q = *reinterpret_cast<const uint4*>(st + off0 + bj * 256 + ((k ^ xr) << 4));
+                    s[k >> 1] = __dp4a((int)q.x, x[j][4 * k], s[k >> 1]);
+                    s[k >> 1] = __dp4a((int)q.y, x[j][4 * k + 1], s[k >> 1]);
+                    s[k >> 1] = __dp4a((int)q.z, x[j][4 * k + 2], s[k >> 1]);
+                    s[k >> 1] = __dp4a((int)q.w, x[j][4 * k + 3], s[k >> 1]);
+                }
+                const float2 dd = __half22float2(*reinterpret_cast<const __half2*>(st + off5 + bj * 16));
+                acc += dd.x * f[j][0] * (__int_as_float(s[0]) - MAGIC_F) + dd.y * f[j][1] * (__int_as_float(s[1]) - MAGIC_F);
             } else {
                 const uint4 hdr = *reinterpret_cast<const uint4*>(st + off0 + bj * 144);
                 const uint4 qa = *reinterpret_cast<const uint4*>(st + off1 + bj * 144), qb = *reinterpret_cast<const uint4*>(st + off1 + bj * 144 + 16);
@@ -374,10 +397,10 @@ __device__ __forceinline__ void rows_body(const GemvArgs& a, uint8_t* rows_smem,
 }
 
 
-template <bool Q6, bool GLU, int R, int J, int KS>
+template <int TY, bool GLU, int R, int J, int KS>
 __global__ void __launch_bounds__(128, ROWS_PER_SM) gemv_rows_kernel(GemvArgs a, int stage_bytes, int n_groups) {
     extern __shared__ __align__(128) uint8_t rows_smem[];
-    rows_body<Q6, GLU, R, J, KS>(a, rows_smem, stage_bytes, n_groups, blockIdx.x, gridDim.x);
+    rows_body<TY, GLU, R, J, KS>(a, rows_smem, stage_bytes, n_groups, blockIdx.x, gridDim.x);
 }
 
 // Two or three matrices over the same activations (query, key and value rows of mixed types): each has the CTAs that its share of the bytes asks for.
@@ -392,8 +415,8 @@ __global__ void __launch_bounds__(128, ROWS_PER_SM) gemv_rows_multi_kernel(GemvM
     a.xq = m.xq; a.xds = m.xds; a.M = 1; a.out_f32 = m.out_f32; a.n_out = a.w.N;
     a.out = m.out_f32 ? (void*)(reinterpret_cast<float*>(m.out) + row0) : (void*)(reinterpret_cast<bf16*>(m.out) + row0);
     const int n_groups = (a.n_out + 1) / 2;
-    if (a.w.type == TSB_Q6_K) rows_body<true, false, 2, J, 1>(a, rows_smem, stage_bytes, n_groups, b - first, blocks);
-    else rows_body<false, false, 2, J, 1>(a, rows_smem, stage_bytes, n_groups, b - first, blocks);
+    if (a.w.type == TSB_Q6_K) rows_body<ROWS_Q6, false, 2, J, 1>(a, rows_smem, stage_bytes, n_groups, b - first, blocks);
+    else rows_body<ROWS_Q4, false, 2, J, 1>(a, rows_smem, stage_bytes, n_groups, b - first, blocks);
 }
 
 template <int J>
@@ -415,20 +438,20 @@ static int launch_rows_multi(const GemvMultiArgs& m, cudaStream_t s) {
     return TSB_OK;
 }
 
-template <bool Q6, bool GLU, int R, int J, int KS>
+template <int TY, bool GLU, int R, int J, int KS>
 static int launch_rows(const GemvArgs& a, int max_blocks, cudaStream_t s) {
     static bool attr = false;
     if (!attr) {
-        TSB_CHECK_CUDA(cudaFuncSetAttribute(gemv_rows_kernel<Q6, GLU, R, J, KS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+        TSB_CHECK_CUDA(cudaFuncSetAttribute(gemv_rows_kernel<TY, GLU, R, J, KS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
         attr = true;
     }
-    const int stage = R * max_blocks * (Q6 ? 210 : 144), stage_bytes = (stage + 127) & ~127;
+    const int stage = R * max_blocks * rows_block_bytes(TY), stage_bytes = (stage + 127) & ~127;
     const size_t smem = (size_t)stage_bytes * ROWS_D * 4;
     const int n_groups = (a.n_out + (GLU ? R / 2 : R) - 1) / (GLU ? R / 2 : R);
     const int fit = (int)((226 * 1024) / (smem + 1024)), most = 148 * (fit < 1 ? 1 : fit > ROWS_PER_SM ? ROWS_PER_SM : fit);
     // fewer groups than warps: every SM takes its share all the same, a warp without a group ends at once
     const int need = KS == 1 ? (n_groups + 3) / 4 : n_groups, ctas = need < (KS == 1 ? 148 : most) ? need : most;
-    TSB_CHECK_CUDA(tsb_launch(gemv_rows_kernel<Q6, GLU, R, J, KS>, dim3(ctas), dim3(128), smem, s, a, stage_bytes, n_groups));
+    TSB_CHECK_CUDA(tsb_launch(gemv_rows_kernel<TY, GLU, R, J, KS>, dim3(ctas), dim3(128), smem, s, a, stage_bytes, n_groups));
     TSB_CHECK_LAUNCH();
     return TSB_OK;
 }
@@ -436,10 +459,10 @@ static int launch_rows(const GemvArgs& a, int max_blocks, cudaStream_t s) {
 // Four rows to a warp where that leaves every warp a group (and a lane's activations, 16 registers a unit, stay at six units), two otherwise:
 // 2 x 9728 x 2560 6.8 us with four rows and 7.4 with two, 32768 x 2560 of Q6_K 13.4 and 14.2; 6144 x 2560 4.2 and 3.6, 2560 x 9728 5.5 and 4.7 (Q6_K
 // 7.5 and 6.3).  Rows longer than 6144 values are split over the CTA.
-template <bool Q6, bool GLU>
+template <int TY, bool GLU>
 static int launch_rows_any(const GemvArgs& a, cudaStream_t s) {
     const int nb = a.w.K >> 8;
-#define TSB_ROWS(RV, JV, KSV) return launch_rows<Q6, GLU, RV, JV, KSV>(a, mb, s)
+#define TSB_ROWS(RV, JV, KSV) return launch_rows<TY, GLU, RV, JV, KSV>(a, mb, s)
     if (nb <= 24) {
         const int mb = nb;
         if (nb <= 12 && a.w.N >= 148 * ROWS_PER_SM * 4 * 4) {
@@ -462,11 +485,13 @@ static int launch_rows_any(const GemvArgs& a, cudaStream_t s) {
         }
     }
     int mb = 0;
-    for (int w = 0; w < 4; ++w) mb = max(mb, rows_slice<Q6, 4>(nb, w + 1) - rows_slice<Q6, 4>(nb, w));
-    switch ((mb + 3) / 4) {                                              // slices of 7 to 16 blocks
+    for (int w = 0; w < 4; ++w) mb = max(mb, rows_slice<TY, 4>(nb, w + 1) - rows_slice<TY, 4>(nb, w));
+    switch ((mb + 3) / 4) {                                              // slices of 7 to 16 blocks, of Q8_0 to 24
     case 2: TSB_ROWS(2, 2, 4);
     case 3: TSB_ROWS(2, 3, 4);
-    default: TSB_ROWS(2, 4, 4);
+    case 4: TSB_ROWS(2, 4, 4);
+    case 5: TSB_ROWS(2, 5, 4);
+    default: TSB_ROWS(2, 6, 4);
     }
 #undef TSB_ROWS
 }
@@ -490,9 +515,8 @@ static int launch_stream_m(const GemvArgs& a, int ppw, int ctas, size_t smem, cu
     return launch_stream<4, GLU, Q5, D>(a, ppw, ctas, smem, s);
 }
 
-// Whether the row pipeline takes this GEMV (called by tsb_gemv_push before the plain launch).  By default
-// only the single-token Q4_K form runs here; the generic form (M <= 4, Q5_K, any row length) measured
-// slower than the plain kernel inside the decode step and is kept behind TSB_GEMV_STREAM=2.
+// Whether the row pipeline takes this GEMV (called by tsb_gemv_push before the plain launch): the single-token forms above.  The generic form
+// (M <= 4, Q5_K, any row length) measured slower than the plain kernel inside the decode step and is kept behind TSB_GEMV_STREAM=2.
 // TSB_GEMV_STREAM=0 turns the pipeline off altogether.
 static int stream_mode() {
     static const int mode = []() { const char* e = getenv("TSB_GEMV_STREAM"); return e ? atoi(e) : 1; }();
@@ -502,6 +526,11 @@ static int stream_mode() {
 static bool q6k_ok(const GemvArgs& a, bool glu) {
     const int nb = a.w.K >> 8;
     return a.w.type == TSB_Q6_K && !glu && a.M == 1 && nb >= 2 && nb % 2 == 0 && nb <= 64 && a.w.N >= 64;
+}
+
+static bool q8_ok(const GemvArgs& a) {
+    return a.w.type == TSB_Q8_0 && a.M == 1 && a.w.K % 256 == 0 && a.w.K <= 96 * 256 && a.w.N >= 64 &&
+           ((reinterpret_cast<uintptr_t>(a.w.p0) | reinterpret_cast<uintptr_t>(a.w.p1)) & 15) == 0;
 }
 
 static bool fast_ok(const GemvArgs& a) {
@@ -532,7 +561,7 @@ bool tsb_gemv_stream_eligible(const GemvArgs& a) {
     const int mode = stream_mode();
     if (!mode || a.ids || a.M > 4 || a.M < 1) return false;
     const bool glu = a.act >= ACT_SWIGLU && a.act <= ACT_SWIGLU_OAI;
-    if (fast_ok(a) && !(glu && a.push)) return true;
+    if ((fast_ok(a) || q8_ok(a)) && !(glu && a.push)) return true;
     if (q6k_ok(a, glu)) return true;
     if (a.push || mode < 2 || (a.w.type != TSB_Q4_K && a.w.type != TSB_Q5_K)) return false;
     const size_t rowbytes = (size_t)(a.w.K >> 8) * (a.w.type == TSB_Q5_K ? 176 : 144);
@@ -540,8 +569,9 @@ bool tsb_gemv_stream_eligible(const GemvArgs& a) {
 }
 
 int tsb_gemv_stream_launch(const GemvArgs& a, bool glu, cudaStream_t s) {
-    if (fast_ok(a)) return glu ? launch_rows_any<false, true>(a, s) : launch_rows_any<false, false>(a, s);
-    if (q6k_ok(a, glu)) return launch_rows_any<true, false>(a, s);
+    if (fast_ok(a)) return glu ? launch_rows_any<ROWS_Q4, true>(a, s) : launch_rows_any<ROWS_Q4, false>(a, s);
+    if (q8_ok(a)) return glu ? launch_rows_any<ROWS_Q8, true>(a, s) : launch_rows_any<ROWS_Q8, false>(a, s);
+    if (q6k_ok(a, glu)) return launch_rows_any<ROWS_Q6, false>(a, s);
     const bool q5 = a.w.type == TSB_Q5_K;
     const size_t rowbytes = (size_t)(a.w.K >> 8) * (q5 ? 176 : 144);
     const size_t smem = rowbytes * 4 * 4;

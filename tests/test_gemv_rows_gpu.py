@@ -1,4 +1,4 @@
-"""Single-token products of Q4_K and Q6_K rows in groups (csrc/gemv_stream.cu), against the decoded weights in double precision."""
+"""Single-token products of Q4_K, Q6_K and Q8_0 rows in groups (csrc/gemv_stream.cu), against the decoded weights in double precision."""
 import pytest
 import torch
 
@@ -11,11 +11,11 @@ DEV = "cuda:0"
 
 # The activations are whole numbers up to 127 with a 127 in every group of 32 (times a power of two), which int8 groups hold exactly: what
 # is left is the rounding of float sums, at most some 300 additions of terms as large as the result's parts (1e-5 with room).
-@pytest.mark.parametrize("t", [GGMLType.Q4_K, GGMLType.Q6_K])
-@pytest.mark.parametrize("blocks", [1, 2, 3, 6, 10, 11, 12, 13, 16, 18, 24, 25, 26, 30, 38, 46, 50, 56, 64])
+@pytest.mark.parametrize("t", [GGMLType.Q4_K, GGMLType.Q6_K, GGMLType.Q8_0])
+@pytest.mark.parametrize("blocks", [1, 2, 3, 6, 10, 11, 12, 13, 16, 18, 24, 25, 26, 30, 38, 46, 50, 56, 64, 84, 93, 96])
 @pytest.mark.parametrize("N,kind", [(64, "plain"), (67, "joined"), (2370, "joined"), (2372, "gated"), (130, "gated")])
 def test_rows_of_every_length(t, blocks, N, kind):
-    if t == GGMLType.Q6_K and (blocks % 2 or kind == "gated"):
+    if t == GGMLType.Q6_K and (blocks % 2 or kind == "gated") or t != GGMLType.Q8_0 and blocks > 64:
         pytest.skip("the general kernels' form")
     from tensorsharp_b200.ops import kernels as k
     torch.manual_seed(blocks * 7 + N)
