@@ -353,7 +353,7 @@ __global__ void __launch_bounds__(128) attn_decode_ring_kernel(AttnArgs a) {
     const int len = a.kv_lens[b];
     const int lo = (a.window > 0 && len > a.window) ? len - a.window : 0;
     const int span = len - lo;
-    const int per = a.split_len > 0 ? a.split_len : max((((span + a.splits - 1) / a.splits) + 31) & ~31, -a.split_len);
+    const int per = a.split_len > 0 ? a.split_len : max((((span + a.splits - 1) / a.splits) + 63) & ~63, -a.split_len);      // whole rounds of the four warps
     const int s0 = lo + split * per, s1 = min(len, s0 + per), w0 = (s0 & ~(KT - 1)) + warp * KT;      // this warp's first chunk
     const int n = max(0, (s1 - w0 + 4 * KT - 1) / (4 * KT));                // and how many it has
     const int* table = a.block_table + (long)b * a.max_pages;

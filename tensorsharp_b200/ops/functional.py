@@ -673,13 +673,14 @@ def ring_attention(Hq: int, Hkv: int, Dh: int, page_size: int, fp8: bool) -> boo
 def decode_splits(batch: Batch, Hkv: int, window: int, ring: bool = False) -> int:
     """Split-KV factor for decode attention: enough CTAs to cover the GPU's 148 SMs.  ``ring``: the kernel that loads ahead, two CTAs an SM and
     no more (with the merge, us for 1 / 2 / 3 / 4 / 9 splits: 16 sequences of about 1600 40.9 / 26.3 / 27.1 / 26.0 / 30.2, 32 46.3 / 42.8 / 45.6 / 47.8;
-    64 of about 800 29.7 / 31.4 / 33.2; 4 of about 3300 for 4 / 9 / 13 / 18 / 37 21.3 / 16.0 / 18.8 / 19.1 / 23.8)."""
+    64 of about 800 29.7 / 31.4 / 33.2; 4 of about 3300 for 4 / 9 / 13 / 18 / 37 21.3 / 16.0 / 18.8 / 19.1 / 23.8); one sequence no more than the
+    merge fetches at once (8111 positions in 37 / 32 splits: 13.0 / 11.6 us with it)."""
     span = batch.max_kv_len if not window else min(batch.max_kv_len, window)
     # one sequence: about two CTAs per SM; batches: up to eight (a CTA is 128 threads and latency-bound, and with 16
     # sequences two splits per (sequence, KV head) left the kernel at a fifth of the memory rate)
     want = max(1, (148 * (2 if batch.B == 1 else 8)) // max(1, batch.B * Hkv))
-    if ring and batch.B > 1:
-        want = -(-296 // (batch.B * Hkv))
+    if ring:
+        want = -(-296 // (batch.B * Hkv)) if batch.B > 1 else min(want, 32)
     per = _split_positions()
     n = int(max(1, min(want, (span + per - 1) // per, 64)))
     # TSB_ATTN_CLUSTER=1: 8 or 16 splits are merged inside the attention kernel by a thread-block cluster (no combine
