@@ -297,15 +297,19 @@ __global__ void attn_combine_kernel(AttnArgs a) {
     const float2 ml0 = in0 ? *reinterpret_cast<const float2*>(a.part_ml + (base + lane) * 2) : make_float2(-INFINITY, 0.f);
     const float2 ml1 = in1 ? *reinterpret_cast<const float2*>(a.part_ml + (base + lane + 32) * 2) : make_float2(-INFINITY, 0.f);
     const float sink = a.sinks ? a.sinks[h] : -INFINITY;
+    const int dd = d < a.Dh ? d : 0;
+    float pv[32];                                       // asked for before the exchange below waits for the maxima
+#pragma unroll
+    for (int i = 0; i < 32; ++i) pv[i] = i < a.splits ? a.part_o[(base + i) * a.Dh + dd] : 0.f;
     const float mm = fmaxf(sink, warp_max(fmaxf(ml0.x, ml1.x)));
     const float c0 = (ml0.x == -INFINITY) ? 0.f : __expf(ml0.x - mm), c1 = (ml1.x == -INFINITY) ? 0.f : __expf(ml1.x - mm);
     const float ll = warp_sum(ml0.y * c0 + ml1.y * c1) + (a.sinks ? __expf(sink - mm) : 0.f);
     float o = 0.f;
-    const int dd = d < a.Dh ? d : 0;
     for (int s0 = 0; s0 < a.splits; s0 += 32) {
-        float pv[32];
+        if (s0 > 0) {
 #pragma unroll
-        for (int i = 0; i < 32; ++i) pv[i] = (s0 + i < a.splits) ? a.part_o[(base + s0 + i) * a.Dh + dd] : 0.f;
+            for (int i = 0; i < 32; ++i) pv[i] = (s0 + i < a.splits) ? a.part_o[(base + s0 + i) * a.Dh + dd] : 0.f;
+        }
 #pragma unroll
         for (int i = 0; i < 32; ++i) {
             const int sp = s0 + i;

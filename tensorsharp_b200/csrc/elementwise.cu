@@ -395,12 +395,14 @@ __device__ __forceinline__ void rope_lookup(const QkvArgs& a, int t, int pair, f
 // NJ = 32-element slices a lane holds (head size up to 32 * NJ): the loops below run NJ times, not 16.
 template <int NJ>
 __global__ void __launch_bounds__(128) qkv_rope_kernel(QkvArgs a) {
-    pdl_wait();
-    pdl_trigger();
     const int lane = threadIdx.x & 31;
     const long wid = (long)blockIdx.x * 4 + (threadIdx.x >> 5);
     const int H = a.Hq + 2 * a.Hkv;
-    if (wid >= (long)a.T * H) return;
+    if (wid >= (long)a.T * H) {
+        pdl_wait();
+        pdl_trigger();
+        return;
+    }
     const int t = (int)(wid / H), h = (int)(wid % H);
     const int Dh = h < a.Hq + a.Hkv ? a.Dh : a.Dv;
     const void* src;
@@ -409,8 +411,13 @@ __global__ void __launch_bounds__(128) qkv_rope_kernel(QkvArgs a) {
     if (h < a.Hq) { kind = 0; src = a.q; off = t * a.q_tok + h * a.q_head; }
     else if (h < a.Hq + a.Hkv) { kind = 1; src = a.k; off = t * a.k_tok + (h - a.Hq) * a.k_head; }
     else { kind = 2; src = a.v; off = t * a.v_tok + (h - a.Hq - a.Hkv) * a.v_head; }
-    const long slot = a.slot ? a.slot[t] : -1;
-    if (kind != 0 && slot < 0) return;
+    const float* nw = kind == 0 ? a.qn : (kind == 1 ? a.kn : nullptr);
+    float nwv[NJ];
+#pragma unroll
+    for (int j = 0; j < NJ; ++j) nwv[j] = (nw && lane + 32 * j < Dh) ? nw[lane + 32 * j] : 1.f;      // weights do not depend on the previous kernel
+    pdl_wait();
+    pdl_trigger();
+    const long slot = a.slot ? a.slot[t] : -1;                               // looked at when the inputs are on their way too
     // each lane holds up to NJ values: element e = lane + 32 * j
     float v[NJ];
     float ss = 0.f;
@@ -423,23 +430,21 @@ __global__ void __launch_bounds__(128) qkv_rope_kernel(QkvArgs a) {
         v[j] = x;
         ss += x * x;
     }
-    const float* nw = kind == 0 ? a.qn : (kind == 1 ? a.kn : nullptr);
-    // Everything else this warp will read (norm weights, cos / sin of its pairs) is requested here, next to
-    // the inputs, so the kernel is one memory round trip deep instead of three.
+    // Everything else this warp will read (cos / sin of its pairs; the norm weights before the wait) is requested here, next to the
+    // inputs, so the kernel is one memory round trip deep instead of three.
     const int rot = a.rp.rot_dim;
     const bool tab = a.cs_table != nullptr && kind != 2 && rot > 0;
-    float nwv[NJ];
     float2 csv[NJ];
 #pragma unroll
     for (int j = 0; j < NJ; ++j) {
         const int e = lane + 32 * j;
-        nwv[j] = (nw && e < Dh) ? nw[e] : 1.f;
         csv[j] = make_float2(1.f, 0.f);
         if (tab && e < rot) {
             const int pair = a.rp.mode == 0 ? (e < (rot >> 1) ? e : e - (rot >> 1)) : (e >> 1);
             csv[j] = a.cs_table[(long)t * (rot >> 1) + pair];
         }
     }
+    if (kind != 0 && slot < 0) return;
     if (nw || (kind == 2 && a.v_norm)) {
         ss = warp_sum(ss);
         const float rs = rsqrtf(ss / (float)(kind == 2 ? Dh : a.norm_n) + a.eps);

@@ -133,7 +133,7 @@ class _GemmaBase(ModelBase):
         return y
 
     def _logits(self, h, batch: Batch) -> torch.Tensor:
-        last = h[batch.last_idx].contiguous()
+        last = F.last_rows(h, batch)
         a = F.norm(last, self.out_norm, self.cfg.eps, want_q8=True)
         logits = F.linear(a, self.lm_head, out_dtype=torch.float32)
         return F.softcap(logits, self.softcap)

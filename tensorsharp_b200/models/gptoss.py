@@ -149,7 +149,7 @@ class GptOssModel(ModelBase):
             a = tpx.reduce_norm(h, nxt, c.eps, norm=nxt is not None, parts=self.top_k)
         if not want_logits:
             return None
-        last = h[batch.last_idx].contiguous()
+        last = F.last_rows(h, batch)
         return F.linear(F.norm(last, self.out_norm, c.eps, want_q8=True), self.lm_head, out_dtype=torch.float32)
 
     def forward_seq_parallel(self, h_all: torch.Tensor, batch: Batch, want_logits: bool, sp) -> Optional[torch.Tensor]:
@@ -268,7 +268,7 @@ class GptOssModel(ModelBase):
             return None
         if not want_logits:
             return None
-        last = h if (not batch.is_decode and n_layers > 0) else h[batch.last_idx].contiguous()
+        last = h if (not batch.is_decode and n_layers > 0) else F.last_rows(h, batch)
         a = F.norm(last.contiguous(), self.out_norm, c.eps, want_q8=True)
         return F.linear(a, self.lm_head, out_dtype=torch.float32)
 

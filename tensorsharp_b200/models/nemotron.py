@@ -181,6 +181,6 @@ class NemotronHModel(ModelBase):
             h = h + y
         if self.stage_handoff(h) or not want_logits:
             return None
-        last = h[batch.last_idx].contiguous()
+        last = F.last_rows(h, batch)
         a = F.norm(last, self.out_norm, c.eps, want_q8=True)
         return F.linear(a, self.lm_head, out_dtype=torch.float32)

@@ -156,7 +156,7 @@ class Qwen3Model(ModelBase):
                 a = F.norm(h, nxt, c.eps, want_q8=small) if nxt is not None else None
         if not want_logits:
             return None
-        last = h[batch.last_idx].contiguous()
+        last = F.last_rows(h, batch)
         a = F.norm(last, self.out_norm, c.eps, want_q8=True)
         return self.lm_head_logits(a)
 
@@ -192,7 +192,7 @@ class Qwen3Model(ModelBase):
             return None
         if not want_logits:
             return None
-        last = h[batch.last_idx].contiguous()
+        last = F.last_rows(h, batch)
         return self.lm_head_logits(F.norm(last, self.out_norm, c.eps, want_q8=True))
 
     def forward_context_parallel(self, batch: Batch, want_logits: bool) -> Optional[torch.Tensor]:
@@ -306,7 +306,7 @@ class Qwen3Model(ModelBase):
                 F.linear_fused(gu, L["down"], residual=h, out=h)
         if not want_logits:
             return None
-        last = h if batch.last_idx.numel() == T else h[batch.last_idx].contiguous()
+        last = F.last_rows(h, batch)
         logits = F.linear_fused(last, self.lm_head, norm_w=self.out_norm, eps=c.eps, do_norm=True)
         if self.vocab_sharded:
             logits = self.comm.all_gather_cat(logits, dim=1)

@@ -196,6 +196,6 @@ class Qwen35Model(ModelBase):
             h = self._ffn(L, a, mid, h)
         if self.stage_handoff(h) or not want_logits:
             return None
-        last = h[batch.last_idx].contiguous()
+        last = F.last_rows(h, batch)
         a = F.norm(last, self.out_norm, c.eps, want_q8=True)
         return F.linear(a, self.lm_head, out_dtype=torch.float32)

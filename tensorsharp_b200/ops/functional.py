@@ -434,6 +434,12 @@ def _dequant_scratch(w: QuantWeight, holder: Optional[QuantWeight] = None, slot:
     return out
 
 
+def last_rows(h: torch.Tensor, batch: Batch) -> torch.Tensor:
+    """The row of every sequence's last token.  One row per sequence (every decode step) is what there is already: gathering it cost a
+    launch of 4.1 us a step, and one that cannot start ahead of its predecessor's end."""
+    return h if batch.last_idx.numel() == h.shape[0] else h[batch.last_idx].contiguous()
+
+
 def gemv_rows(w: QuantWeight, act: Optional[str] = None) -> int:
     """Most rows of bf16 activations for which a product goes to the GEMV kernels: two (one where the matrix is large) where the tensor cores
     take the weight as it is, which costs the same for one row as for sixteen.  Measured, us for 1 / 2 / 3 / 4 / 8 rows (GEMV; tensor cores):
