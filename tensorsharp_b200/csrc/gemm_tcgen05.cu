@@ -3,7 +3,7 @@
 //
 // The problem is run "weights as the M operand": each CTA owns 128 rows of W (output
 // features) and BN tokens, so that a small token count still fills the 128-lane MMA.  Up to 64
-// tokens (and the tensor-parallel forms) take the kernels below; plain and grouped products of more
+// tokens of bf16 weights (and the tensor-parallel forms) take the kernels below, GGUF blocks gemm_blocks.cu; plain and grouped products of more
 // run on pairs of CTAs (gemm_bf16_pair_kernel).
 //
 //   warp 0    : TMA producer - W and X tiles (64-element K slabs, 128-byte swizzle) into a

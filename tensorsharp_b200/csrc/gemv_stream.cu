@@ -456,7 +456,7 @@ static int launch_rows(const GemvArgs& a, int max_blocks, cudaStream_t s) {
     return TSB_OK;
 }
 
-// Four rows to a warp where that leaves every warp a group (and a lane's activations, 16 registers a unit, stay at six units), two otherwise:
+// Four rows to a warp where that leaves every warp a group of some length (and a lane's activations, 16 registers a unit, stay at six units), two otherwise:
 // 2 x 9728 x 2560 6.8 us with four rows and 7.4 with two, 32768 x 2560 of Q6_K 13.4 and 14.2; 6144 x 2560 4.2 and 3.6, 2560 x 9728 5.5 and 4.7 (Q6_K
 // 7.5 and 6.3).  Rows longer than 6144 values are split over the CTA.
 template <int TY, bool GLU>
@@ -465,10 +465,8 @@ static int launch_rows_any(const GemvArgs& a, cudaStream_t s) {
 #define TSB_ROWS(RV, JV, KSV) return launch_rows<TY, GLU, RV, JV, KSV>(a, mb, s)
     if (nb <= 24) {
         const int mb = nb;
-        if (nb <= 12 && a.w.N >= 148 * ROWS_PER_SM * 4 * 4) {
+        if (nb > 4 && nb <= 12 && a.w.N >= 148 * ROWS_PER_SM * 4 * 4) {
             switch ((mb + 1) / 2) {
-            case 1: TSB_ROWS(4, 1, 1);
-            case 2: TSB_ROWS(4, 2, 1);
             case 3: TSB_ROWS(4, 3, 1);
             case 4: TSB_ROWS(4, 4, 1);
             case 5: TSB_ROWS(4, 5, 1);
@@ -490,9 +488,13 @@ static int launch_rows_any(const GemvArgs& a, cudaStream_t s) {
     case 2: TSB_ROWS(2, 2, 4);
     case 3: TSB_ROWS(2, 3, 4);
     case 4: TSB_ROWS(2, 4, 4);
-    case 5: TSB_ROWS(2, 5, 4);
-    default: TSB_ROWS(2, 6, 4);
+    default: break;
     }
+    if constexpr (TY == ROWS_Q8) {
+        if ((mb + 3) / 4 == 5) TSB_ROWS(2, 5, 4);
+        TSB_ROWS(2, 6, 4);
+    }
+    return TSB_ERR_UNSUPPORTED;
 #undef TSB_ROWS
 }
 

@@ -944,6 +944,7 @@ __global__ void __launch_bounds__(128) gemv_tiles_mma_wide_kernel(TileArgs a) {
 // experts come from DRAM once, at a quarter of its rate.
 // Measured, 32 experts of 2880 x 2880, top 4 of 64 tokens, us per launch (8-byte-load version of the kernel above / this
 // one): gate and up 194 / 148, down 113 / 90 (four warps a CTA over the whole of K: 157 and 102).
+// MXFP4 shapes that gemm_blocks.cu takes go there (110 and 70 us); this kernel serves Q4_0 and the others.
 template <bool GLU, bool MX>
 struct RingSmem {
     static constexpr int S = GLU ? 2 : 1, STG = 3, SB = MX ? 1 : 2;     // weight row sets; ring stages; bytes of a block scale

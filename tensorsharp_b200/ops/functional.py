@@ -31,8 +31,9 @@ EXPERT_GEMV_PAIRS = 8
 PAIR_GEMM_MIN_M = 64  # above this many rows the tensor-core GEMM is the one that can end with the gated activation
 GATED_ACTS = ("swiglu", "geglu", "geglu_tanh", "geglu_erf", "swiglu_oai")
 GEMV_MAX_M = 16   # "small batch": token count up to which the models take their decode-style paths (int8 activations, mailbox exchanges)
-# Dense projections of 9 to 16 rows go to the tensor-core GEMM on the bf16 weight copy all the same: measured on the
-# Qwen3-4B shape at batch 16, 10.95 ms per step with the weight-streaming GEMVs against 8.15 ms (TSB_GEMV_MAX_M moves it)
+# Dense projections of more rows than this go to the tensor cores all the same, from the blocks (csrc/gemm_blocks.cu) or, for types that it does not take,
+# from the bf16 copy: the Qwen3-4B shape at batch 16 took 10.95 ms a step with the weight-streaming GEMVs and 8.15 ms with copies (TSB_GEMV_MAX_M moves
+# it; gemv_rows below lowers it where the blocks are taken as they are)
 DENSE_GEMV_MAX_M = min(GEMV_MAX_M, int(os.environ.get("TSB_GEMV_MAX_M", "8")))
 
 
@@ -447,7 +448,8 @@ def gemv_rows(w: QuantWeight, act: Optional[str] = None) -> int:
     2560 10.9 / 23.3 / 30.1 / 31.6 / 18.7; 16.8; Q6_K 2560 x 9728 7.6 / 12.4 / 20.7 / 20.9 / 59.8; 11.5; Q8_0 5376 x 21504 26.9 / 29.5 / 43.8 / 44.0 / 90.2; 27; bf16 2880 x
     4096 7.5 / 9.0 / 12.8 / 12.8 / 21.8; 9.2, 32768 x 2880 29.8 / 36.2 / 56.4 / 58.0 / 102.8; 35."""
     from ..gguf.constants import GGMLType
-    if w.experts != 1:
+    if w.experts != 1 or (w.ggml_type == GGMLType.Q8_0 and w.N * w.K < 1 << 20):
+        # (512 x 1024 of Q8_0, 3 / 5 / 8 rows 3.1 / 3.8 / 4.1 us with the rows' quantisation, which a norm brings along; 3.5 on the tensor cores.  Q4_K 4.1 / 5.0 / 5.2)
         return DENSE_GEMV_MAX_M
     if w.ggml_type == GGMLType.BF16:
         return min(DENSE_GEMV_MAX_M, 2) if w.N * w.K >= 4 << 20 and w.K % 8 == 0 and w.planes[0].data_ptr() % 16 == 0 else DENSE_GEMV_MAX_M
@@ -1258,7 +1260,7 @@ def _pair_tile(avg: int) -> int:
     expected number of tiles of a group whose size spreads about the average by 1.8 times its root (what softmax routers of random rows show:
     groups of 72 rows 11, 128 17, 256 30, 800 59).
     Measured, a prompt through the layers around them (ms; the tile that half an empty tile per group would choose / this one): 256 experts of 2 x
-    512 x 2048, groups of 72 rows 3.85 / 3.68, of 128 5.50 / 5.37, of 256 9.96 / 9.81; 32 of 2 x 2880 x 2880, of 250 3.14 / 2.85, of 800 6.86 / 6.86."""
+    512 x 2048, groups of 72 rows 3.88 / 3.68, of 128 5.43 / 5.36, of 256 10.08 / 9.94; 32 of 2 x 2880 x 2880, of 250 3.14 / 2.85, of 800 6.86 / 6.86."""
     sd = 1.8 * math.sqrt(avg)
 
     def cost(bn):
