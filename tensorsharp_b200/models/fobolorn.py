@@ -166,7 +166,7 @@ class FobolornModel(FolderModel):
         c, n, dt = self.cfg, self.width, self.compute_dtype
         h = self.inject_pending_embeddings(F.embed(self.tok_emb, batch.tokens))
         want_logits = want_logits and batch.last_idx.numel() > 0
-        every_row = batch.is_decode and batch.last_idx.numel() == batch.T     # decode: all rows give logits, in their order
+        every_row = batch.is_decode and batch.rows_in_order     # decode: all rows give logits, in their order
 
         def seam(y, post, nxt):
             """Close a sublayer (``y`` through its post norm) and open the one at ``nxt``: (run, sublayer) or None."""

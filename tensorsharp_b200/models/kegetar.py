@@ -289,7 +289,7 @@ class KegetarModel(FolderModel):
             h = self.inject_pending_embeddings(h)
             x = h.to(x.dtype)
         want_logits = want_logits and batch.last_idx.numel() > 0
-        every_row = batch.is_decode and batch.last_idx.numel() == batch.T     # decode: all rows give logits, in their order
+        every_row = batch.is_decode and batch.rows_in_order     # decode: all rows give logits, in their order
         last = len(self.runs) - 1
         if last < 0:
             x = F.post_norm_seam(h, c.eps, n, pre=self.out_norm, dtype=dt)

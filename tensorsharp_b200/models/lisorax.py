@@ -245,7 +245,7 @@ class LisoraxModel(FolderModel):
         c, n, dt = self.cfg, self.width, self.compute_dtype
         h = self.inject_pending_embeddings(F.embed(self.tok_emb, batch.tokens, self.embed_scale))
         want_logits = want_logits and batch.last_idx.numel() > 0
-        every_row = batch.is_decode and batch.last_idx.numel() == batch.T     # decode: all rows give logits, in their order
+        every_row = batch.is_decode and batch.rows_in_order     # decode: all rows give logits, in their order
         y, parts, last = None, None, len(self.layers) - 1
         for i, L in enumerate(self.layers):
             h, v, x = F.conv_seam(h, c.eps, n, w=L["norm1"], y=y, parts=parts, taps=L["canon"], state=self.carried[i]["canon"], batch=batch,

@@ -218,7 +218,7 @@ class SogulixModel(FolderModel):
         c, n, D, dt = self.cfg, self.width, self.cfg.hidden, self.compute_dtype
         h = self.inject_pending_embeddings(F.embed(self.tok_emb, batch.tokens))
         want_logits = want_logits and batch.last_idx.numel() > 0
-        every_row = batch.is_decode and batch.last_idx.numel() == batch.T     # decode: all rows give logits, in their order
+        every_row = batch.is_decode and batch.rows_in_order     # decode: all rows give logits, in their order
         both = None                                     # [x | x0]: what enters a pass of the loop
         if self.loop_in is not None:
             both = torch.empty((batch.T, 2 * D), dtype=dt, device=h.device)

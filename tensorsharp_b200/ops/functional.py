@@ -89,6 +89,7 @@ class Batch:
     # table (logical page -> physical page of the ring).  None when the pool keeps every page of every layer.
     slots_w: Optional[torch.Tensor] = None
     block_table_w: Optional[torch.Tensor] = None
+    rows_in_order: bool = False   # last_idx counts 0 .. T - 1; said by whoever built the batch, as equal numbers of rows do not show it
 
     def windowed(self) -> "Batch":
         """The view of this batch that a sliding-window layer uses: the same tokens and lengths with the ring's slots
@@ -436,9 +437,9 @@ def _dequant_scratch(w: QuantWeight, holder: Optional[QuantWeight] = None, slot:
 
 
 def last_rows(h: torch.Tensor, batch: Batch) -> torch.Tensor:
-    """The row of every sequence's last token.  One row per sequence (every decode step) is what there is already: gathering it cost a
-    launch of 4.1 us a step, and one that cannot start ahead of its predecessor's end."""
-    return h if batch.last_idx.numel() == h.shape[0] else h[batch.last_idx].contiguous()
+    """The rows whose logits are wanted.  Where these are all rows in their order (every decode step) they are there already: gathering
+    them cost a launch of 4.1 us a step, and one that cannot start ahead of its predecessor's end."""
+    return h if batch.rows_in_order else h[batch.last_idx].contiguous()
 
 
 def gemv_rows(w: QuantWeight, act: Optional[str] = None) -> int:
