@@ -121,24 +121,6 @@ __device__ __forceinline__ uint64_t signed_bytes(uint32_t v, int i) {
                 pair(-12582912.f, -12582912.f));                                         // 2^23 + 2^22
 }
 
-// Bounded wait (some seconds) of a whole warp; IDLE: it has nothing else to do.
-template <bool IDLE = false>
-__device__ __forceinline__ bool hold(uint64_t* bar, uint32_t parity) {
-    uint32_t ok;
-    if (IDLE)
-        asm volatile("{\n\t.reg .pred p, q;\n\t.reg .u32 c;\n\tmov.u32 c, 0;\n\t"
-                     "POLL:\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t@p bra ENDED;\n\tnanosleep.u32 60;\n\t"
-                     "add.u32 c, c, 1;\n\tsetp.lt.u32 q, c, 40000000;\n\t@q bra POLL;\n\t"
-                     "ENDED:\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                     : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
-    else
-        asm volatile("{\n\t.reg .pred p, q;\n\t.reg .u32 c;\n\tmov.u32 c, 0;\n\t"
-                     "POLL:\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t@p bra ENDED;\n\t"
-                     "add.u32 c, c, 1;\n\tsetp.lt.u32 q, c, 40000000;\n\t@q bra POLL;\n\t"
-                     "ENDED:\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                     : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
-    return __all_sync(0xffffffffu, ok);
-}
 __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32]) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,"
                  "%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};"
@@ -426,10 +408,11 @@ __global__ void __launch_bounds__(BG_THREADS, 2) gemm_blocks_kernel(const __grid
             }
         }
         if (!ok && lane == 0) atomicExch(status, 1);
-        // no copy is in flight when the CTA leaves, whichever wait gave up
-        for (int i = max(0, it - stages); i < it; ++i) hold(&full[i % stages], (i / stages) & 1);
+        // no copy is in flight when the CTA leaves, whichever wait gave up (unless it takes longer than a wait's limit)
+        uint64_t until = 0;
+        for (int i = max(0, it - stages); i < it; ++i) settle(&full[i % stages], (i / stages) & 1, until);
         if (TYPE == TSB_MXFP4)
-            for (int i = max(0, j - 2); i < j; ++i) hold(&s_full[i & 1], (i >> 1) & 1);
+            for (int i = max(0, j - 2); i < j; ++i) settle(&s_full[i & 1], (i >> 1) & 1, until);
     } else if (warp == 2) {
         int it = 0, at = 0;
         uint32_t ph = 1;
@@ -450,7 +433,8 @@ __global__ void __launch_bounds__(BG_THREADS, 2) gemm_blocks_kernel(const __grid
             }
         }
         if (!ok && lane == 0) atomicExch(status, 1);
-        for (int i = max(0, it - XS); i < it; ++i) hold(&x_full[i % XS], (i / XS) & 1);
+        uint64_t until = 0;
+        for (int i = max(0, it - XS); i < it; ++i) settle(&x_full[i % XS], (i / XS) & 1, until);
     } else if (warp == 1) {
         constexpr uint32_t idesc = make_idesc_bf16(128, NT);
         const uint64_t dx = make_desc_sw128(smem_u32(sX));
