@@ -710,9 +710,12 @@ __global__ void __launch_bounds__(512) gdn_chunk_scan_kernel(GdnPrepArgs a) {
         }
         __syncthreads();
     }
-    if (c < nc && threadIdx.x == 0) {      // a wait gave up: leave with no copy in flight
-        atomicExch(a.status, 6);
-        if (c + 1 < nc) tc::mbar_wait(&full[(c + 1) & 1], ((c + 1) >> 1) & 1);
+    if (c < nc && threadIdx.x == 0) {      // a wait gave up: this chunk's copies and the next one's may be on their way, and land before the CTA leaves
+        atomicExch(a.status, 6);           // (unless that takes longer than a wait's limit)
+        uint64_t until = 0;
+        tc::settle(&full[c & 1], (c >> 1) & 1, until);
+        tc::settle(&full[2], c & 1, until);
+        if (c + 1 < nc) tc::settle(&full[(c + 1) & 1], ((c + 1) >> 1) & 1, until);
     }
     if (keys) {
 #pragma unroll
