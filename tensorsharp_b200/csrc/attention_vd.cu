@@ -513,7 +513,7 @@ static int dispatch_vd(const AttnArgs& in, int max_q, cudaStream_t s) {
     TSB_CHECK_ARG(a.keep_first >= 0 && (a.keep_first == 0 || a.window > 0), "attention: kept first positions without a window");
     TSB_CHECK_ARG(a.sig_bias == nullptr || (a.sinks == nullptr && a.lse_out == nullptr), "attention: sigmoid weights have no sink and no log-sum-exp");
     TSB_CHECK_ARG((a.log_r1 == nullptr) == (a.log_r2 == nullptr), "attention: a logarithmic distance bias has two numbers per head");
-    TSB_CHECK_ARG(a.split_len == 0 || a.window <= 0, "attention: fixed splits with a window");
+    TSB_CHECK_ARG(a.split_len <= 0 || a.window <= 0, "attention: fixed splits with a window");
     TSB_CHECK_ARG(a.k_ld % 8 == 0 && a.v_ld % 8 == 0, "attention: cache rows of %ld / %ld elements are not 16-byte aligned", a.k_ld, a.v_ld);
     if (a.Dh <= 0 || a.Dh > 256 || a.Dh % 16 || a.Dv <= 0 || a.Dv > 256 || a.Dv % 16) {
         tsb_set_error("attention: unsupported head sizes %d / %d (multiples of 16 up to 256, or 512 with equal sizes)", a.Dh, a.Dv);

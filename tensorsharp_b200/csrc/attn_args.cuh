@@ -29,6 +29,7 @@ struct AttnArgs {
     unsigned* ticket;
     // Decode: positions per split fixed by the caller (a multiple of 32), so that a CTA's range and its block-table
     // entries do not wait for the sequence length; 0 = derive it from the length (ceil(span / splits), rounded to 32).
+    // Negative: derive it too, and where attn_decode_ring_kernel runs take parts of -split_len positions at least.
     int split_len;
     // Output gate: head h of query row t is multiplied by sigmoid(gate[t * gate_tok + h]) (t: packed query row; decode:
     // the sequence).  Null: none.

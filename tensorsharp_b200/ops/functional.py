@@ -674,9 +674,10 @@ def _split_positions() -> int:
     return int(os.environ.get("TSB_ATTN_SPLIT_LEN", "128"))
 
 
-def ring_attention(Hq: int, Hkv: int, Dh: int, page_size: int, fp8: bool) -> bool:
-    """Whether decode attention takes attn_decode_ring_kernel (csrc/attention_decode_mma.cu)."""
-    return Dh in (64, 128) and Hq % Hkv == 0 and Hq // Hkv <= 16 and page_size % 16 == 0 and not fp8
+def ring_attention(Hq: int, Hkv: int, Dh: int, page_size: int, k_cache: torch.Tensor, v_cache: torch.Tensor) -> bool:
+    """Whether decode attention takes attn_decode_ring_kernel (csrc/attention_decode_mma.cu): bf16 pages whose rows lie one behind the other."""
+    return (Dh in (64, 128) and Hq % Hkv == 0 and Hq // Hkv <= 16 and page_size % 16 == 0 and not is_fp8(k_cache)
+            and all(c.dim() != 3 or c.stride(0) == Hkv * Dh for c in (k_cache, v_cache)))
 
 
 def decode_splits(batch: Batch, Hkv: int, window: int, ring: bool = False) -> int:
@@ -725,7 +726,7 @@ def attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, bat
                                 kv_scale=Hkv * Dh if own_values else 0, log_bias=log_bias, sigmoid_bias=sigmoid_bias)
     if as_act:
         if q.is_cuda and batch.is_decode and Dh % 32 == 0:
-            ring = ring_attention(Hq, Hkv, Dh, batch.page_size, is_fp8(k_cache))
+            ring = ring_attention(Hq, Hkv, Dh, batch.page_size, k_cache, v_cache)
             sp = decode_splits(batch, Hkv, window, ring)
             out, oq, ods = _k().attn_decode(q, k_cache, v_cache, batch.block_table, batch.kv_lens, scale=scale, Hq=Hq, Hkv=Hkv,
                                             Dh=Dh, page_size=batch.page_size, splits=sp, split_len=decode_split_len(batch, sp, window, ring),
@@ -736,7 +737,7 @@ def attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, bat
     if q.is_cuda:
         kk = _k()
         if batch.is_decode:
-            ring = ring_attention(Hq, Hkv, Dh, batch.page_size, is_fp8(k_cache))
+            ring = ring_attention(Hq, Hkv, Dh, batch.page_size, k_cache, v_cache)
             sp = decode_splits(batch, Hkv, window, ring)
             out = kk.attn_decode(q, k_cache, v_cache, batch.block_table, batch.kv_lens, scale=scale, Hq=Hq, Hkv=Hkv,
                                  Dh=Dh, page_size=batch.page_size, splits=sp, split_len=decode_split_len(batch, sp, window, ring),

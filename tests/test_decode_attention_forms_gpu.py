@@ -1,0 +1,63 @@
+"""Decode attention through F.attention: caches whose rows are slices of wider rows, keys written just ahead, lengths far apart."""
+import pytest
+import torch
+
+from tensorsharp_b200.ops import functional as F
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def i32(x):
+    return torch.tensor(x, dtype=torch.int32, device=DEV)
+
+
+def decode_batch(lens, page, positions=None):
+    """A batch of one new token per sequence, the last of its ``lens`` positions; pages in a random order."""
+    need = [-(-n // page) for n in lens]
+    order, at = torch.randperm(sum(need)).tolist(), 0
+    table = torch.zeros(len(lens), max(need), dtype=torch.int32)
+    for b, n in enumerate(need):
+        table[b, :n] = torch.tensor(order[at:at + n])
+        at += n
+    slots = [int(table[b, (n - 1) // page]) * page + (n - 1) % page for b, n in enumerate(lens)]
+    B = len(lens)
+    return F.Batch(tokens=i32([0] * B), positions=i32([n - 1 for n in lens]), slots=torch.tensor(slots, device=DEV), cu_q=i32(list(range(B + 1))),
+                   kv_lens=i32(lens), block_table=table.to(DEV), last_idx=torch.arange(B, device=DEV), seq_slots=torch.arange(B, device=DEV), max_q_len=1,
+                   max_kv_len=max(lens), is_decode=True, page_size=page, h_cu_q=tuple(range(B + 1)), h_kv_lens=tuple(lens), rows_in_order=True), sum(need) * page
+
+
+def exact(q, k, v, batch, scale, window=0, sinks=None):
+    """Attention in 64 bits."""
+    B, Hq, Dh = q.shape
+    out = torch.empty(B, Hq, Dh, dtype=torch.float64, device=DEV)
+    for b, n in enumerate(batch.h_kv_lens):
+        j = torch.arange(max(0, n - window) if window else 0, n, device=DEV)
+        rows = batch.block_table[b, j // batch.page_size].long() * batch.page_size + j % batch.page_size
+        kb, vb = (x[rows].double() for x in (k, v))
+        qb = q[b].double().view(kb.shape[1], -1, Dh)
+        s = torch.einsum("kgd,nkd->kgn", qb, kb) * scale
+        if sinks is not None:
+            s = torch.cat([s, sinks.double().view(s.shape[0], s.shape[1], 1)], 2)
+        out[b] = torch.einsum("kgn,nkd->kgd", torch.softmax(s, 2)[..., :len(j)], vb).reshape(Hq, Dh)
+    return out
+
+
+def worst(got, want):
+    """Largest relative error of a (sequence, head)."""
+    got, want = got.double().view_as(want), want
+    return ((got - want).norm(dim=-1) / want.norm(dim=-1)).max().item()
+
+
+# weights and the result in bf16, 2^-9 each at most: of a head 5e-3 at most, whatever the lengths
+@pytest.mark.parametrize("as_act", [False, True])
+@pytest.mark.parametrize("window", [0, 50])
+def test_rows_that_are_slices(window, as_act):
+    torch.manual_seed(1)
+    Hq, Hkv, Dh, page = 8, 2, 64, 64
+    batch, rows = decode_batch([1, 40, 130, 700], page)
+    wide = torch.randn(rows, 3 * Hkv * Dh, device=DEV).bfloat16()
+    k, v = (wide[:, i * Hkv * Dh:(i + 1) * Hkv * Dh].unflatten(1, (Hkv, Dh)) for i in (0, 2))
+    q = torch.randn(4, Hq, Dh, device=DEV).bfloat16()
+    got = F.attention(q, k, v, batch, scale=Dh ** -0.5, Hq=Hq, Hkv=Hkv, Dh=Dh, window=window, as_act=as_act)
+    assert worst(got.b if as_act else got, exact(q, k, v, batch, Dh ** -0.5, window)) < 5e-3
