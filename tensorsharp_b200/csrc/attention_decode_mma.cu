@@ -335,8 +335,8 @@ __global__ void __launch_bounds__(128) attn_decode_mma_kernel(AttnArgs a) {
 // A chunk lies in one page, so a lane's pieces are one pointer and a stride; fragment addresses are one XOR each; masks and the
 // rescaling of the sums run only for chunks that need them.  (With an address per piece and all of that on every chunk the
 // kernel issued 990 instructions a chunk, and that bound it: 41 % of the issue slots with two warps per scheduler, HBM at 38 %.)
-// The chunks are asked for before the wait for the kernel ahead, except the one that holds the newest key: the kernel ahead writes the
-// rows of this step's tokens, and the lengths, the block table and all earlier rows are older than that.
+// Where the caller says that the kernel ahead writes no more than the rows of this step's tokens (AttnArgs::ahead: a decode step's rotary kernel),
+// the chunks are asked for before the wait for it, except the one that holds the newest key; otherwise all is read after the wait.
 // Measured with the merge kernel, us (the kernel above with its own splits / this one): 16 sequences of 2048 down to 1088 31.4 / 27.1,
 // 32 of them 50.8 / 42.8, 4 of 4096 down to 2560 21.6 / 16.5 (32 query, 8 key heads of 128); 64 of 1024 down to 520, 64 query, 8 key heads of 64 36.5 / 22.1, with a window of
 // 128 15.2 / 5.9; one of 131 7.1 / 5.1, one of 8111 14.3 / 13.7.
@@ -350,6 +350,8 @@ __global__ void __launch_bounds__(128) attn_decode_ring_kernel(AttnArgs a) {
     const uint32_t ring = (uint32_t)__cvta_generic_to_shared(smem_raw) + 16 * DH * 2 + warp * (STG * 2 * TILE);      // [STG][K, V][16][DH]
     const int split = blockIdx.x, hk = blockIdx.y, b = blockIdx.z;
     const int G = a.Hq / a.Hkv, h0 = hk * G;
+    bool waited = !a.ahead;
+    if (waited) pdl_wait();
     const int len = a.kv_lens[b];
     const int lo = (a.window > 0 && len > a.window) ? len - a.window : 0;
     const int span = len - lo;
@@ -367,7 +369,6 @@ __global__ void __launch_bounds__(128) attn_decode_ring_kernel(AttnArgs a) {
     const long stride = (long)a.Hkv * DH;
     const bf16* kp = a.k_cache + (long)hk * DH + c * 8 + key0 * stride;
     const bf16* vp = a.v_cache + (long)hk * DH + c * 8 + key0 * stride;
-    bool waited = false;
     auto fetch = [&](int i, int slot) {
         if (i < n) {
             const int base = w0 + i * 4 * KT;

@@ -49,6 +49,10 @@ struct AttnArgs {
     const float* log_r1;      // [Hq] or null: log_r1[h] ln(1 + log_r2[h] (query position - key position)) is taken off the score
     const float* log_r2;
     const float* sig_bias;    // [Hq] or null: no softmax; a visible key's weight is sigmoid(score + sig_bias[h])
+    // Decode (attn_decode_ring_kernel): 1 = the launch just ahead on the stream waits for its own predecessor before it lets this one start, and
+    // writes nothing of lengths, block table and cache but the rows of this step's tokens, each sequence's newest one: everything older
+    // may be read while it ends.  0 = it may have written anything.
+    int ahead;
 };
 
 // Whether only the kernels for head sizes of their own know a form that these arguments ask for.

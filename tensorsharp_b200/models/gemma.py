@@ -126,7 +126,7 @@ class _GemmaBase(ModelBase):
                               write_kv=write_kv)
         if write_kv:
             self.cp_sync_kv(kv_layer)
-        o = F.attention(qr, kc, vc, batch, scale=scale, Hq=Hq, Hkv=Hkv, Dh=Dh, window=window)
+        o = F.attention(qr, kc, vc, batch, scale=scale, Hq=Hq, Hkv=Hkv, Dh=Dh, ahead=True, window=window)
         y = F.linear(F.as_act(o), L["wo"], out_dtype=torch.float32)
         if self.tp_size > 1:
             self.tp_all_reduce(y)

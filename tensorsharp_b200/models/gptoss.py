@@ -125,7 +125,7 @@ class GptOssModel(ModelBase):
         qr = F.qkv_rope_cache(q, k, v, Hq=Hq, Hkv=Hkv, Dh=Dh, batch=batch, k_cache=self.kv.k[l], v_cache=self.kv.v[l],
                               rope=self.rope, eps=c.eps)
         self.cp_sync_kv(l)
-        return F.attention(qr, self.kv.k[l], self.kv.v[l], batch, scale=Dh ** -0.5, Hq=Hq, Hkv=Hkv, Dh=Dh,
+        return F.attention(qr, self.kv.k[l], self.kv.v[l], batch, scale=Dh ** -0.5, Hq=Hq, Hkv=Hkv, Dh=Dh, ahead=True,
                            window=self.window if l % 2 == 0 else 0, sinks=L["sinks"])
 
     def forward_exchange_small(self, h: torch.Tensor, batch: Batch, want_logits: bool, tpx) -> Optional[torch.Tensor]:

@@ -143,7 +143,7 @@ class NemotronHModel(ModelBase):
         qr = F.qkv_rope_cache(q, k, v, Hq=Hq, Hkv=Hkv, Dh=Dh, batch=batch, k_cache=self.kv.k[l],
                               v_cache=self.kv.v[l], rope=None, eps=c.eps)
         scale = self.attn_scale if self.attn_scale > 0 else Dh ** -0.5
-        o = F.attention(qr, self.kv.k[l], self.kv.v[l], batch, scale=scale, Hq=Hq, Hkv=Hkv, Dh=Dh)
+        o = F.attention(qr, self.kv.k[l], self.kv.v[l], batch, scale=scale, Hq=Hq, Hkv=Hkv, Dh=Dh, ahead=True)
         return F.linear(F.as_act(o), L["wo"], out_dtype=torch.float32)
 
     def _ffn(self, L, a, mid) -> torch.Tensor:

@@ -135,7 +135,7 @@ class Qwen3Model(ModelBase):
                                   v_cache=self.kv.v[self.l0 + l], rope=self.rope, qn=L["q_norm"], kn=L["k_norm"], eps=c.eps)
             qr = self.q_post_scale(qr, batch)
             self.cp_sync_kv(self.l0 + l)
-            o = F.attention(qr, self.kv.k[self.l0 + l], self.kv.v[self.l0 + l], batch, scale=Dh ** -0.5, Hq=Hq, Hkv=Hkv, Dh=Dh,
+            o = F.attention(qr, self.kv.k[self.l0 + l], self.kv.v[self.l0 + l], batch, scale=Dh ** -0.5, Hq=Hq, Hkv=Hkv, Dh=Dh, ahead=True,
                             as_act=small and L["wo"].uses_q8_activations)
             if tpx is not None:
                 tpx.linear_push(F.as_act(o), L["wo"])
@@ -179,7 +179,7 @@ class Qwen3Model(ModelBase):
             qr = F.qkv_rope_cache(q, k, v, Hq=Hq, Hkv=Hkv, Dh=Dh, batch=batch, k_cache=self.kv.k[self.l0 + l],
                                   v_cache=self.kv.v[self.l0 + l], rope=self.rope, qn=L["q_norm"], kn=L["k_norm"], eps=c.eps)
             qr = self.q_post_scale(qr, batch)
-            o = F.attention(qr, self.kv.k[self.l0 + l], self.kv.v[self.l0 + l], batch, scale=Dh ** -0.5, Hq=Hq, Hkv=Hkv, Dh=Dh)
+            o = F.attention(qr, self.kv.k[self.l0 + l], self.kv.v[self.l0 + l], batch, scale=Dh ** -0.5, Hq=Hq, Hkv=Hkv, Dh=Dh, ahead=True)
             h = self.row_parallel(F.as_act(o), L["wo"], h)
             a = F.norm(h, L["ffn_norm"], c.eps, want_q8=small)
             if "gate_up" in L:
@@ -277,7 +277,7 @@ class Qwen3Model(ModelBase):
             qr = F.qkv_rope_cache(q, k, v, Hq=Hq, Hkv=Hkv, Dh=Dh, batch=batch, k_cache=self.kv.k[self.l0 + l],
                                   v_cache=self.kv.v[self.l0 + l], rope=self.rope, qn=L["q_norm"], kn=L["k_norm"], eps=c.eps)
             qr = self.q_post_scale(qr, batch)
-            o = F.attention(qr, self.kv.k[self.l0 + l], self.kv.v[self.l0 + l], batch, scale=Dh ** -0.5, Hq=Hq, Hkv=Hkv, Dh=Dh).view(T, Hq * Dh)
+            o = F.attention(qr, self.kv.k[self.l0 + l], self.kv.v[self.l0 + l], batch, scale=Dh ** -0.5, Hq=Hq, Hkv=Hkv, Dh=Dh, ahead=True).view(T, Hq * Dh)
             if tpx is not None:
                 tpx.linear_push_fused(o, L["wo"])
                 a = tpx.reduce_norm(h, L["ffn_norm"], c.eps)
@@ -340,7 +340,7 @@ class Qwen3Model(ModelBase):
             qr = F.qkv_rope_cache(q, k, v, Hq=Hq, Hkv=Hkv, Dh=Dh, batch=batch, k_cache=self.kv.k[self.l0 + l],
                                   v_cache=self.kv.v[self.l0 + l], rope=self.rope, qn=L["q_norm"], kn=L["k_norm"], eps=c.eps)
             qr = self.q_post_scale(qr, batch)
-            o = F.attention(qr, self.kv.k[self.l0 + l], self.kv.v[self.l0 + l], batch, scale=Dh ** -0.5, Hq=Hq, Hkv=Hkv, Dh=Dh)
+            o = F.attention(qr, self.kv.k[self.l0 + l], self.kv.v[self.l0 + l], batch, scale=Dh ** -0.5, Hq=Hq, Hkv=Hkv, Dh=Dh, ahead=True)
             sp.gemm_rs(o.view(T, Hq * Dh), L["wo"])
             sp.norm_gather(h, L["ffn_norm"], c.eps, True)
             if "gate_up" in L:

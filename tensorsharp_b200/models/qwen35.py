@@ -175,7 +175,7 @@ class Qwen35Model(ModelBase):
         q, gate = qg[:, :, :Dh], qg[:, :, Dh:]
         qr = F.qkv_rope_cache(q, k, v, Hq=Hq, Hkv=Hkv, Dh=Dh, batch=batch, k_cache=self.kv.k[l],
                               v_cache=self.kv.v[l], rope=self.rope, qn=L["q_norm"], kn=L["k_norm"], eps=c.eps)
-        o = F.attention(qr, self.kv.k[l], self.kv.v[l], batch, scale=Dh ** -0.5, Hq=Hq, Hkv=Hkv, Dh=Dh)
+        o = F.attention(qr, self.kv.k[l], self.kv.v[l], batch, scale=Dh ** -0.5, Hq=Hq, Hkv=Hkv, Dh=Dh, ahead=True)
         o = F.glu("sigmoid_mul", gate.reshape(T, Hq * Dh).contiguous(), o)
         if self.tp_size == 1:
             return F.linear(F.as_act(o), L["wo"], out_dtype=torch.float32, residual=h)

@@ -89,6 +89,7 @@ class Batch:
     # table (logical page -> physical page of the ring).  None when the pool keeps every page of every layer.
     slots_w: Optional[torch.Tensor] = None
     block_table_w: Optional[torch.Tensor] = None
+    rows_apart: bool = False      # no sequence is in the batch twice: a decode step's rows each see one new key, their own; said by whoever built the batch
     rows_in_order: bool = False   # last_idx counts 0 .. T - 1; said by whoever built the batch, as equal numbers of rows do not show it
 
     def windowed(self) -> "Batch":
@@ -707,7 +708,7 @@ def attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, bat
               Hq: int, Hkv: int, Dh: int, window: int = 0, sinks: Optional[torch.Tensor] = None,
               softcap: float = 0.0, as_act: bool = False, Dv: Optional[int] = None, gate: Optional[torch.Tensor] = None, keep_first: int = 0,
               slopes: Optional[torch.Tensor] = None, own_values: bool = False, log_bias: Optional[Tuple[torch.Tensor, torch.Tensor]] = None,
-              sigmoid_bias: Optional[torch.Tensor] = None):
+              sigmoid_bias: Optional[torch.Tensor] = None, ahead: bool = False):
     """Causal attention of the packed queries against the paged cache -> [T, Hq * Dh].  ``as_act`` returns an
     ``Act``; on the CUDA decode path it already carries the int8 form written by the combine kernel, so
     the quantised projection that follows needs no quantise launch.  ``Dv``: value head size where it differs from
@@ -716,7 +717,9 @@ def attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, bat
     ``keep_first``: with a window, so many positions at the start stay visible; ``slopes`` [Hq]: slopes[h] times the distance
     is taken off the score; ``own_values``: a row of ``k_cache`` (see :func:`joint_norm_cache`) is key and value at once;
     ``log_bias`` (r1, r2) [Hq] each: r1[h] ln(1 + r2[h] distance) is taken off the score (after the soft cap);
-    ``sigmoid_bias`` [Hq]: no softmax, a visible key has the weight sigmoid(score + sigmoid_bias[h])."""
+    ``sigmoid_bias`` [Hq]: no softmax, a visible key has the weight sigmoid(score + sigmoid_bias[h]).
+    ``ahead``: the call follows :func:`qkv_rope_cache` of the same batch, and nothing else has written to the cache in between; a decode step may then read
+    older rows while that launch ends."""
     T = q.shape[0]
     Dv = Dv or Dh
     if q.is_cuda and (Dv != Dh or gate is not None or k_cache.dtype == torch.float32 or keep_first or slopes is not None or own_values
@@ -730,10 +733,10 @@ def attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, bat
             sp = decode_splits(batch, Hkv, window, ring)
             out, oq, ods = _k().attn_decode(q, k_cache, v_cache, batch.block_table, batch.kv_lens, scale=scale, Hq=Hq, Hkv=Hkv,
                                             Dh=Dh, page_size=batch.page_size, splits=sp, split_len=decode_split_len(batch, sp, window, ring),
-                                            sinks=sinks, softcap=softcap, window=window, want_q8=True)
+                                            sinks=sinks, softcap=softcap, window=window, want_q8=True, ahead=ahead and batch.rows_apart)
             return Act(out.view(T, Hq * Dh), oq, ods)
         return as_act_of(attention(q, k_cache, v_cache, batch, scale=scale, Hq=Hq, Hkv=Hkv, Dh=Dh, window=window, sinks=sinks,
-                                   softcap=softcap))
+                                   softcap=softcap, ahead=ahead))
     if q.is_cuda:
         kk = _k()
         if batch.is_decode:
@@ -741,7 +744,7 @@ def attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, bat
             sp = decode_splits(batch, Hkv, window, ring)
             out = kk.attn_decode(q, k_cache, v_cache, batch.block_table, batch.kv_lens, scale=scale, Hq=Hq, Hkv=Hkv,
                                  Dh=Dh, page_size=batch.page_size, splits=sp, split_len=decode_split_len(batch, sp, window, ring),
-                                 sinks=sinks, softcap=softcap, window=window)
+                                 sinks=sinks, softcap=softcap, window=window, ahead=ahead and batch.rows_apart)
         else:
             table, ps = batch.block_table, batch.page_size
             if is_fp8(k_cache):

@@ -90,7 +90,7 @@ class AttnArgs(C.Structure):
                 ("out_q", _vp), ("out_ds", _vp), ("ticket", _vp), ("split_len", C.c_int),
                 ("gate", _vp), ("gate_tok", C.c_long), ("gate_f32", C.c_int), ("Dv", C.c_int),
                 ("k_ld", C.c_long), ("v_ld", C.c_long), ("keep_first", C.c_int), ("slopes", _vp), ("gate_cols", C.c_int),
-                ("kv_scale", C.c_int), ("log_r1", _vp), ("log_r2", _vp), ("sig_bias", _vp)]
+                ("kv_scale", C.c_int), ("log_r1", _vp), ("log_r2", _vp), ("sig_bias", _vp), ("ahead", C.c_int)]
 
 
 _KIND = {"p": _vp, "i": C.c_int, "l": C.c_long, "f": C.c_float}
@@ -579,10 +579,13 @@ def _attn_args(q, k_cache, v_cache, out, block_table, kv_lens, cu_q, sinks, scal
 
 
 def attn_decode(q, k_cache, v_cache, block_table, kv_lens, *, scale, Hq, Hkv, Dh, page_size, splits, sinks=None,
-                softcap=0.0, window=0, out=None, want_q8=False, split_len=0, Dv=None, gate=None, **forms):
+                softcap=0.0, window=0, out=None, want_q8=False, split_len=0, Dv=None, gate=None, ahead=False, **forms):
     """q [B, Hq, Dh] bf16; one query per sequence against the paged cache.  ``want_q8`` also returns the
     output as int8 groups of 32 with (scale, sum) written by the combine kernel: (out, q, ds).  ``forms``: keep_first,
-    slopes, kv_scale, log_bias, sigmoid_bias (see AttnArgs)."""
+    slopes, kv_scale, log_bias, sigmoid_bias (see AttnArgs).  ``split_len``: see AttnArgs too.
+
+    ``ahead``: the caller's word that the launch just ahead on the stream writes nothing of the lengths, the block table and the cache but the newest row of
+    each sequence (as a decode step's rotary kernel does), so that everything older may be read before that launch has ended."""
     B = q.shape[0]
     Dv = Dv or Dh
     if out is None:
@@ -590,7 +593,7 @@ def attn_decode(q, k_cache, v_cache, block_table, kv_lens, *, scale, Hq, Hkv, Dh
     a = _attn_args(q, k_cache, v_cache, out, block_table, kv_lens, None, sinks, scale, softcap, window, Hq, Hkv, Dh,
                    page_size, B, Dv, gate, **forms)
     a.splits = splits
-    a.split_len = split_len
+    a.split_len, a.ahead = split_len, int(ahead)
     part_o = torch.empty((B, Hq, splits, Dv), dtype=torch.float32, device=q.device)
     part_ml = torch.empty((B, Hq, splits, 2), dtype=torch.float32, device=q.device)
     a.part_o, a.part_ml = _p(part_o), _p(part_ml)

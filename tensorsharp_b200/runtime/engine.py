@@ -69,7 +69,7 @@ class DecodeGraph:
             cu_q=torch.arange(B + 1, dtype=torch.int32, device=dev),
             kv_lens=torch.zeros(B, dtype=torch.int32, device=dev),
             block_table=table.to(dev),
-            last_idx=torch.arange(B, dtype=torch.int64, device=dev), rows_in_order=True,
+            last_idx=torch.arange(B, dtype=torch.int64, device=dev), rows_in_order=True, rows_apart=len(set(map(id, self.seqs))) == B,
             seq_slots=torch.tensor([s.slot for s in self.seqs], dtype=torch.int64, device=dev),
             max_q_len=1, max_kv_len=max_len, is_decode=True, page_size=ps,
             h_cu_q=tuple(range(B + 1)), h_kv_lens=tuple(s.length + 1 for s in self.seqs))
@@ -290,7 +290,7 @@ class BatchGraphStepper:
                      slots=torch.zeros(B, dtype=torch.int64, device=dev), cu_q=torch.arange(B + 1, dtype=torch.int32, device=dev),
                      kv_lens=torch.ones(B, dtype=torch.int32, device=dev),
                      block_table=torch.zeros((B, self.width), dtype=torch.int32, device=dev),
-                     last_idx=torch.arange(B, dtype=torch.int64, device=dev), rows_in_order=True,
+                     last_idx=torch.arange(B, dtype=torch.int64, device=dev), rows_in_order=True, rows_apart=True,
                      seq_slots=torch.zeros(B, dtype=torch.int64, device=dev),
                      max_q_len=1, max_kv_len=bucket, is_decode=True, page_size=self.model.kv.page_size,
                      h_cu_q=tuple(range(B + 1)), h_kv_lens=tuple([1] * B))

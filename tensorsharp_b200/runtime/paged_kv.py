@@ -219,4 +219,4 @@ class PagedKV:
             parts.update(slots_w=(np.concatenate(wslots), np.int64), block_table_w=([self.wtable_row(s, width) for s in seqs], np.int32))
         return Batch(**_on_device(parts, self.device),
             max_q_len=max_q, max_kv_len=max(lens), is_decode=(max_q == 1 and cu[-1] == len(seqs)),
-            rows_in_order=len(last) == cu[-1] and last == list(range(cu[-1])), page_size=ps, h_cu_q=tuple(cu), h_kv_lens=tuple(lens), h_seq_slots=tuple(s.slot for s in seqs))
+            rows_in_order=len(last) == cu[-1] and last == list(range(cu[-1])), rows_apart=len(set(map(id, seqs))) == len(seqs), page_size=ps, h_cu_q=tuple(cu), h_kv_lens=tuple(lens), h_seq_slots=tuple(s.slot for s in seqs))

@@ -61,3 +61,41 @@ def test_rows_that_are_slices(window, as_act):
     q = torch.randn(4, Hq, Dh, device=DEV).bfloat16()
     got = F.attention(q, k, v, batch, scale=Dh ** -0.5, Hq=Hq, Hkv=Hkv, Dh=Dh, window=window, as_act=as_act)
     assert worst(got.b if as_act else got, exact(q, k, v, batch, Dh ** -0.5, window)) < 5e-3
+
+
+def stepped(batch, rows, Hq, Hkv, Dh, ahead):
+    """Rows of this step through the rotary kernel and the attention right behind it, over a cache that holds everything older."""
+    k, v = (torch.randn(rows, Hkv, Dh, device=DEV).bfloat16() for _ in range(2))
+    k[batch.slots], v[batch.slots] = float("nan"), float("nan")           # not yet there
+    q, kn, vn = (torch.randn(batch.B, h, Dh, device=DEV) for h in (Hq, Hkv, Hkv))
+    outs = []
+    for _ in range(20):                                                   # launched in a row: rotary, attention, rotary, ...
+        k[batch.slots], v[batch.slots] = float("nan"), float("nan")
+        qr = F.qkv_rope_cache(q, kn, vn, Hq=Hq, Hkv=Hkv, Dh=Dh, batch=batch, k_cache=k, v_cache=v, rope=None)
+        outs.append(F.attention(qr, k, v, batch, scale=Dh ** -0.5, Hq=Hq, Hkv=Hkv, Dh=Dh, ahead=ahead))
+    want = exact(qr, k, v, batch, Dh ** -0.5)
+    assert torch.equal(k[batch.slots], kn.bfloat16())
+    return max(worst(o, want) for o in outs)
+
+
+# newest keys at the start, in the middle and at the end of a chunk of 16; bounds as above
+@pytest.mark.parametrize("ahead", [False, True])
+@pytest.mark.parametrize("lens", [[1], [17, 300, 64], [2049], [33, 32, 31, 1000, 1, 1217, 640, 16]])
+def test_newest_rows_written_just_ahead(lens, ahead):
+    torch.manual_seed(2)
+    batch, rows = decode_batch(lens, 64)
+    batch.rows_apart = True
+    assert stepped(batch, rows, 32, 8, 128, ahead) < 5e-3
+
+
+def test_a_sequence_twice():
+    """Two tokens of one sequence as two entries: the second sees the first's key, which the rotary kernel writes in the same launch, in the chunk before its own."""
+    torch.manual_seed(3)
+    n, page = 1025, 64
+    batch, rows = decode_batch([n], page)
+    t = batch.block_table[0]
+    batch.cu_q, batch.h_cu_q, batch.kv_lens, batch.h_kv_lens = i32([0, 1, 2]), (0, 1, 2), i32([n - 1, n]), (n - 1, n)
+    batch.tokens, batch.positions, batch.block_table = i32([0, 0]), i32([n - 2, n - 1]), torch.stack([t, t])
+    batch.slots = torch.tensor([int(t[p // page]) * page + p % page for p in (n - 2, n - 1)], device=DEV)
+    assert not batch.rows_apart
+    assert stepped(batch, rows, 32, 8, 128, True) < 5e-3
