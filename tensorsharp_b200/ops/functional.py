@@ -1261,16 +1261,14 @@ def moe_tile_list(flat: torch.Tensor, n_groups: int, bn: int):
 
 @functools.lru_cache(maxsize=1024)
 def _pair_tile(avg: int) -> int:
-    """Token tile of the grouped pair GEMM for groups of ``avg`` rows: the kernel's cost of a tile (csrc/gemm_tcgen05.cu: gemm_cost) times the
-    expected number of tiles of a group whose size spreads about the average by 1.8 times its root (what softmax routers of random rows show:
-    groups of 72 rows 11, 128 17, 256 30, 800 59).
-    Measured, a prompt through the layers around them (ms; the tile that half an empty tile per group would choose / this one): 256 experts of 2 x
-    512 x 2048, groups of 72 rows 3.88 / 3.68, of 128 5.43 / 5.36, of 256 10.08 / 9.94; 32 of 2 x 2880 x 2880, of 250 3.14 / 2.85, of 800 6.86 / 6.86."""
-    sd = 1.8 * math.sqrt(avg)
-
+    """Token tile of the grouped pair GEMM for groups of ``avg`` rows: the cost per useful row, from the kernel's cost of a tile
+    (csrc/gemm_tcgen05.cu: gemm_cost) and half an empty tile per group.  Half a tile is what groups of far apart sizes leave empty, as trained routers make
+    them; tiles that the average fills well gain little where all groups are alike and lose elsewhere.  Measured, an expert layer (us) with a tile for groups
+    that spread by 1.8 times the root of their average / this one, sizes spread by 1, by 13 to 18, by 28 to 30 and by 43 to 57 times that root: 256
+    experts of 2 x 512 x 2048, groups of 71 rows 446 / 447, 507 / 492, 499 / 466, 390 / 344, of 256 896 / 885, 920 / 868, 925 / 868, 818 / 740; 32 of 2 x 2880 x
+    2880, of 287 724 / 706, 750 / 673, 743 / 707, 735 / 694; 64 of 2 x 1536 x 2048, of 256 551 / 556, 585 / 548, 597 / 537, 538 / 481."""
     def cost(bn):
-        tiles = sum(0.5 * math.erfc((j * bn - avg) / (sd * math.sqrt(2.0))) for j in range(1 + int((avg + 4 * sd) / bn)))
-        return max(2.0 * bn, (128 + bn / 2) * 128 / 70) * tiles
+        return max(2.0 * bn, (128 + bn / 2) * 128 / 70) / bn * (1 + bn / (2 * avg))
     return min(range(80, 257, 16), key=cost)
 
 
