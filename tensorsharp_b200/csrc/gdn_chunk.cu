@@ -712,10 +712,10 @@ __global__ void __launch_bounds__(512) gdn_chunk_scan_kernel(GdnPrepArgs a) {
     }
     if (c < nc && threadIdx.x == 0) {      // a wait gave up: this chunk's copies and the next one's may be on their way, and land before the CTA leaves
         atomicExch(a.status, 6);           // (unless that takes longer than a wait's limit)
-        uint64_t until = 0;
-        tc::settle(&full[c & 1], (c >> 1) & 1, until);
-        tc::settle(&full[2], c & 1, until);
-        if (c + 1 < nc) tc::settle(&full[(c + 1) & 1], ((c + 1) >> 1) & 1, until);
+        bool given_up = false;
+        tc::settle(&full[c & 1], (c >> 1) & 1, given_up);
+        tc::settle(&full[2], c & 1, given_up);
+        if (c + 1 < nc) tc::settle(&full[(c + 1) & 1], ((c + 1) >> 1) & 1, given_up);
     }
     if (keys) {
 #pragma unroll

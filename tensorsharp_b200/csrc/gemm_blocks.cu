@@ -409,10 +409,10 @@ __global__ void __launch_bounds__(BG_THREADS, 2) gemm_blocks_kernel(const __grid
         }
         if (!ok && lane == 0) atomicExch(status, 1);
         // no copy is in flight when the CTA leaves, whichever wait gave up (unless it takes longer than a wait's limit)
-        uint64_t until = 0;
-        for (int i = max(0, it - stages); i < it; ++i) settle(&full[i % stages], (i / stages) & 1, until);
+        bool given_up = false;
+        for (int i = max(0, it - stages); i < it; ++i) settle(&full[i % stages], (i / stages) & 1, given_up);
         if (TYPE == TSB_MXFP4)
-            for (int i = max(0, j - 2); i < j; ++i) settle(&s_full[i & 1], (i >> 1) & 1, until);
+            for (int i = max(0, j - 2); i < j; ++i) settle(&s_full[i & 1], (i >> 1) & 1, given_up);
     } else if (warp == 2) {
         int it = 0, at = 0;
         uint32_t ph = 1;
@@ -433,8 +433,8 @@ __global__ void __launch_bounds__(BG_THREADS, 2) gemm_blocks_kernel(const __grid
             }
         }
         if (!ok && lane == 0) atomicExch(status, 1);
-        uint64_t until = 0;
-        for (int i = max(0, it - XS); i < it; ++i) settle(&x_full[i % XS], (i / XS) & 1, until);
+        bool given_up = false;
+        for (int i = max(0, it - XS); i < it; ++i) settle(&x_full[i % XS], (i / XS) & 1, given_up);
     } else if (warp == 1) {
         constexpr uint32_t idesc = make_idesc_bf16(128, NT);
         const uint64_t dx = make_desc_sw128(smem_u32(sX));

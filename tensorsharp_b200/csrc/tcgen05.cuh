@@ -1,7 +1,6 @@
 // Thin inline-PTX layer for the Blackwell (sm_100a) tensor pipeline: mbarriers, TMA tile
 // loads (never with cluster multicast), tcgen05 MMA / commit / TMEM load, TMEM allocation.
-// Every wait is bounded: it returns false after about two seconds on the GPU's timer instead of
-// spinning for ever, and the caller reports through a status word and unwinds normally.
+// Every wait is bounded: it returns false after one to two seconds instead of spinning for ever, and the caller reports through a status word and unwinds normally.
 #pragma once
 #include <cuda.h>
 #include "common.cuh"
@@ -52,43 +51,37 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint64
 // phase end at different polls, and a branch on the result alone would not bring them together again before a tcgen05.ld.
 __device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity)); }
 
-// A warp's wait with fewer instructions a poll: 64 polls between two looks at the timer (with one at each, as above, three waiting warps took
-// half of a decoding kernel's issue slots).  IDLE: the warp has nothing else to do and sleeps between its polls.  The limit is the same.
-template <bool IDLE>
+// A wait of five instructions a poll, for kernels whose other warps need the issue slots (with a look at the timer at each poll, as above, three waiting warps
+// took half of them).  A poll is suspended for 7 us at most, so its number bounds the time: 2^18 of them end at 1.9 s, at 1.05 s as measured
+// where nobody arrives (csrc/tests/wait_check.cu).  A look at the timer after the polls, 64 or 1024 of them, cost 1 to 4 % of the products of
+// gemm_blocks.cu and up to 8 of its expert tiles, in line, out of line or in the same instructions; this costs nothing (18.5 / 17.8 us, 2 x 9728 x 2560 by 16 rows).
+// IDLE: the thread has nothing else to do and sleeps between its polls.
+template <bool IDLE, int POLLS>
 __device__ __forceinline__ bool mbar_poll(uint64_t* bar, uint32_t parity) {
     uint32_t ok;
     if (IDLE)
         asm volatile("{\n\t.reg .pred p, q;\n\t.reg .u32 c;\n\tmov.u32 c, 0;\n\t"
-                     "POLL:\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t@p bra ENDED;\n\tnanosleep.u32 60;\n\t"
-                     "add.u32 c, c, 1;\n\tsetp.lt.u32 q, c, 64;\n\t@q bra POLL;\n\t"
+                     "POLL:\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, 7000;\n\t@p bra ENDED;\n\tnanosleep.u32 60;\n\t"
+                     "add.u32 c, c, 1;\n\tsetp.lt.u32 q, c, %3;\n\t@q bra POLL;\n\t"
                      "ENDED:\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                     : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+                     : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity), "n"(POLLS) : "memory");
     else
         asm volatile("{\n\t.reg .pred p, q;\n\t.reg .u32 c;\n\tmov.u32 c, 0;\n\t"
-                     "POLL:\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t@p bra ENDED;\n\t"
-                     "add.u32 c, c, 1;\n\tsetp.lt.u32 q, c, 64;\n\t@q bra POLL;\n\t"
+                     "POLL:\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, 7000;\n\t@p bra ENDED;\n\t"
+                     "add.u32 c, c, 1;\n\tsetp.lt.u32 q, c, %3;\n\t@q bra POLL;\n\t"
                      "ENDED:\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                     : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+                     : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity), "n"(POLLS) : "memory");
     return ok != 0;
 }
-template <bool IDLE = false>
-__device__ __forceinline__ bool hold(uint64_t* bar, uint32_t parity, uint64_t limit_ns = 2000000000ull) {
-    bool ok = mbar_poll<IDLE>(bar, parity);
-    if (!ok) {
-        const uint64_t t0 = global_timer_ns();
-        do ok = mbar_poll<IDLE>(bar, parity);
-        while (!ok && global_timer_ns() - t0 <= limit_ns);
-    }
-    return __all_sync(0xffffffffu, ok);
-}
-// Waits for what may still be on its way when a thread leaves, one barrier after another, all of them together no longer than one limit:
-// `until` is 0 ahead of the first and holds the common end from the first that is not there yet.
-__device__ __forceinline__ bool settle(uint64_t* bar, uint32_t parity, uint64_t& until, uint64_t limit_ns = 2000000000ull) {
-    if (mbar_poll<false>(bar, parity)) return true;
-    if (until == 0) until = global_timer_ns() + limit_ns;
-    bool ok;
-    do ok = mbar_poll<true>(bar, parity);
-    while (!ok && global_timer_ns() < until);
+// The wait of a whole warp.
+template <bool IDLE = false, int POLLS = 1 << 18>
+__device__ __forceinline__ bool hold(uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_poll<IDLE, POLLS>(bar, parity)); }
+// Waits for what may still be on its way when a thread leaves, one barrier after another: once one has not come within a wait's limit (`given_up`, false ahead
+// of the first) the others are only looked at, so that all of them together take no longer than one.
+template <int POLLS = 1 << 18>
+__device__ __forceinline__ bool settle(uint64_t* bar, uint32_t parity, bool& given_up) {
+    const bool ok = given_up ? mbar_poll<true, 1>(bar, parity) : mbar_poll<true, POLLS>(bar, parity);
+    given_up = given_up || !ok;
     return ok;
 }
 
