@@ -288,27 +288,32 @@ __device__ __forceinline__ void attn_decode_body(const AttnArgs& a) {
 // Latency is all that matters here (a few KB per block), so nothing is read in a dependent loop: each
 // lane fetches the (max, sum) of two splits at once, the warp reduces them, and the partial outputs
 // are fetched thirty-two splits at a time before any is used.  At most 64 splits.
+template <bool PLAN = false>
 __global__ void attn_combine_kernel(AttnArgs a) {
+    const int h = blockIdx.x, d = threadIdx.x, lane = threadIdx.x & 31;
+    int4 of = make_int4(blockIdx.y, 0, a.splits, 0);
+    if (PLAN) of = __ldcg(a.plan + a.parts + blockIdx.y);      // older than the launch ahead, whose parts these are
     pdl_wait();
     pdl_trigger();
-    const int h = blockIdx.x, b = blockIdx.y, d = threadIdx.x, lane = threadIdx.x & 31;
-    const long base = ((long)b * a.Hq + h) * a.splits;
-    const bool in0 = lane < a.splits, in1 = lane + 32 < a.splits;
-    const float2 ml0 = in0 ? *reinterpret_cast<const float2*>(a.part_ml + (base + lane) * 2) : make_float2(-INFINITY, 0.f);
-    const float2 ml1 = in1 ? *reinterpret_cast<const float2*>(a.part_ml + (base + lane + 32) * 2) : make_float2(-INFINITY, 0.f);
+    if (PLAN && of.x < 0) return;
+    const int b = of.x, splits = of.z, step = PLAN ? a.Hq : 1;
+    const long base = PLAN ? (long)of.y * a.Hq + h : ((long)b * a.Hq + h) * splits;
+    const bool in0 = lane < splits, in1 = lane + 32 < splits;
+    const float2 ml0 = in0 ? *reinterpret_cast<const float2*>(a.part_ml + (base + lane * step) * 2) : make_float2(-INFINITY, 0.f);
+    const float2 ml1 = in1 ? *reinterpret_cast<const float2*>(a.part_ml + (base + (lane + 32) * step) * 2) : make_float2(-INFINITY, 0.f);
     const float sink = a.sinks ? a.sinks[h] : -INFINITY;
     const int dd = d < a.Dh ? d : 0;
     float pv[32];                                       // asked for before the exchange below waits for the maxima
 #pragma unroll
-    for (int i = 0; i < 32; ++i) pv[i] = i < a.splits ? a.part_o[(base + i) * a.Dh + dd] : 0.f;
+    for (int i = 0; i < 32; ++i) pv[i] = i < splits ? a.part_o[(base + i * step) * a.Dh + dd] : 0.f;
     const float mm = fmaxf(sink, warp_max(fmaxf(ml0.x, ml1.x)));
     const float c0 = (ml0.x == -INFINITY) ? 0.f : __expf(ml0.x - mm), c1 = (ml1.x == -INFINITY) ? 0.f : __expf(ml1.x - mm);
     const float ll = warp_sum(ml0.y * c0 + ml1.y * c1) + (a.sinks ? __expf(sink - mm) : 0.f);
     float o = 0.f;
-    for (int s0 = 0; s0 < a.splits; s0 += 32) {
+    for (int s0 = 0; s0 < splits; s0 += 32) {
         if (s0 > 0) {
 #pragma unroll
-            for (int i = 0; i < 32; ++i) pv[i] = (s0 + i < a.splits) ? a.part_o[(base + s0 + i) * a.Dh + dd] : 0.f;
+            for (int i = 0; i < 32; ++i) pv[i] = (s0 + i < splits) ? a.part_o[(base + (s0 + i) * step) * a.Dh + dd] : 0.f;
         }
 #pragma unroll
         for (int i = 0; i < 32; ++i) {
@@ -410,12 +415,14 @@ static int attn_decode_impl(const AttnArgs* args, void* stream, bool allow_fused
     cudaStream_t s = (cudaStream_t)stream;
     int rc;
     if (a.gate != nullptr) a.ticket = nullptr;          // the in-kernel merges know no gate
+    TSB_CHECK_ARG(a.plan == nullptr || (a.each > 0 && a.parts > a.B * a.each), "attn_decode: %d parts of %d sequences, %d each", a.parts, a.B, a.each);
     if (attn_needs_vd(a)) {
+        a.plan = nullptr;
         if (a.Dv == 0) a.Dv = a.Dh;
         rc = tsb_attn_decode_vd_launch(a, s);
         if (rc != TSB_OK) return rc;
         a.Dh = a.Dv;                                    // the combine works on output columns
-        TSB_CHECK_CUDA(tsb_launch(attn_combine_kernel, dim3(a.Hq, a.B), dim3((a.Dh + 31) & ~31), 0, s, a));
+        TSB_CHECK_CUDA(tsb_launch(attn_combine_kernel<false>, dim3(a.Hq, a.B), dim3((a.Dh + 31) & ~31), 0, s, a));
         TSB_CHECK_LAUNCH();
         return TSB_OK;
     }
@@ -432,11 +439,15 @@ static int attn_decode_impl(const AttnArgs* args, void* stream, bool allow_fused
         if (rc != TSB_OK) return rc;
         TSB_CHECK_LAUNCH();
         if (!merged) {
-            TSB_CHECK_CUDA(tsb_launch(attn_combine_kernel, dim3(a.Hq, a.B), dim3((a.Dh + 31) & ~31), 0, s, a));
+            if (a.plan != nullptr)
+                TSB_CHECK_CUDA(tsb_launch(attn_combine_kernel<true>, dim3(a.Hq, attn_part_merges(a.parts, a.each, a.B)), dim3((a.Dh + 31) & ~31), 0, s, a));
+            else
+                TSB_CHECK_CUDA(tsb_launch(attn_combine_kernel<false>, dim3(a.Hq, a.B), dim3((a.Dh + 31) & ~31), 0, s, a));
             TSB_CHECK_LAUNCH();
         }
         return TSB_OK;
     }
+    a.plan = nullptr;
     switch (a.Dh) {
     case 64: rc = launch_decode_g<64>(a, s); break;
     case 128: rc = launch_decode_g<128>(a, s); break;
@@ -449,7 +460,7 @@ static int attn_decode_impl(const AttnArgs* args, void* stream, bool allow_fused
     if (rc != TSB_OK) return rc;
     TSB_CHECK_LAUNCH();
     if (a.ticket == nullptr) {
-        TSB_CHECK_CUDA(tsb_launch(attn_combine_kernel, dim3(a.Hq, a.B), dim3((a.Dh + 31) & ~31), 0, s, a));
+        TSB_CHECK_CUDA(tsb_launch(attn_combine_kernel<false>, dim3(a.Hq, a.B), dim3((a.Dh + 31) & ~31), 0, s, a));
         TSB_CHECK_LAUNCH();
     }
     return TSB_OK;
@@ -460,9 +471,9 @@ extern "C" int tsb_attn_decode(const AttnArgs* args, void* stream) { return attn
 // The merge of the split partials on its own, for split kernels that live in other translation units.
 extern "C" int tsb_attn_combine(const AttnArgs* args, void* stream) {
     const AttnArgs& a = *args;
-    TSB_CHECK_ARG(a.splits >= 1 && a.splits <= 64 && a.part_o && a.part_ml, "attn_combine: scratch for %d splits (limit 64)", a.splits);
+    TSB_CHECK_ARG(a.splits >= 1 && a.splits <= 64 && a.part_o && a.part_ml && a.plan == nullptr, "attn_combine: scratch for %d splits (limit 64)", a.splits);
     if (a.B == 0) return TSB_OK;
-    TSB_CHECK_CUDA(tsb_launch(attn_combine_kernel, dim3(a.Hq, a.B), dim3((a.Dh + 31) & ~31), 0, (cudaStream_t)stream, a));
+    TSB_CHECK_CUDA(tsb_launch(attn_combine_kernel<false>, dim3(a.Hq, a.B), dim3((a.Dh + 31) & ~31), 0, (cudaStream_t)stream, a));
     TSB_CHECK_LAUNCH();
     return TSB_OK;
 }

@@ -340,7 +340,7 @@ __global__ void __launch_bounds__(128) attn_decode_mma_kernel(AttnArgs a) {
 // Measured with the merge kernel, us (the kernel above with its own splits / this one): 16 sequences of 2048 down to 1088 31.4 / 27.1,
 // 32 of them 50.8 / 42.8, 4 of 4096 down to 2560 21.6 / 16.5 (32 query, 8 key heads of 128); 64 of 1024 down to 520, 64 query, 8 key heads of 64 36.5 / 22.1, with a window of
 // 128 15.2 / 5.9; one of 131 7.1 / 5.1, one of 8111 14.3 / 13.7.
-template <int DH>
+template <int DH, bool PLAN>
 __global__ void __launch_bounds__(128) attn_decode_ring_kernel(AttnArgs a) {
     constexpr int CH = DH / 8, KT = 16, STG = 3, TILE = KT * DH * 2;                       // bytes of a K or V tile
     constexpr float LOG2E = 1.4426950408889634f;
@@ -348,14 +348,24 @@ __global__ void __launch_bounds__(128) attn_decode_ring_kernel(AttnArgs a) {
     bf16* sQ = reinterpret_cast<bf16*>(smem_raw);                          // [16][DH]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t ring = (uint32_t)__cvta_generic_to_shared(smem_raw) + 16 * DH * 2 + warp * (STG * 2 * TILE);      // [STG][K, V][16][DH]
-    const int split = blockIdx.x, hk = blockIdx.y, b = blockIdx.z;
-    const int G = a.Hq / a.Hkv, h0 = hk * G;
+    // with a plan the heads of a part run side by side: their rows of a position lie together
+    const int hk = PLAN ? blockIdx.x : blockIdx.y, G = a.Hq / a.Hkv, h0 = hk * G;
     bool waited = !a.ahead;
     if (waited) pdl_wait();
+    int4 part = make_int4(blockIdx.z, blockIdx.x, a.splits, 0);             // sequence, which of its parts, how many, positions of one
+    if (PLAN) {
+        part = __ldcg(a.plan + blockIdx.y);
+        if (part.x < 0) {
+            if (!waited) pdl_wait();
+            pdl_trigger();
+            return;
+        }
+    }
+    const int b = part.x, split = part.y, splits = part.z;
     const int len = a.kv_lens[b];
     const int lo = (a.window > 0 && len > a.window) ? len - a.window : 0;
     const int span = len - lo;
-    const int per = a.split_len > 0 ? a.split_len : max((((span + a.splits - 1) / a.splits) + 63) & ~63, -a.split_len);      // whole rounds of the four warps
+    const int per = PLAN ? part.w : a.split_len > 0 ? a.split_len : max((((span + splits - 1) / splits) + 63) & ~63, -a.split_len);      // whole rounds of the four warps
     const int s0 = lo + split * per, s1 = min(len, s0 + per), w0 = (s0 & ~(KT - 1)) + warp * KT;      // this warp's first chunk
     const int n = max(0, (s1 - w0 + 4 * KT - 1) / (4 * KT));                // and how many it has
     const int* table = a.block_table + (long)b * a.max_pages;
@@ -525,8 +535,8 @@ __global__ void __launch_bounds__(128) attn_decode_ring_kernel(AttnArgs a) {
             ll += red_l[w * 16 + g] * c;
             ov += red_o[(w * G + g) * DH + d] * c;
         }
-        if (a.splits > 1 || a.gate != nullptr) {
-            const long pi = ((long)b * a.Hq + h0 + g) * a.splits + split;
+        if (splits > 1 || a.gate != nullptr) {
+            const long pi = PLAN ? (long)blockIdx.y * a.Hq + h0 + g : ((long)b * a.Hq + h0 + g) * a.splits + split;
             a.part_o[pi * DH + d] = ov;
             if (d == 0) { a.part_ml[pi * 2] = mm; a.part_ml[pi * 2 + 1] = ll; }
             continue;
@@ -545,15 +555,58 @@ __global__ void __launch_bounds__(128) attn_decode_ring_kernel(AttnArgs a) {
     }
 }
 
-template <int DH>
+// The plan of a merged step (AttnArgs::plan), once for all layers of a window: formed in the CTAs of every launch it cost 5 us more.  One warp.
+__global__ void __launch_bounds__(32) attn_plan_kernel(const int* __restrict__ lens, int B, int window, int parts, int each, int least, int4* __restrict__ plan) {
+    pdl_wait();
+    pdl_trigger();
+    const int lane = threadIdx.x, merges = attn_part_merges(parts, each, B);
+    auto span = [&](int b) { return window > 0 ? min(lens[b], window) : lens[b]; };
+    int total = 0;
+    for (int b = lane; b < B; b += 32) total += span(b);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
+    const int length = attn_part_len(total, parts - B * each, least);
+    int before = 0, merged = 0;
+    for (int b0 = 0; b0 < B; b0 += 32) {
+        const int b = b0 + lane;
+        int per = 0;
+        const int n = b < B ? attn_part_count(span(b), length, each, least, &per) : 0;
+        int end = n;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, end, o);
+            if (lane >= o) end += v;
+        }
+        const int first = before + end - n;
+        for (int i = 0; i < n && first + i < parts; ++i) plan[first + i] = make_int4(b, i, n, per);
+        const unsigned several = __ballot_sync(0xffffffffu, n > 1);
+        const int at = merged + __popc(several & ((1u << lane) - 1u));
+        if (n > 1 && at < merges) plan[parts + at] = make_int4(b, first, n, 0);
+        merged += __popc(several);
+        before += __shfl_sync(0xffffffffu, end, 31);
+    }
+    for (int i = before + lane; i < parts; i += 32) plan[i] = make_int4(-1, 0, 0, 0);
+    for (int i = merged + lane; i < merges; i += 32) plan[parts + i] = make_int4(-1, 0, 0, 0);
+}
+
+extern "C" int tsb_attn_plan(const int* lens, int B, int window, int parts, int each, int least, void* plan, void* stream) {
+    TSB_CHECK_ARG(B > 0 && each > 0 && each <= 64 && parts > B * each && least > 0, "attn_plan: %d parts of %d sequences, %d each", parts, B, each);
+    TSB_CHECK_ARG((reinterpret_cast<uintptr_t>(plan) & 15) == 0, "attn_plan: the plan must start on 16 bytes");
+    TSB_CHECK_CUDA(tsb_launch(attn_plan_kernel, dim3(1), dim3(32), 0, (cudaStream_t)stream, lens, B, window, parts, each, least, (int4*)plan));
+    TSB_CHECK_LAUNCH();
+    return TSB_OK;
+}
+
+template <int DH, bool PLAN>
 static int launch_decode_ring(const AttnArgs& a, cudaStream_t s) {
     constexpr size_t smem = (size_t)(16 + 4 * 3 * 2 * 16) * DH * sizeof(bf16);     // the merge needs 4 x 16 rows of floats and less
     static bool configured = false;
     if (!configured) {
-        TSB_CHECK_CUDA(cudaFuncSetAttribute(attn_decode_ring_kernel<DH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        TSB_CHECK_CUDA(cudaFuncSetAttribute(attn_decode_ring_kernel<DH, PLAN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         configured = true;
     }
-    TSB_CHECK_CUDA(tsb_launch(attn_decode_ring_kernel<DH>, dim3(a.splits, a.Hkv, a.B), dim3(128), smem, s, a));
+    const dim3 grid = PLAN ? dim3(a.Hkv, a.parts, 1) : dim3(a.splits, a.Hkv, a.B);
+    TSB_CHECK_CUDA(tsb_launch(attn_decode_ring_kernel<DH, PLAN>, grid, dim3(128), smem, s, a));
     return TSB_OK;
 }
 
@@ -610,14 +663,16 @@ bool tsb_attn_decode_mma_cluster(const AttnArgs& a) {
 }
 
 // Returns TSB_OK; `*merged` tells whether the outputs are final (cluster form, a single split) or the caller has to launch the combine.
-int tsb_attn_decode_mma_launch(const AttnArgs& a, cudaStream_t s, bool* merged) {
+int tsb_attn_decode_mma_launch(AttnArgs& a, cudaStream_t s, bool* merged) {
     const bool cl = tsb_attn_decode_mma_cluster(a);
     *merged = cl;
+    if (cl || a.page_size % 16 != 0 || a.gate != nullptr) a.plan = nullptr;     // `splits` parts each
     if (cl && a.splits == 8) return a.Dh == 64 ? launch_decode_mma<64, 8>(a, s) : launch_decode_mma<128, 8>(a, s);
     if (cl) return a.Dh == 64 ? launch_decode_mma<64, 16>(a, s) : launch_decode_mma<128, 16>(a, s);
     if (a.page_size % 16 != 0) return a.Dh == 64 ? launch_decode_mma<64, 0>(a, s) : launch_decode_mma<128, 0>(a, s);
-    *merged = a.splits == 1 && a.gate == nullptr;
-    return a.Dh == 64 ? launch_decode_ring<64>(a, s) : launch_decode_ring<128>(a, s);
+    *merged = a.splits == 1 && a.plan == nullptr && a.gate == nullptr;
+    if (a.plan != nullptr) return a.Dh == 64 ? launch_decode_ring<64, true>(a, s) : launch_decode_ring<128, true>(a, s);
+    return a.Dh == 64 ? launch_decode_ring<64, false>(a, s) : launch_decode_ring<128, false>(a, s);
 }
 
 // The same split kernel on e4m3 pages (`k_cache` / `v_cache` point at bytes); the caller launches the combine.

@@ -281,6 +281,7 @@ static int launch_fp8_g(const AttnArgs& a, cudaStream_t s) {
 extern "C" int tsb_attn_decode_fp8(const AttnArgs* args, void* stream) {
     AttnArgs a = *args;
     a.ticket = nullptr;
+    a.plan = nullptr;
     TSB_CHECK_ARG(a.Hkv > 0 && a.Hq % a.Hkv == 0, "attn_decode_fp8: Hq=%d not a multiple of Hkv=%d", a.Hq, a.Hkv);
     TSB_CHECK_ARG(a.splits >= 1 && a.splits <= 64 && a.part_o && a.part_ml, "attn_decode_fp8: scratch for %d splits (limit 64)", a.splits);
     if (a.B == 0) return TSB_OK;

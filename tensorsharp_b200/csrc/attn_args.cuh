@@ -11,8 +11,8 @@ struct AttnArgs {
     const int* kv_lens;       // [B] tokens in the cache for this sequence (including the new ones)
     const int* cu_q;          // [B + 1] query offsets (prefill); null for decode (one query per sequence)
     const float* sinks;       // [Hq] or null
-    float* part_o;            // decode scratch [B, Hq, splits, Dh]
-    float* part_ml;           // decode scratch [B, Hq, splits, 2]
+    float* part_o;            // decode scratch [B, Hq, splits, Dh] (with `parts`: [parts, Hq, Dh])
+    float* part_ml;           // decode scratch [B, Hq, splits, 2] ([parts, Hq, 2])
     float scale;
     float softcap;            // 0 = off
     int window;               // 0 = full causal
@@ -53,7 +53,33 @@ struct AttnArgs {
     // writes nothing of lengths, block table and cache but the rows of this step's tokens, each sequence's newest one: everything older
     // may be read while it ends.  0 = it may have written anything.
     int ahead;
+    // Decode (attn_decode_ring_kernel): `plan` not null: the parts of all sequences are a list of `parts` places, in which a long sequence among short ones
+    // has more of them than the `each` (at most) of the others, in place of `splits` parts each.  Of tsb_attn_plan for the same lengths and window: int4
+    // {sequence (-1: none), which of its parts, how many it has, positions of one} for every place; then int4 {sequence (-1: none), first place, how many}
+    // for the sequences of more than one, of which there are no more than attn_part_merges.
+    int parts, each;
+    const int4* plan;
 };
+
+// How the sequences of a merged step are cut: `total` positions of all of them over `room` parts are the length that a part should have, of whole rounds of the
+// ring kernel's four warps and no less than `least`.  A sequence takes `each` parts, none below `least`, as it would alone; one whose parts would be longer
+// than twice that length takes as many as it needs to meet it, at most the 64 that the merge takes.  All of them together have each B + room places at most:
+// what is cut finer has less than one part beyond its share of room.
+__host__ __device__ __forceinline__ int attn_part_merges(int parts, int each, int B) { return each > 1 || parts - B * each > B ? B : parts - B * each; }
+__host__ __device__ __forceinline__ int attn_part_len(long total, int room, int least) {
+    const int p = (int)((total + room - 1) / room);
+    return ((p > least ? p : least) + 63) & ~63;
+}
+__host__ __device__ __forceinline__ int attn_part_count(int span, int length, int each, int least, int* per) {
+    int p = ((span + each - 1) / each + 63) & ~63;
+    if (p < least) p = least;
+    if (p > 2 * length) {
+        const int k = (span + length - 1) / length;
+        p = k > 64 ? ((span + 63) / 64 + 63) & ~63 : ((span + k - 1) / k + 63) & ~63;
+    }
+    *per = p;
+    return span > p ? (span + p - 1) / p : 1;
+}
 
 // Whether only the kernels for head sizes of their own know a form that these arguments ask for.
 static inline bool attn_needs_vd(const AttnArgs& a) {
@@ -79,7 +105,8 @@ int tsb_attn_prefill_vd_launch(const AttnArgs& a, int max_q, cudaStream_t s);
 int tsb_attn_decode_vd_launch(const AttnArgs& a, cudaStream_t s);         // the caller launches the combine
 
 // attention_decode_mma.cu: the tensor-core split kernel for decode batches (head sizes 64 / 128, up to 16 query heads
-// per KV head); the caller launches the combine unless `*merged` comes back true (splits merged by a thread-block cluster).
+// per KV head); the caller launches the combine unless `*merged` comes back true (splits merged by a thread-block cluster), with `a` as it comes back:
+// without `parts` where the kernel that runs knows none.
 bool tsb_attn_decode_mma_supported(const AttnArgs& a);
-int tsb_attn_decode_mma_launch(const AttnArgs& a, cudaStream_t s, bool* merged);
+int tsb_attn_decode_mma_launch(AttnArgs& a, cudaStream_t s, bool* merged);
 int tsb_attn_decode_mma_fp8_launch(const AttnArgs& a, cudaStream_t s);      // e4m3 pages; the caller launches the combine

@@ -662,7 +662,7 @@ def fp8_prefill_view(k_cache: torch.Tensor, v_cache: torch.Tensor, batch: Batch)
 def decode_split_len(batch: Batch, splits: int, window: int, ring: bool = False) -> int:
     """Positions per split fixed on the host from the reserved maximum length (0 with a sliding window, whose
     start depends on the actual length): the kernel then knows its range before it has read the length.  ``ring``: a sequence's own
-    length is shared out, which that kernel reads ahead of its wait, in parts of no less than decode_splits counts with (the negative
+    length is shared out, in parts of no less than decode_splits counts with (the negative
     number): a captured step, whose splits go by its bucket, then cuts a sequence where an eager one does."""
     if ring:
         return -_split_positions()
@@ -681,17 +681,47 @@ def ring_attention(Hq: int, Hkv: int, Dh: int, page_size: int, k_cache: torch.Te
             and all(c.dim() != 3 or c.stride(0) == Hkv * Dh for c in (k_cache, v_cache)))
 
 
+def decode_parts(batch: Batch, Hkv: int, window: int) -> Optional[Tuple[int, int]]:
+    """(places of all sequences' parts, parts of a sequence) of a merged step for the kernel that loads ahead, which cuts a long sequence among short ones into
+    more of them (csrc/attn_args.cuh: attn_part_count): 296 CTAs, two on an SM, shared out among the sequences, and as many over the key heads for what is cut
+    finer.  None for one sequence, and where none can be longer than one part, whose result then needs no merge launch.  It goes by the number of
+    sequences alone, and the lengths are read on the device: a captured step cuts a sequence where an eager one does.
+    Measured with the merge launch, us (the general kernel with its splits / `each` parts of every sequence whatever its length / these; 32 query, 8 key heads of
+    128): 16 sequences of 2048 down to 1088 32.3 / 28.6 / 28.7, one of 32000 among 15 of 300 91 / 173 / 34, one of 8192 among 15 of 1000 39.9 / 53.8 / 26.7; 4 of
+    4096 down 22.5 / 17.6 / 17.9, with one of 32000 39.0 / 57.5 / 29.4; 32 of 2048 down 52.6 / 42.2 / 44.5, with one of 32000 177 / 271 / 39; 64 of 1024 down (64
+    query, 8 key heads of 64) 38.2 / 22.9 / 27.3, with one of 32000 230 / 350 / 30."""
+    span = min(batch.max_kv_len, window) if window else batch.max_kv_len
+    if batch.B == 1 or span <= _split_positions() or os.environ.get("TSB_ATTN_CLUSTER", "0") not in ("", "0"):
+        return None
+    each = min(-(-296 // (batch.B * Hkv)), 64)
+    return batch.B * each + -(-296 // Hkv), each
+
+
+def _decode_kw(batch: Batch, Hq: int, Hkv: int, Dh: int, window: int, k_cache: torch.Tensor, v_cache: torch.Tensor, ahead: bool) -> dict:
+    """How attn_decode cuts a decode batch."""
+    ring = ring_attention(Hq, Hkv, Dh, batch.page_size, k_cache, v_cache)
+    sp = decode_splits(batch, Hkv, window, ring)
+    kw = dict(splits=sp, split_len=decode_split_len(batch, sp, window, ring), ahead=ahead and batch.rows_apart)
+    cut = decode_parts(batch, Hkv, window) if ring else None
+    if cut is not None:
+        key = ("attn_plan", cut, window)
+        plan = batch.cache.get(key)
+        if plan is None:                        # once a step; this launch is then the one just ahead
+            plan = batch.cache[key] = _k().attn_plan(batch.kv_lens, window, *cut, _split_positions())
+            kw.update(ahead=False)
+        kw.update(plan=plan)
+    return kw
+
+
 def decode_splits(batch: Batch, Hkv: int, window: int, ring: bool = False) -> int:
-    """Split-KV factor for decode attention: enough CTAs to cover the GPU's 148 SMs.  ``ring``: the kernel that loads ahead, two CTAs an SM and
-    no more (with the merge, us for 1 / 2 / 3 / 4 / 9 splits: 16 sequences of about 1600 40.9 / 26.3 / 27.1 / 26.0 / 30.2, 32 46.3 / 42.8 / 45.6 / 47.8;
-    64 of about 800 29.7 / 31.4 / 33.2; 4 of about 3300 for 4 / 9 / 13 / 18 / 37 21.3 / 16.0 / 18.8 / 19.1 / 23.8); one sequence no more than the
-    merge fetches at once (8111 positions in 37 / 32 splits: 13.0 / 11.6 us with it)."""
+    """Split-KV factor for decode attention: enough CTAs to cover the GPU's 148 SMs.  ``ring``: the kernel that loads ahead takes no more of one sequence than
+    the merge fetches at once (8111 positions in 37 / 32 splits: 13.0 / 11.6 us with it); merged steps have decode_parts."""
     span = batch.max_kv_len if not window else min(batch.max_kv_len, window)
     # one sequence: about two CTAs per SM; batches: up to eight (a CTA is 128 threads and latency-bound, and with 16
     # sequences two splits per (sequence, KV head) left the kernel at a fifth of the memory rate)
     want = max(1, (148 * (2 if batch.B == 1 else 8)) // max(1, batch.B * Hkv))
-    if ring:
-        want = -(-296 // (batch.B * Hkv)) if batch.B > 1 else min(want, 32)
+    if ring and batch.B == 1:
+        want = min(want, 32)
     per = _split_positions()
     n = int(max(1, min(want, (span + per - 1) // per, 64)))
     # TSB_ATTN_CLUSTER=1: 8 or 16 splits are merged inside the attention kernel by a thread-block cluster (no combine
@@ -729,22 +759,17 @@ def attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, bat
                                 kv_scale=Hkv * Dh if own_values else 0, log_bias=log_bias, sigmoid_bias=sigmoid_bias)
     if as_act:
         if q.is_cuda and batch.is_decode and Dh % 32 == 0:
-            ring = ring_attention(Hq, Hkv, Dh, batch.page_size, k_cache, v_cache)
-            sp = decode_splits(batch, Hkv, window, ring)
-            out, oq, ods = _k().attn_decode(q, k_cache, v_cache, batch.block_table, batch.kv_lens, scale=scale, Hq=Hq, Hkv=Hkv,
-                                            Dh=Dh, page_size=batch.page_size, splits=sp, split_len=decode_split_len(batch, sp, window, ring),
-                                            sinks=sinks, softcap=softcap, window=window, want_q8=True, ahead=ahead and batch.rows_apart)
+            out, oq, ods = _k().attn_decode(q, k_cache, v_cache, batch.block_table, batch.kv_lens, scale=scale, Hq=Hq, Hkv=Hkv, Dh=Dh, page_size=batch.page_size,
+                                            sinks=sinks, softcap=softcap, window=window, want_q8=True,
+                                            **_decode_kw(batch, Hq, Hkv, Dh, window, k_cache, v_cache, ahead))
             return Act(out.view(T, Hq * Dh), oq, ods)
         return as_act_of(attention(q, k_cache, v_cache, batch, scale=scale, Hq=Hq, Hkv=Hkv, Dh=Dh, window=window, sinks=sinks,
                                    softcap=softcap, ahead=ahead))
     if q.is_cuda:
         kk = _k()
         if batch.is_decode:
-            ring = ring_attention(Hq, Hkv, Dh, batch.page_size, k_cache, v_cache)
-            sp = decode_splits(batch, Hkv, window, ring)
-            out = kk.attn_decode(q, k_cache, v_cache, batch.block_table, batch.kv_lens, scale=scale, Hq=Hq, Hkv=Hkv,
-                                 Dh=Dh, page_size=batch.page_size, splits=sp, split_len=decode_split_len(batch, sp, window, ring),
-                                 sinks=sinks, softcap=softcap, window=window, ahead=ahead and batch.rows_apart)
+            out = kk.attn_decode(q, k_cache, v_cache, batch.block_table, batch.kv_lens, scale=scale, Hq=Hq, Hkv=Hkv, Dh=Dh, page_size=batch.page_size,
+                                 sinks=sinks, softcap=softcap, window=window, **_decode_kw(batch, Hq, Hkv, Dh, window, k_cache, v_cache, ahead))
         else:
             table, ps = batch.block_table, batch.page_size
             if is_fp8(k_cache):

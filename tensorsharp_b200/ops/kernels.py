@@ -90,7 +90,7 @@ class AttnArgs(C.Structure):
                 ("out_q", _vp), ("out_ds", _vp), ("ticket", _vp), ("split_len", C.c_int),
                 ("gate", _vp), ("gate_tok", C.c_long), ("gate_f32", C.c_int), ("Dv", C.c_int),
                 ("k_ld", C.c_long), ("v_ld", C.c_long), ("keep_first", C.c_int), ("slopes", _vp), ("gate_cols", C.c_int),
-                ("kv_scale", C.c_int), ("log_r1", _vp), ("log_r2", _vp), ("sig_bias", _vp), ("ahead", C.c_int)]
+                ("kv_scale", C.c_int), ("log_r1", _vp), ("log_r2", _vp), ("sig_bias", _vp), ("ahead", C.c_int), ("parts", C.c_int), ("each", C.c_int), ("plan", _vp)]
 
 
 _KIND = {"p": _vp, "i": C.c_int, "l": C.c_long, "f": C.c_float}
@@ -578,11 +578,25 @@ def _attn_args(q, k_cache, v_cache, out, block_table, kv_lens, cu_q, sinks, scal
     return a
 
 
+def attn_plan(kv_lens: torch.Tensor, window: int, parts: int, each: int, least: int):
+    """The plan of ``parts`` parts, ``each`` of a sequence and more of one that is long among the others, of ``least`` positions at least, for
+    :func:`attn_decode` of sequences of ``kv_lens`` (int32 on the device)."""
+    B = kv_lens.shape[0]
+    assert kv_lens.dtype == torch.int32 and kv_lens.is_contiguous()
+    rows = torch.empty((parts + B, 4), dtype=torch.int32, device=kv_lens.device)
+    lib = _lib()
+    lib.tsb_attn_plan.restype = C.c_int
+    native.check(lib.tsb_attn_plan(_p(kv_lens), C.c_int(B), C.c_int(int(window or 0)), C.c_int(parts), C.c_int(each), C.c_int(least), _p(rows), _stream()), "attn_plan")
+    _count(1)
+    return rows, parts, each
+
+
 def attn_decode(q, k_cache, v_cache, block_table, kv_lens, *, scale, Hq, Hkv, Dh, page_size, splits, sinks=None,
-                softcap=0.0, window=0, out=None, want_q8=False, split_len=0, Dv=None, gate=None, ahead=False, **forms):
+                softcap=0.0, window=0, out=None, want_q8=False, split_len=0, Dv=None, gate=None, ahead=False, plan=None, **forms):
     """q [B, Hq, Dh] bf16; one query per sequence against the paged cache.  ``want_q8`` also returns the
     output as int8 groups of 32 with (scale, sum) written by the combine kernel: (out, q, ds).  ``forms``: keep_first,
-    slopes, kv_scale, log_bias, sigmoid_bias (see AttnArgs).  ``split_len``: see AttnArgs too.
+    slopes, kv_scale, log_bias, sigmoid_bias (see AttnArgs).  ``split_len``: see AttnArgs.  ``plan``: of
+    :func:`attn_plan`; where the kernel for the call knows none every sequence is cut into ``splits``.
 
     ``ahead``: the caller's word that the launch just ahead on the stream writes nothing of the lengths, the block table and the cache but the newest row of
     each sequence (as a decode step's rotary kernel does), so that everything older may be read before that launch has ended."""
@@ -594,8 +608,12 @@ def attn_decode(q, k_cache, v_cache, block_table, kv_lens, *, scale, Hq, Hkv, Dh
                    page_size, B, Dv, gate, **forms)
     a.splits = splits
     a.split_len, a.ahead = split_len, int(ahead)
-    part_o = torch.empty((B, Hq, splits, Dv), dtype=torch.float32, device=q.device)
-    part_ml = torch.empty((B, Hq, splits, 2), dtype=torch.float32, device=q.device)
+    parts = 0
+    if plan is not None:
+        rows, parts, a.each = plan
+        a.plan, a.parts = _p(rows), parts
+    part_o = torch.empty((max(B * splits, parts), Hq, Dv), dtype=torch.float32, device=q.device)
+    part_ml = torch.empty((max(B * splits, parts), Hq, 2), dtype=torch.float32, device=q.device)
     a.part_o, a.part_ml = _p(part_o), _p(part_ml)
     oq = ods = None
     if want_q8 and Dh % 32 == 0:

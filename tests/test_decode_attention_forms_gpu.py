@@ -99,3 +99,35 @@ def test_a_sequence_twice():
     batch.slots = torch.tensor([int(t[p // page]) * page + p % page for p in (n - 2, n - 1)], device=DEV)
     assert not batch.rows_apart
     assert stepped(batch, rows, 32, 8, 128, True) < 5e-3
+
+
+# one long sequence among short ones, whose parts are then cut by all positions together; bounds as above
+@pytest.mark.parametrize("Hq,Hkv,Dh", [(32, 8, 128), (64, 8, 64), (8, 1, 128)])
+@pytest.mark.parametrize("lens", [[300, 9000, 17, 1], [3000, 2500, 600, 1023, 1024, 1025, 500, 64], [129] * 40, [1] * 33 + [20000], [16000, 16000]])
+@pytest.mark.parametrize("window,sink", [(0, False), (700, True)])
+def test_lengths_far_apart(Hq, Hkv, Dh, lens, window, sink):
+    torch.manual_seed(4)
+    batch, rows = decode_batch(lens, 64)
+    k, v = (torch.randn(rows, Hkv, Dh, device=DEV).bfloat16() for _ in range(2))
+    q, sinks = torch.randn(len(lens), Hq, Dh, device=DEV).bfloat16(), torch.randn(Hq, device=DEV) if sink else None
+    kw = dict(scale=Dh ** -0.5, Hq=Hq, Hkv=Hkv, Dh=Dh, window=window, sinks=sinks)
+    got = F.attention(q, k, v, batch, as_act=True, **kw)
+    assert worst(got.b, exact(q, k, v, batch, Dh ** -0.5, window, sinks)) < 5e-3
+    back = got.q.view(len(lens), -1, 32).double() * got.ds.view(len(lens), -1, 2)[..., :1].double()
+    assert (back.view_as(got.b.double()) - got.b.double()).abs().max() <= got.b.abs().max().double() / 254 * 1.01       # half a step of 127ths of a group's largest value
+    batch.max_kv_len = 32768                                             # a captured step's bucket: the same parts, the same bits
+    assert torch.equal(F.attention(q, k, v, batch, **kw), got.b)
+
+
+@pytest.mark.parametrize("Hq,Hkv,Dh,lens", [(32, 8, 128, [2048 - 64 * i for i in range(16)]), (64, 8, 64, [1024 - 8 * i for i in range(64)]), (32, 8, 128, [700, 400])])
+def test_even_lengths_are_cut_as_each_alone(Hq, Hkv, Dh, lens):
+    """Where no sequence is far longer than the others the plan changes nothing: the bits of a launch that cuts each sequence into the same number of parts."""
+    torch.manual_seed(5)
+    batch, rows = decode_batch(lens, 64)
+    k, v = (torch.randn(rows, Hkv, Dh, device=DEV).bfloat16() for _ in range(2))
+    q = torch.randn(len(lens), Hq, Dh, device=DEV).bfloat16()
+    got = F.attention(q, k, v, batch, scale=0.1, Hq=Hq, Hkv=Hkv, Dh=Dh)
+    assert any(key[0] == "attn_plan" for key in batch.cache)
+    each = F.decode_parts(batch, Hkv, 0)[1]
+    alone = F._k().attn_decode(q, k, v, batch.block_table, batch.kv_lens, scale=0.1, Hq=Hq, Hkv=Hkv, Dh=Dh, page_size=64, splits=each, split_len=-128)
+    assert torch.equal(got.view_as(alone), alone)
