@@ -32,9 +32,10 @@ PAIR_GEMM_MIN_M = 64  # above this many rows the tensor-core GEMM is the one tha
 GATED_ACTS = ("swiglu", "geglu", "geglu_tanh", "geglu_erf", "swiglu_oai")
 GEMV_MAX_M = 16   # "small batch": token count up to which the models take their decode-style paths (int8 activations, mailbox exchanges)
 # Dense projections of more rows than this go to the tensor cores all the same, from the blocks (csrc/gemm_blocks.cu) or, for types that it does not take,
-# from the bf16 copy: the Qwen3-4B shape at batch 16 took 10.95 ms a step with the weight-streaming GEMVs and 8.15 ms with copies (TSB_GEMV_MAX_M moves
-# it; gemv_rows below lowers it where the blocks are taken as they are)
+# from the bf16 copy: the Qwen3-4B shape at batch 16 took 10.95 ms a step with the weight-streaming GEMVs and 8.15 ms with copies.  gemv_rows below lowers
+# it where the tensor cores take the weight as it is; where TSB_GEMV_MAX_M is given, that number holds for every weight.
 DENSE_GEMV_MAX_M = min(GEMV_MAX_M, int(os.environ.get("TSB_GEMV_MAX_M", "8")))
+GEMV_ROWS_GIVEN = "TSB_GEMV_MAX_M" in os.environ
 
 
 @dataclass
@@ -450,7 +451,7 @@ def gemv_rows(w: QuantWeight, act: Optional[str] = None) -> int:
     2560 10.9 / 23.3 / 30.1 / 31.6 / 18.7; 16.8; Q6_K 2560 x 9728 7.6 / 12.4 / 20.7 / 20.9 / 59.8; 11.5; Q8_0 5376 x 21504 26.9 / 29.5 / 43.8 / 44.0 / 90.2; 27; bf16 2880 x
     4096 7.5 / 9.0 / 12.8 / 12.8 / 21.8; 9.2, 32768 x 2880 29.8 / 36.2 / 56.4 / 58.0 / 102.8; 35."""
     from ..gguf.constants import GGMLType
-    if w.experts != 1 or (w.ggml_type == GGMLType.Q8_0 and w.N * w.K < 1 << 20):
+    if GEMV_ROWS_GIVEN or w.experts != 1 or (w.ggml_type == GGMLType.Q8_0 and w.N * w.K < 1 << 20):
         # (512 x 1024 of Q8_0, 3 / 5 / 8 rows 3.1 / 3.8 / 4.1 us with the rows' quantisation, which a norm brings along; 3.5 on the tensor cores.  Q4_K 4.1 / 5.0 / 5.2)
         return DENSE_GEMV_MAX_M
     if w.ggml_type == GGMLType.BF16:
@@ -482,7 +483,7 @@ def linear(a: Act, w: QuantWeight, *, bias: Optional[torch.Tensor] = None, resid
             y = y + residual.float()
         return y.to(out_dtype) if out_dtype != torch.float32 else y
     k = _k()
-    if T <= (DENSE_GEMV_MAX_M if a.b is None else 1) or (T <= GEMV_MAX_M and (a.b is None or w.experts != 1 or w.K % 8)) or T <= gemv_rows(w, act):
+    if (T <= DENSE_GEMV_MAX_M and (T <= 1 or T <= gemv_rows(w, act))) or (T <= GEMV_MAX_M and (a.b is None or w.experts != 1 or w.K % 8)):
         if w.uses_q8_activations:
             _ensure_q8(a)
             return k.gemv(w, xq=a.q, xds=a.ds, M=T, out_dtype=out_dtype, bias=bias, residual=residual, act=act)
@@ -511,8 +512,8 @@ def linear_multi(a: Act, ws, *, out_dtype=torch.float32):
     type); anything else is the plain sequence of ``linear`` calls."""
     ws = list(ws)
     T = a.T
-    if (ws[0].device.type == "cuda" and T <= (1 if a.b is not None and T > 1 and all(T > gemv_rows(w) for w in ws) else DENSE_GEMV_MAX_M) and 2 <= len(ws) <= 3 and all(w.experts == 1 and w.K == ws[0].K for w in ws)
-            and len({w.uses_q8_activations for w in ws}) == 1):
+    if (ws[0].device.type == "cuda" and T <= DENSE_GEMV_MAX_M and 2 <= len(ws) <= 3 and all(w.experts == 1 and w.K == ws[0].K for w in ws)
+            and len({w.uses_q8_activations for w in ws}) == 1 and (a.b is None or T <= 1 or any(T <= gemv_rows(w) for w in ws))):
         if ws[0].uses_q8_activations:
             _ensure_q8(a)
             y = _k().gemv_multi(ws, xq=a.q, xds=a.ds, M=T, out_dtype=out_dtype)

@@ -96,7 +96,7 @@ def test_the_number_of_rows_that_is_given_holds(recorder, monkeypatch, rows):
             assert (route(recorder, w, T) == "gemv") == (T <= rows), (t, T)
             recorder.calls.clear()
             F.linear_multi(F.Act(torch.randn(T, w.K).bfloat16()), [w, w])
-            assert (recorder.calls == ["gemv_multi"]) == (T <= min(rows, 8) or T <= rows), (t, T)
+            assert (recorder.calls == ["gemv_multi"]) == (T <= rows), (t, T)
 
 
 def test_the_switch_is_read():
