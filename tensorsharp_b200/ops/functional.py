@@ -461,6 +461,14 @@ def gemv_rows(w: QuantWeight, act: Optional[str] = None) -> int:
     return min(DENSE_GEMV_MAX_M, 1 if w.N * w.K >= 20 << 20 else 2)
 
 
+def _tma_rows(x: torch.Tensor) -> torch.Tensor:
+    """Rows as the tensor-core products read them, dense and on 16 bytes each: the GEMV takes any, so that few rows come in any form."""
+    if x.stride(1) == 1 and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0:
+        return x
+    x = x.contiguous().view(-1).view(x.shape)                # a single row may have any stride
+    return x if x.data_ptr() % 16 == 0 else x.clone()
+
+
 def linear(a: Act, w: QuantWeight, *, bias: Optional[torch.Tensor] = None, residual: Optional[torch.Tensor] = None,
            out_dtype=torch.float32, act: Optional[str] = None) -> torch.Tensor:
     """y = a @ w^T (+ bias) (+ residual), optional GLU over the row halves of ``w``
@@ -488,14 +496,15 @@ def linear(a: Act, w: QuantWeight, *, bias: Optional[torch.Tensor] = None, resid
             _ensure_q8(a)
             return k.gemv(w, xq=a.q, xds=a.ds, M=T, out_dtype=out_dtype, bias=bias, residual=residual, act=act)
         return k.gemv(w, xb=a.b.contiguous(), M=T, out_dtype=out_dtype, bias=bias, residual=residual, act=act)
+    x = _tma_rows(a.b) if T <= DENSE_GEMV_MAX_M else a.b
     if T <= BLOCK_GEMM_MAX_M and k.gemm_blocks_takes(w, act) and (residual is None or (residual.dtype == out_dtype and residual.is_contiguous())):
-        return k.gemm_blocks(w, a.b, out_dtype=out_dtype, bias=bias, residual=residual, act=act)
+        return k.gemm_blocks(w, x, out_dtype=out_dtype, bias=bias, residual=residual, act=act)
     wb = _dequant_scratch(w)
     if act is None:
-        return k.gemm_bf16(wb, a.b, out_dtype=out_dtype, bias=bias, residual=residual)
+        return k.gemm_bf16(wb, x, out_dtype=out_dtype, bias=bias, residual=residual)
     if T > PAIR_GEMM_MIN_M and act in GATED_ACTS and out_dtype == torch.bfloat16 and residual is None:
-        return k.gemm_bf16_glu(wb, a.b, act, bias=bias)
-    y = k.gemm_bf16(wb, a.b, out_dtype=torch.bfloat16, bias=bias)
+        return k.gemm_bf16_glu(wb, x, act, bias=bias)
+    y = k.gemm_bf16(wb, x, out_dtype=torch.bfloat16, bias=bias)
     half = w.N // 2
     if act in ("relu2", "silu"):
         out, _, _ = k.glu(y, None, act, w.N, w.N, 0, T)

@@ -111,3 +111,36 @@ def test_rows_without_a_bf16_form(recorder):
     x = torch.randn(9, 4096).bfloat16()
     F.linear(F.Act(None, x, x), LARGE[GGMLType.Q4_K])
     assert recorder.calls == ["gemv"]
+
+
+def forms(T, K):
+    """The same rows dense, with a stride that is no multiple of 16 bytes, off 16 bytes, transposed, and behind one another at any distance."""
+    x = torch.randn(T, K).bfloat16()
+    out = [x]
+    for stride, off in ((K + 3, 0), (K + 8, 5), (K + 1, 1)):
+        buf = torch.zeros(T * stride + off + 8, dtype=torch.bfloat16)
+        y = buf[off:].as_strided((T, K), (stride, 1))
+        out.append(y.copy_(x))
+    out.append(x.t().contiguous().t())
+    flat = torch.zeros(T * K + 1, dtype=torch.bfloat16)
+    flat[1:] = x.reshape(-1)
+    return out + [flat[1:].view(T, K)]
+
+
+@pytest.mark.parametrize("t", list(LARGE))
+@pytest.mark.parametrize("T", [1, 2, 3, 8])
+@pytest.mark.parametrize("act", [None, "relu2"])
+def test_few_rows_in_any_form(recorder, monkeypatch, t, T, act):
+    """Rows that the GEMV took in any form are made what the tensor cores read where they go there."""
+    w = weight(t, 2048, 2048) if t != GGMLType.BF16 else LARGE[t]
+    monkeypatch.setattr(Kernels, "glu", lambda self, y, up, act, n, s0, s1, T: (y.float().clamp(min=0).square(), None, None), raising=False)
+    monkeypatch.setattr(F, "gemv_rows", lambda *a: 1)
+    seen = set()
+    for x in forms(T, w.K):
+        recorder.calls.clear()
+        y = F.linear(F.Act(x), w, act=act)
+        seen.add(recorder.calls[-1])
+        assert y.shape == (T, w.N)
+        if act is None:
+            assert torch.allclose(y.float(), x.float() @ w.dequantize().float().t(), atol=1e-4, rtol=1e-5)
+    assert seen == {"gemv" if T == 1 else "gemm_bf16" if t == GGMLType.BF16 else "gemm_blocks"}
