@@ -444,21 +444,48 @@ def last_rows(h: torch.Tensor, batch: Batch) -> torch.Tensor:
     return h if batch.rows_in_order else h[batch.last_idx].contiguous()
 
 
-def gemv_rows(w: QuantWeight, act: Optional[str] = None) -> int:
-    """Most rows of bf16 activations for which a product goes to the GEMV kernels: two (one where the matrix is large) where the tensor cores
-    take the weight as it is, which costs the same for one row as for sixteen.  Measured, us for 1 / 2 / 3 / 4 / 8 rows (GEMV; tensor cores):
-    Q4_K 1024 x 2560 2.6 / 2.6 / 4.7 / 5.6 / 5.9; 4.8, 2560 x 4096 3.4 / 4.1 / 7.2 / 7.7 / 10.5; 6.2, 6144 x 2560 4.4 / 7.8 / 13.0 / 14.5 / 8.7; 7.5, 2 x 9728 x
-    2560 10.9 / 23.3 / 30.1 / 31.6 / 18.7; 16.8; Q6_K 2560 x 9728 7.6 / 12.4 / 20.7 / 20.9 / 59.8; 11.5; Q8_0 5376 x 21504 26.9 / 29.5 / 43.8 / 44.0 / 90.2; 27; bf16 2880 x
-    4096 7.5 / 9.0 / 12.8 / 12.8 / 21.8; 9.2, 32768 x 2880 29.8 / 36.2 / 56.4 / 58.0 / 102.8; 35."""
+def gemv_rows(w: QuantWeight, act: Optional[str] = None, takes: Optional[bool] = None) -> int:
+    """Most rows of bf16 activations for which a product goes to the GEMV kernels.  Where the tensor cores take the weight as it is, a product costs the same for
+    two rows as for sixteen, and the GEMV is the faster one for few rows or small matrices (``takes``: gemm_blocks_takes, where the caller has it).
+    Measured, weights from memory, us for 3 / 4 / 8 rows (GEMV; tensor cores for 4): Q4_K 512 x 512 2.4 / 2.6 / 2.2; 3.6, 1024 x 1024 2.6 / 2.8 / 4.5; 3.7, 2048 x 2048 4.6 /
+    4.9 / 7.2; 5.1, 1024 x 2560 5.1 / 5.8 / 9.5; 4.9, 6144 x 2560 14 / 16 / 10; 7.7, gated 4096 x 1024 5.8 / 6.4 / 6.4; 5.1; Q6_K 1024 x 1024 3.1 / 3.3 / 5.2; 3.5, 2560 x 1024 3.8 /
+    4.0 / 10.7; 4.5, 2048 x 2048 5.2 / 5.3 / 8.0; 5.1, 1024 x 2560 5.3 / 5.6 / 9.1; 4.8; Q8_0 1024 x 2560 3.1 / 3.2 / 4.7; 4.9, 2560 x 1024 2.5 / 2.6 / 5.9; 4.6, 2560 x 4096 5.8 /
+    5.8 / 13.6; 6.7, 4096 x 4096 10 / 10 / 15; 8.5, gated 512 x 2048 2.9 / 3.2 / 6.8; 3.9, gated 4096 x 2048 6.9 / 7.4 / 10; 7.0.  Two rows: Q4_K 2560 x 9728 8.8; 10.9, 9728 x 2560 11.8;
+    10.3, Q6_K 2560 x 9728 12.5; 11.9, Q8_0 5376 x 21504 29.5; 27.  bf16, whose tensor-core form has no activation of its own: 2048 x 2048 5.1 / 6.3 / 11.2; 6.5, 2560 x 4096 12 /
+    13 / 22; 9.6, gated 4096 x 2048 7.5 / 7.9 / 16; 9.7, gated 19456 x 2560 29 / 30 / 57; 32."""
     from ..gguf.constants import GGMLType
-    if GEMV_ROWS_GIVEN or w.experts != 1 or (w.ggml_type == GGMLType.Q8_0 and w.N * w.K < 1 << 20):
-        # (512 x 1024 of Q8_0, 3 / 5 / 8 rows 3.1 / 3.8 / 4.1 us with the rows' quantisation, which a norm brings along; 3.5 on the tensor cores.  Q4_K 4.1 / 5.0 / 5.2)
+    if GEMV_ROWS_GIVEN or w.experts != 1:
         return DENSE_GEMV_MAX_M
-    if w.ggml_type == GGMLType.BF16:
-        return min(DENSE_GEMV_MAX_M, 2) if w.N * w.K >= 4 << 20 and w.K % 8 == 0 and w.planes[0].data_ptr() % 16 == 0 else DENSE_GEMV_MAX_M
-    if not _k().gemm_blocks_takes(w, act):
+    n, gated, t = w.N * w.K, act in GATED_ACTS, w.ggml_type
+    if t == GGMLType.BF16:
+        if n < 4 << 20 or w.K % 8 or w.planes[0].data_ptr() % 16:
+            return DENSE_GEMV_MAX_M
+        return min(DENSE_GEMV_MAX_M, 4 if gated or n < 6 << 20 else 2)
+    if not (_k().gemm_blocks_takes(w, act) if takes is None else takes):
         return DENSE_GEMV_MAX_M
-    return min(DENSE_GEMV_MAX_M, 1 if w.N * w.K >= 20 << 20 else 2)
+    rows = 1 if n >= 20 << 20 and (w.N >= 4096 or t == GGMLType.Q6_K) else 2
+    if t == GGMLType.Q8_0:
+        if gated:
+            rows = 4 if n <= 2 << 20 else 3 if n <= 8 << 20 else rows
+        else:
+            rows = 8 if n < 1 << 20 or (n <= 4 << 20 and w.N <= 2048) else 4 if n <= 10 << 20 else rows
+    elif t == GGMLType.Q4_K:
+        if n <= 1 << 20:
+            rows = 8 if w.K <= 512 or (n <= 1 << 19 and w.K <= 1024) else 4 if w.K <= 2048 else rows
+        elif n <= 4 << 20 and w.K <= 2048 and not gated:
+            rows = 4
+    elif n < 3 << 20 and w.K <= 2048:
+        rows = 4
+    return min(DENSE_GEMV_MAX_M, rows)
+
+
+def block_rows(w: QuantWeight, act: Optional[str]) -> int:
+    """Most rows for which a product reads the blocks where it may; more read the bf16 copy.  Rows of one or two blocks leave the decoding nothing to be hidden behind:
+    us of 9 / 16 / 32 / 64 rows (blocks; copy) Q4_K 256 x 256 3.4 / 3.9 / 5.3 / 8.2; 3.4 / 3.5 / 3.6 / 4.7, 512 x 512 4.0 / 4.4 / 5.8 / 8.3; 5.3 / 5.4 / 5.7 / 6.7, 512 x 1024 3.7 / 4.3 / 4.9 /
+    6.5; 5.3 / 5.4 / 5.7 / 6.8; gated 1536 x 512 3.8 / 4.3 / 5.1 / 7.0; 7.1 / 7.2 / 7.5 / 8.7."""
+    if w.K > 512 or (w.K > 256 and act in GATED_ACTS):
+        return BLOCK_GEMM_MAX_M
+    return 40 if w.K > 256 or act in GATED_ACTS else 12
 
 
 def _tma_rows(x: torch.Tensor) -> torch.Tensor:
@@ -491,13 +518,14 @@ def linear(a: Act, w: QuantWeight, *, bias: Optional[torch.Tensor] = None, resid
             y = y + residual.float()
         return y.to(out_dtype) if out_dtype != torch.float32 else y
     k = _k()
-    if (T <= DENSE_GEMV_MAX_M and (T <= 1 or T <= gemv_rows(w, act))) or (T <= GEMV_MAX_M and (a.b is None or w.experts != 1 or w.K % 8)):
+    takes = 1 < T <= BLOCK_GEMM_MAX_M and k.gemm_blocks_takes(w, act)
+    if (T <= DENSE_GEMV_MAX_M and (T <= 1 or T <= gemv_rows(w, act, takes))) or (T <= GEMV_MAX_M and (a.b is None or w.experts != 1 or w.K % 8)):
         if w.uses_q8_activations:
             _ensure_q8(a)
             return k.gemv(w, xq=a.q, xds=a.ds, M=T, out_dtype=out_dtype, bias=bias, residual=residual, act=act)
         return k.gemv(w, xb=a.b.contiguous(), M=T, out_dtype=out_dtype, bias=bias, residual=residual, act=act)
     x = _tma_rows(a.b) if T <= DENSE_GEMV_MAX_M else a.b
-    if T <= BLOCK_GEMM_MAX_M and k.gemm_blocks_takes(w, act) and (residual is None or (residual.dtype == out_dtype and residual.is_contiguous())):
+    if takes and T <= block_rows(w, act) and (residual is None or (residual.dtype == out_dtype and residual.is_contiguous())):
         return k.gemm_blocks(w, x, out_dtype=out_dtype, bias=bias, residual=residual, act=act)
     wb = _dequant_scratch(w)
     if act is None:
@@ -522,7 +550,7 @@ def linear_multi(a: Act, ws, *, out_dtype=torch.float32):
     ws = list(ws)
     T = a.T
     if (ws[0].device.type == "cuda" and T <= DENSE_GEMV_MAX_M and 2 <= len(ws) <= 3 and all(w.experts == 1 and w.K == ws[0].K for w in ws)
-            and len({w.uses_q8_activations for w in ws}) == 1 and (a.b is None or T <= 1 or any(T <= gemv_rows(w) for w in ws))):
+            and len({w.uses_q8_activations for w in ws}) == 1 and (a.b is None or T <= 1 or sum(w.N for w in ws) * ws[0].K <= 8 << 20 or any(T <= gemv_rows(w) for w in ws))):
         if ws[0].uses_q8_activations:
             _ensure_q8(a)
             y = _k().gemv_multi(ws, xq=a.q, xds=a.ds, M=T, out_dtype=out_dtype)

@@ -144,3 +144,51 @@ def test_few_rows_in_any_form(recorder, monkeypatch, t, T, act):
         if act is None:
             assert torch.allclose(y.float(), x.float() @ w.dequantize().float().t(), atol=1e-4, rtol=1e-5)
     assert seen == {"gemv" if T == 1 else "gemm_bf16" if t == GGMLType.BF16 else "gemm_blocks"}
+
+
+# (type, N, K, activation) -> us with 2, 3, 4, 8, 16 and 64 rows: the GEMV (more than eight: the bf16 copy), and the tensor cores on the weight as it is
+ROWS = (2, 3, 4, 8, 16, 64)
+MEASURED = {
+    ("Q4_K", 256, 256, None): [(1.5, 2.7), (2.3, 2.8), (2.6, 2.9), (1.7, 3.2), (3.5, 3.9), (4.7, 8.2)],
+    ("Q4_K", 512, 512, None): [(1.7, 3.4), (2.4, 3.6), (2.6, 3.6), (2.2, 4.0), (5.4, 4.4), (6.7, 8.3)],
+    ("Q4_K", 512, 1024, None): [(1.7, 3.6), (2.5, 3.6), (2.7, 3.6), (3.1, 3.7), (5.4, 4.3), (6.8, 6.5)],
+    ("Q4_K", 1024, 1024, None): [(1.7, 3.7), (2.6, 3.6), (2.8, 3.7), (4.5, 3.8), (5.5, 4.4), (7.0, 6.5)],
+    ("Q4_K", 2048, 2048, None): [(2.7, 5.0), (4.6, 5.1), (4.9, 5.1), (7.2, 5.2), (7.5, 5.3), (9.3, 6.6)],
+    ("Q4_K", 1024, 2560, None): [(2.8, 4.9), (5.0, 4.8), (5.8, 4.9), (9.5, 4.9), (6.4, 5.7), (8.2, 8.0)],
+    ("Q4_K", 6144, 2560, None): [(8.6, 7.7), (13.9, 7.7), (15.6, 7.7), (10.2, 7.9), (10.7, 8.5), (13.3, 11.0)],
+    ("Q4_K", 2560, 9728, None): [(8.7, 10.9), (16.1, 11.0), (17.6, 11.0), (31.2, 11.1), (13.5, 11.3), (15.6, 13.7)],
+    ("Q4_K", 1536, 512, "swiglu"): [(2.3, 3.8), (2.8, 3.8), (3.1, 3.8), (3.9, 3.8), (7.2, 4.3), (8.7, 7.0)],
+    ("Q6_K", 1024, 1024, None): [(1.9, 3.5), (3.1, 3.5), (3.3, 3.5), (5.2, 3.6), (5.5, 4.2), (7.0, 6.4)],
+    ("Q6_K", 2560, 1024, None): [(2.5, 4.2), (3.8, 4.5), (4.0, 4.5), (10.7, 4.5), (6.0, 5.2), (8.0, 7.3)],
+    ("Q6_K", 2560, 9728, None): [(12.5, 11.9), (20.6, 12.1), (20.9, 12.1), (59.8, 12.2), (13.7, 12.4), (15.7, 14.8)],
+    ("Q8_0", 1024, 1024, None): [(1.7, 3.5), (1.9, 3.6), (1.9, 3.6), (2.8, 3.7), (5.5, 4.2), (7.0, 6.5)],
+    ("Q8_0", 1024, 2560, None): [(2.8, 4.9), (3.1, 4.9), (3.2, 4.9), (4.7, 4.9), (6.4, 5.7), (8.2, 8.0)],
+    ("Q8_0", 2560, 4096, None): [(4.2, 6.6), (5.8, 6.7), (5.8, 6.7), (13.6, 6.9), (9.5, 7.0), (11.5, 8.9)],
+    ("Q8_0", 4096, 4096, None): [(7.4, 8.4), (10.0, 8.5), (10.2, 8.5), (15.5, 8.6), (11.2, 8.8), (13.1, 10.7)],
+    ("Q8_0", 4096, 2048, "swiglu"): [(4.7, 6.7), (6.9, 6.9), (7.4, 7.0), (10.0, 7.1), (10.0, 7.3), (12.2, 9.1)],
+    ("BF16", 2048, 2048, None): [(4.1, 6.4), (5.1, 6.5), (6.3, 6.5), (11.2, 7.1), (7.6, 7.6), (9.3, 9.3)],
+    ("BF16", 4096, 4096, None): [(9.6, 10.7), (13.0, 10.8), (13.5, 10.9), (23.1, 11.2), (11.4, 11.4), (13.3, 13.3)],
+    ("BF16", 19456, 2560, "swiglu"): [(21.6, 32.0), (29.2, 31.9), (30.3, 32.2), (57.3, 32.3), (32.7, 32.7), (36.3, 36.3)],
+}
+
+
+@pytest.mark.parametrize("name,N,K,act", list(MEASURED))
+def test_no_slower_than_the_general_kernels(name, N, K, act):
+    t = GGMLType[name]
+    w = QuantWeight(t, N, K, [torch.empty(0, dtype=torch.uint8)] * 4)
+    for T, (general, blocks) in zip(ROWS, MEASURED[name, N, K, act]):
+        takes = t != GGMLType.BF16
+        on_blocks = T > F.gemv_rows(w, act, takes) if T <= 8 else takes and T <= F.block_rows(w, act)
+        assert (blocks if on_blocks else general) <= 1.03 * general, T
+        assert T > 2 or not on_blocks or blocks <= general
+
+
+def test_the_route_is_worked_out_once(recorder):
+    for T, most in ((1, 0), (2, 1), (5, 1), (9, 1), (64, 1), (65, 0), (300, 0)):
+        for t in (GGMLType.Q4_K, GGMLType.Q8_0):
+            recorder.asked = 0
+            w = LARGE[t]
+            F.linear(F.Act(torch.randn(T, w.K).bfloat16()), w)
+            ours = recorder.calls.count("gemm_blocks")             # the recorder's own check of what it is given
+            recorder.calls.clear()
+            assert recorder.asked - ours <= most, (t, T)
