@@ -25,9 +25,6 @@ from ..quant.qweight import QuantWeight
 from . import reference as ref
 
 BLOCK_GEMM_MAX_M = 64  # up to this many rows the weights' bytes are the bound, and the tensor cores read the GGUF blocks themselves
-# Routed pairs up to which MXFP4 experts go to the GEMV of one pair each: measured, a layer of 32 experts of 2880 x 2880 (us, GEMV / tensor cores): 4 pairs
-# 46 / 53, 8 72 / 72, 12 97 / 85, 16 122 / 99, 32 220 / 131, 64 420 / 165
-EXPERT_GEMV_PAIRS = 8
 PAIR_GEMM_MIN_M = 64  # above this many rows the tensor-core GEMM is the one that can end with the gated activation
 GATED_ACTS = ("swiglu", "geglu", "geglu_tanh", "geglu_erf", "swiglu_oai")
 GEMV_MAX_M = 16   # "small batch": token count up to which the models take their decode-style paths (int8 activations, mailbox exchanges)
@@ -1200,6 +1197,17 @@ def moe_expert_parts(a: Act, ids: torch.Tensor, weights: torch.Tensor, gate_up: 
     return MoeParts(y2, k, pos, wts, flat_ids)
 
 
+def expert_blocks(pairs: int, gate_up: QuantWeight, down: QuantWeight) -> bool:
+    """Whether MXFP4 experts that the tensor cores take go there, by the values of one expert: elsewhere up to 64 pairs go to the GEMV of one pair each and more to the
+    tile kernels of csrc/moe.cu.  A layer by 8 / 16 / 32 / 64 / 128 / 512 pairs, us (those; tensor cores): 32 experts of 2880 x 2880 71 / 122 / 224 / 430 / 232 / 390; 84 / 102 /
+    150 / 181 / 210 / 234, 8 of 4096 x 4096 108 / 199 / 373 / 719 / 241 / 696; 96 / 132 / 134 / 136 / 140 / 276, 128 of 768 x 2048 33 / 48 / 75 / 132 / 135 / 198; 45 / 52 / 71 / 96 /
+    125 / 184, 64 of 512 x 1024 25 / 32 / 45 / 73 / 47 / 68; 34 / 36 / 37 / 48 / 53 / 67, 16 of 256 x 512 20 / 24 / 30 / 44 / 31 / 40; 29 / 30 / 30 / 32 / 33 / 46."""
+    values = gate_up.N * gate_up.K + down.N * down.K
+    if pairs > 4 * GEMV_MAX_M:
+        return values >= 2 << 20 or (pairs >= 512 and values >= 1 << 20)
+    return pairs > (8 if values >= 8 << 20 else 20 if values >= 1 << 20 else 32)
+
+
 def moe_experts(a: Act, ids: torch.Tensor, weights: torch.Tensor, gate_up: QuantWeight, down: QuantWeight, *,
                 act: str, gate_up_bias: Optional[torch.Tensor] = None, down_bias: Optional[torch.Tensor] = None,
                 expert_offset: int = 0, down_scale: Optional[torch.Tensor] = None, push=None,
@@ -1228,9 +1236,9 @@ def moe_experts(a: Act, ids: torch.Tensor, weights: torch.Tensor, gate_up: Quant
     local = ids - expert_offset
     if expert_offset != 0 or E_local != int(1e9):
         local = torch.where((local >= 0) & (local < E_local), local, torch.full_like(local, -1))
-    blocks = (dev.type == "cuda" and push is None and a.b is not None and a.b.dtype == torch.bfloat16
+    blocks = (dev.type == "cuda" and push is None and a.b is not None and a.b.dtype == torch.bfloat16 and expert_blocks(T * k, gate_up, down)
               and _k().gemm_experts_takes(gate_up, act if glu_act or act == "relu2" else "silu") > 0 and _k().gemm_experts_takes(down) > 0)
-    if dev.type == "cuda" and T * k <= (EXPERT_GEMV_PAIRS if blocks else 4 * GEMV_MAX_M):
+    if dev.type == "cuda" and T * k <= 4 * GEMV_MAX_M and not blocks:
         kk = _k()
         flat = local.reshape(-1).contiguous()
         if gate_up.uses_q8_activations:
