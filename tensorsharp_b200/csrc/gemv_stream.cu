@@ -525,14 +525,28 @@ static int stream_mode() {
     return mode;
 }
 
-static bool q6k_ok(const GemvArgs& a, bool glu) {
-    const int nb = a.w.K >> 8;
-    return a.w.type == TSB_Q6_K && !glu && a.M == 1 && nb >= 2 && nb % 2 == 0 && nb <= 64 && a.w.N >= 64;
+// Whether a second round of groups would have less than a fifth of the warps at work, rows of up to 4096 values: such a matrix is twice the time of a group with
+// most of the chip idle, and the row-per-warp kernel is the faster one for Q6_K and Q8_0.  Measured behind a norm, us of both (this pipeline; a row per
+// warp): Q8_0 4096 x 4096 7.3; 6.5, 8192 x 2048 7.3; 6.8, gated 4096 x 1024 4.3; 3.7, gated 4096 x 2048 5.3; 4.3, Q6_K 4096 x 4096 7.8; 7.1, 8192 x 2048 7.8; 7.5; a second round that
+// is half full Q8_0 5120 x 1024 4.3; 5.0, 5376 x 4096 pays.  (Q4_K 4096 x 4096 6.3; 6.4.)
+static bool rows_second_round_idle(const GemvArgs& a, bool glu, int block_bytes) {
+    const int nb = a.w.K >> 8, rows = nb > 4 && nb <= 12 && a.w.N >= 148 * ROWS_PER_SM * 4 * 4 ? 4 : 2;
+    if (nb > 16) return false;
+    const size_t smem = (size_t)((rows * nb * block_bytes + 127) & ~127) * ROWS_D * 4;
+    const int fit = (int)((226 * 1024) / (smem + 1024)), warps = 148 * 4 * (fit < 1 ? 1 : fit > ROWS_PER_SM ? ROWS_PER_SM : fit);
+    const int per = glu ? rows / 2 : rows, groups = (a.n_out + per - 1) / per;
+    return groups > warps && 5 * (groups - warps) <= warps;
 }
 
-static bool q8_ok(const GemvArgs& a) {
+static bool q6k_ok(const GemvArgs& a, bool glu) {
+    const int nb = a.w.K >> 8;
+    return a.w.type == TSB_Q6_K && !glu && a.M == 1 && nb >= 2 && nb % 2 == 0 && nb <= 64 && a.w.N >= 64 &&
+           !rows_second_round_idle(a, glu, rows_block_bytes(ROWS_Q6));
+}
+
+static bool q8_ok(const GemvArgs& a, bool glu) {
     return a.w.type == TSB_Q8_0 && a.M == 1 && a.w.K % 256 == 0 && a.w.K <= 96 * 256 && a.w.N >= 64 &&
-           ((reinterpret_cast<uintptr_t>(a.w.p0) | reinterpret_cast<uintptr_t>(a.w.p1)) & 15) == 0;
+           ((reinterpret_cast<uintptr_t>(a.w.p0) | reinterpret_cast<uintptr_t>(a.w.p1)) & 15) == 0 && !rows_second_round_idle(a, glu, rows_block_bytes(ROWS_Q8));
 }
 
 static bool fast_ok(const GemvArgs& a) {
@@ -563,7 +577,7 @@ bool tsb_gemv_stream_eligible(const GemvArgs& a) {
     const int mode = stream_mode();
     if (!mode || a.ids || a.M > 4 || a.M < 1) return false;
     const bool glu = a.act >= ACT_SWIGLU && a.act <= ACT_SWIGLU_OAI;
-    if ((fast_ok(a) || q8_ok(a)) && !(glu && a.push)) return true;
+    if ((fast_ok(a) || q8_ok(a, glu)) && !(glu && a.push)) return true;
     if (q6k_ok(a, glu)) return true;
     if (a.push || mode < 2 || (a.w.type != TSB_Q4_K && a.w.type != TSB_Q5_K)) return false;
     const size_t rowbytes = (size_t)(a.w.K >> 8) * (a.w.type == TSB_Q5_K ? 176 : 144);
@@ -572,7 +586,7 @@ bool tsb_gemv_stream_eligible(const GemvArgs& a) {
 
 int tsb_gemv_stream_launch(const GemvArgs& a, bool glu, cudaStream_t s) {
     if (fast_ok(a)) return glu ? launch_rows_any<ROWS_Q4, true>(a, s) : launch_rows_any<ROWS_Q4, false>(a, s);
-    if (q8_ok(a)) return glu ? launch_rows_any<ROWS_Q8, true>(a, s) : launch_rows_any<ROWS_Q8, false>(a, s);
+    if (q8_ok(a, glu)) return glu ? launch_rows_any<ROWS_Q8, true>(a, s) : launch_rows_any<ROWS_Q8, false>(a, s);
     if (q6k_ok(a, glu)) return launch_rows_any<ROWS_Q6, false>(a, s);
     const bool q5 = a.w.type == TSB_Q5_K;
     const size_t rowbytes = (size_t)(a.w.K >> 8) * (q5 ? 176 : 144);
