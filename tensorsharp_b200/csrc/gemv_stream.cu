@@ -458,14 +458,16 @@ static int launch_rows(const GemvArgs& a, int max_blocks, cudaStream_t s) {
 
 // Four rows to a warp where that leaves every warp a group of some length (and a lane's activations, 16 registers a unit, stay at six units), two otherwise:
 // 2 x 9728 x 2560 6.8 us with four rows and 7.4 with two, 32768 x 2560 of Q6_K 13.4 and 14.2; 6144 x 2560 4.2 and 3.6, 2560 x 9728 5.5 and 4.7 (Q6_K
-// 7.5 and 6.3).  Rows longer than 6144 values are split over the CTA.
+// 7.5 and 6.3).  Not where a second round of groups would have less than a fifth of the warps at work: behind a norm, us of four rows; two, 8192 x 2048 6.3; 5.5
+// (Q6_K 7.8; 6.8, Q8_0 7.3; 6.2), 8448 x 3072 8.2; 6.5 (10.1; 8.2, 7.6; 7.4).  Rows longer than 6144 values are split over the CTA.
 template <int TY, bool GLU>
 static int launch_rows_any(const GemvArgs& a, cudaStream_t s) {
     const int nb = a.w.K >> 8;
 #define TSB_ROWS(RV, JV, KSV) return launch_rows<TY, GLU, RV, JV, KSV>(a, mb, s)
     if (nb <= 24) {
         const int mb = nb;
-        if (nb > 4 && nb <= 12 && a.w.N >= 148 * ROWS_PER_SM * 4 * 4) {
+        const int quads = (a.w.N + 3) / 4, warps = 148 * ROWS_PER_SM * 4;
+        if (nb > 4 && nb <= 12 && quads >= warps && 5 * (quads - warps) > warps) {
             switch ((mb + 1) / 2) {
             case 3: TSB_ROWS(4, 3, 1);
             case 4: TSB_ROWS(4, 4, 1);
@@ -527,10 +529,10 @@ static int stream_mode() {
 
 // Whether a second round of groups would have less than a fifth of the warps at work, rows of up to 4096 values: such a matrix is twice the time of a group with
 // most of the chip idle, and the row-per-warp kernel is the faster one for Q6_K and Q8_0.  Measured behind a norm, us of both (this pipeline; a row per
-// warp): Q8_0 4096 x 4096 7.3; 6.5, 8192 x 2048 7.3; 6.8, gated 4096 x 1024 4.3; 3.7, gated 4096 x 2048 5.3; 4.3, Q6_K 4096 x 4096 7.8; 7.1, 8192 x 2048 7.8; 7.5; a second round that
+// warp): Q8_0 4096 x 4096 7.3; 6.5, gated 4096 x 1024 4.3; 3.7, gated 4096 x 2048 5.3; 4.3, Q6_K 4096 x 4096 7.8; 7.1; a second round that
 // is half full Q8_0 5120 x 1024 4.3; 5.0, 5376 x 4096 pays.  (Q4_K 4096 x 4096 6.3; 6.4.)
 static bool rows_second_round_idle(const GemvArgs& a, bool glu, int block_bytes) {
-    const int nb = a.w.K >> 8, rows = nb > 4 && nb <= 12 && a.w.N >= 148 * ROWS_PER_SM * 4 * 4 ? 4 : 2;
+    const int nb = a.w.K >> 8, rows = 2;                                 // (four rows: launch_rows_any takes two in that case)
     if (nb > 16) return false;
     const size_t smem = (size_t)((rows * nb * block_bytes + 127) & ~127) * ROWS_D * 4;
     const int fit = (int)((226 * 1024) / (smem + 1024)), warps = 148 * 4 * (fit < 1 ? 1 : fit > ROWS_PER_SM ? ROWS_PER_SM : fit);
