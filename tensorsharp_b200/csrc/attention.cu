@@ -402,6 +402,13 @@ static unsigned* attn_ticket_for_current_device() {
     return g_attn_ticket_ptr[dev];
 }
 
+// TSB_ATTN_MMA=0 keeps the CUDA-core kernels for every shape, TSB_ATTN_MMA_MIN_CTAS=n for grids of fewer than n CTAs.
+static bool attn_decode_takes_mma(const AttnArgs& a) {
+    static const bool mma_on = []() { const char* e = getenv("TSB_ATTN_MMA"); return !e || atoi(e) != 0; }();
+    static const long mma_min_ctas = []() { const char* e = getenv("TSB_ATTN_MMA_MIN_CTAS"); return e ? atol(e) : 1L; }();
+    return mma_on && (long)a.splits * a.Hkv * a.B >= mma_min_ctas && tsb_attn_decode_mma_supported(a);
+}
+
 // `allow_fused`: whether this call may use the in-kernel split merge (and with it the shared arrival tickets).
 static int attn_decode_impl(const AttnArgs* args, void* stream, bool allow_fused) {
     AttnArgs a = *args;
@@ -428,11 +435,8 @@ static int attn_decode_impl(const AttnArgs* args, void* stream, bool allow_fused
     }
     // Head sizes 64 / 128 with up to 16 query heads per KV head: Q K^T and P V on the tensor cores, the query heads of a
     // KV head as the rows of one tile (attention_decode_mma.cu).  Measured on the Qwen3-4B shape: one sequence 2.015 ->
-    // 1.750 ms per step, 16 sequences 5.76 -> 4.48 ms.  TSB_ATTN_MMA=0 keeps the CUDA-core kernels for every shape,
-    // TSB_ATTN_MMA_MIN_CTAS=n for grids of fewer than n CTAs.
-    static const bool mma_on = []() { const char* e = getenv("TSB_ATTN_MMA"); return !e || atoi(e) != 0; }();
-    static const long mma_min_ctas = []() { const char* e = getenv("TSB_ATTN_MMA_MIN_CTAS"); return e ? atol(e) : 1L; }();
-    if (mma_on && (long)a.splits * a.Hkv * a.B >= mma_min_ctas && tsb_attn_decode_mma_supported(a)) {
+    // 1.750 ms per step, 16 sequences 5.76 -> 4.48 ms.
+    if (attn_decode_takes_mma(a)) {
         a.ticket = nullptr;
         bool merged = false;
         rc = tsb_attn_decode_mma_launch(a, s, &merged);
@@ -467,6 +471,12 @@ static int attn_decode_impl(const AttnArgs* args, void* stream, bool allow_fused
 }
 
 extern "C" int tsb_attn_decode(const AttnArgs* args, void* stream) { return attn_decode_impl(args, stream, true); }
+
+// Whether a split's result is the result, without a merge launch: the kernel that loads ahead with one part a sequence.
+extern "C" int tsb_attn_decode_is_one_launch(const AttnArgs* args) {
+    const AttnArgs& a = *args;
+    return !attn_needs_vd(a) && attn_decode_takes_mma(a) && a.page_size % 16 == 0 && a.splits == 1 && a.plan == nullptr && a.gate == nullptr;
+}
 
 // The merge of the split partials on its own, for split kernels that live in other translation units.
 extern "C" int tsb_attn_combine(const AttnArgs* args, void* stream) {

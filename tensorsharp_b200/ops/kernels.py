@@ -625,7 +625,10 @@ def attn_decode(q, k_cache, v_cache, block_table, kv_lens, *, scale, Hq, Hkv, Dh
         lib.tsb_attn_decode_fp8.restype = C.c_int
         native.check(lib.tsb_attn_decode_fp8(C.byref(a), _stream()), "attn_decode_fp8")
     else:
-        native.check(_lib().tsb_attn_decode(C.byref(a), _stream()), "attn_decode")
+        lib = _lib()
+        native.check(lib.tsb_attn_decode(C.byref(a), _stream()), "attn_decode")
+        if splits == 1 and lib.tsb_attn_decode_is_one_launch(C.byref(a)):
+            _count(-1)
     _count(2)
     return (out, oq, ods) if want_q8 else out
 

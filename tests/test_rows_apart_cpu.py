@@ -40,8 +40,8 @@ def test_who_reads_ahead(monkeypatch, apart, told, as_act):
             seen.append(args._obj.ahead)
             return 0
 
-        def tsb_attn_decode_launches(self, args):
-            return 2
+        def tsb_attn_decode_is_one_launch(self, args):
+            return 0
     monkeypatch.setattr(kernels, "_lib", lambda: Lib())
     monkeypatch.setattr(kernels, "_stream", lambda: C.c_void_p(0))
 
@@ -55,3 +55,14 @@ def test_who_reads_ahead(monkeypatch, apart, told, as_act):
     F.attention(q, cache, cache, batch, scale=0.1, Hq=4, Hkv=2, Dh=64, as_act=as_act, **({} if told is None else dict(ahead=told)))
     kernels.attn_decode(q, cache, cache, batch.block_table, batch.kv_lens, scale=0.1, Hq=4, Hkv=2, Dh=64, page_size=64, splits=1)
     assert seen == [int(bool(told) and apart), 0]
+
+
+@pytest.mark.skipif(not kernels.native.available(), reason="the kernel library is not built here")
+@pytest.mark.parametrize("kw,one", [(dict(), True), (dict(splits=2), False), (dict(page_size=24), False), (dict(Dh=256, Dv=256), False), (dict(gate=64), False),
+                                    (dict(k_ld=1024), False), (dict(plan=64, parts=9, each=1), False)])
+def test_launches_of_a_step(kw, one):
+    """The launch count asks the library, by a host function that follows no pointer."""
+    a = kernels.AttnArgs()
+    for k, v in {**dict(B=2, Hq=8, Hkv=2, Dh=128, Dv=128, page_size=64, splits=1), **kw}.items():
+        setattr(a, k, v)
+    assert bool(kernels._lib().tsb_attn_decode_is_one_launch(C.byref(a))) is one
