@@ -131,3 +131,20 @@ def test_even_lengths_are_cut_as_each_alone(Hq, Hkv, Dh, lens):
     each = F.decode_parts(batch, Hkv, 0)[1]
     alone = F._k().attn_decode(q, k, v, batch.block_table, batch.kv_lens, scale=0.1, Hq=Hq, Hkv=Hkv, Dh=Dh, page_size=64, splits=each, split_len=-128)
     assert torch.equal(got.view_as(alone), alone)
+
+
+# every warp goes round its ring of three chunks many times; bounds as above, for each sequence and head
+@pytest.mark.parametrize("Hq,Hkv,Dh", [(32, 8, 128), (64, 8, 64), (16, 1, 64)])
+@pytest.mark.parametrize("page", [16, 64])
+@pytest.mark.parametrize("window", [0, 900])
+@pytest.mark.parametrize("splits,split_len", [(1, 0), (2, 0), (2, -128), (1, 3072)])
+def test_long_parts(Hq, Hkv, Dh, page, window, splits, split_len):
+    if window and split_len > 0:
+        pytest.skip("a fixed split length goes with no window")
+    torch.manual_seed(6)
+    batch, rows = decode_batch([500, 777, 1023, 1024, 1025, 2048, 3000], page)
+    k, v = (torch.randn(rows, Hkv, Dh, device=DEV).bfloat16() for _ in range(2))
+    q = torch.randn(7, Hq, Dh, device=DEV).bfloat16()
+    got = F._k().attn_decode(q, k, v, batch.block_table, batch.kv_lens, scale=Dh ** -0.5, Hq=Hq, Hkv=Hkv, Dh=Dh, page_size=page, splits=splits, split_len=split_len,
+                             window=window)
+    assert worst(got, exact(q, k, v, batch, Dh ** -0.5, window)) < 5e-3
