@@ -1,4 +1,6 @@
-// Chunked GatedDeltaNet prefill: the part that has to run chunk after chunk, as one kernel.
+// Chunked prefill of the linear-attention layers: GatedDeltaNet from a layer's packed projections (the second half of this file), Mamba2, and first the kernel that
+// carries a state over chunks whose operands are there already: Mamba2 takes it (with no correction, U_c = U0_c), and the delta rule where its own kernels are
+// turned off and the chunk algebra runs as tensor ops.
 //
 // In the chunked (WY) form of the delta rule the work inside a chunk of 64 tokens is batched matrix algebra over
 // (heads x chunks) that has no dependency between chunks (the decay mask, K K^T, the unit-triangular solve, Q K^T);

@@ -1,6 +1,6 @@
-// Products of 9 to 64 rows with weights in GGUF blocks, on the 5th-generation tensor cores:
+// Products of up to 64 rows (dispatched from two or three) with weights in GGUF blocks, on the 5th-generation tensor cores:
 //   Y[t, n] = sum_k X[t, k] * W[n, k]  (+ bias[n]) (+ residual[t, n]), or the gated activation of two row halves of W,
-// and the same for tiles of up to 32 rows of the experts of a mixture (gemm_experts below).
+// and the same for tiles of up to 64 rows of the experts of a mixture (gemm_experts below).
 //
 // So few rows are bound by the bytes of the weights, so the blocks themselves are read (0.56 bytes a weight in Q4_K where a
 // bf16 copy has two) and never leave the SM in another form: a warp decodes them in registers and stores the bf16 values to
@@ -13,7 +13,7 @@
 //   warp 2      TMA of X, one slot at a time
 //   warps 3-10  decode: two sets of four warps take the slots in turn, a thread owns one weight row (one lane of tensor
 //               memory); they are the epilogue too
-// Bound by what decoding issues, not by the bytes.  The first three warps sleep between their polls, of five instructions each (polling as
+// Bound by what decoding issues, not by the bytes.  The first three warps sleep between their polls, of five instructions each (tc::hold; polling as
 // tc::mbar_wait does they took half of the issue slots; one warp for all three is too slow a chain).  They run with all their lanes and
 // elect one for what a single thread issues: with a branch on the lane the products took 620 cycles a slab to issue.
 // Two CTAs fit an SM.  Dense products split K over the CTAs of a cluster, which add their parts through distributed shared
@@ -23,7 +23,7 @@
 // scales ahead of that); MXFP4 values are exact in bf16.
 //
 // Measured, us per launch in a row (the bf16 copy through gemm_bf16_kernel, with its split-K and activation kernels / this one): Q4_K, 16 rows,
-// 6144 x 2560 11.0 / 8.5, 2560 x 4096 9.6 / 6.6, 2 x 9728 x 2560 with SwiGLU 31.7 / 17.8, 2560 x 9728 13.7 / 11.0, 1024 x 2560 5.9 / 5.6; 64 rows 13.6 /
+// 6144 x 2560 11.0 / 8.5, 2560 x 4096 9.6 / 6.6, 2 x 9728 x 2560 with SwiGLU 31.7 / 17.8 (18.7 from memory), 2560 x 9728 13.7 / 11.0, 1024 x 2560 5.9 / 5.6; 64 rows 13.6 /
 // 10.9, 11.5 / 8.6, 35.1 / 23.3, 15.7 / 13.3, 7.8 / 7.9; Q6_K, 16 rows, 32768 x 2560 32.3 / 22.9; Q8_0, 16 rows, 5376 x 21504 41.8 / 27.5.  A layer of 32
 // MXFP4 experts of 2880 x 2880 with its routing (the int8 kernels of moe.cu / this one): 68 pairs 185 / 166, 256 254 / 194, 512 386 / 200, 1024 620 / 237.
 #include <cudaTypedefs.h>

@@ -496,7 +496,10 @@ def _tma_rows(x: torch.Tensor) -> torch.Tensor:
 def linear(a: Act, w: QuantWeight, *, bias: Optional[torch.Tensor] = None, residual: Optional[torch.Tensor] = None,
            out_dtype=torch.float32, act: Optional[str] = None) -> torch.Tensor:
     """y = a @ w^T (+ bias) (+ residual), optional GLU over the row halves of ``w``
-    (rows [0, N/2) gate, [N/2, N) up).  ``residual`` is added in the output dtype."""
+    (rows [0, N/2) gate, [N/2, N) up).  ``residual`` is added in the output dtype.
+
+    On the GPU the operands are rounded by route: the GEMV multiplies the weights' codes as they are by rows rounded to eight bits in groups of 32, the tensor cores
+    (:func:`gemv_rows`, :func:`block_rows`) decoded weights rounded to bf16 by bf16 rows as they are, which is the nearer one to 64 bits of the two."""
     T = a.T
     if w.device.type == "cuda" and a.b is not None and a.b.dtype == torch.float32:      # a model that runs in 32 bits
         y = _k().gemm_f32(w, a.b, bias=bias)

@@ -248,7 +248,7 @@ def gather_bf16_rows(x: torch.Tensor, order: torch.Tensor, div: int) -> torch.Te
 
 
 def expert_tile_rows(most: int, P: int, E: int) -> int:
-    """Rows of a tile of :func:`gemm_experts` for P pairs over E experts: twice the average and more, so that most experts' weights are
+    """Rows of a tile of :func:`gemm_experts` for P pairs over E experts (32 or 64; its tiles of 16 are for callers of their own): twice the average and more, so that most experts' weights are
     decoded once.  Measured, a layer of 32 experts of 2880 x 2880 (us; tiles of 16 / 32 / 64): 256 pairs 194 / 194 / 201, 512 280 / 200 / 211, 768
     342 / 224 / 225, 1024 433 / 305 / 237."""
     return min(most, 32 if P <= 16 * E else 64)
@@ -259,7 +259,7 @@ def moe_grouped(*, xq=None, xds=None, xb=None, ids: torch.Tensor, weights: torch
     """Grouped expert projections with the routing kept on the device (no host read-back, fixed launch
     sequence): group the (token, slot) pairs by local expert, gather activations into that order, run
     gate/up and down as tile GEMVs (each tile streams its expert's rows once for up to 8 pairs, 16 in 4-bit blocks) or, where
-    the experts are MXFP4 and bf16 rows are given, as tensor-core products of tiles of 16 to 64 pairs, and
+    the experts are MXFP4 and bf16 rows are given, as tensor-core products of tiles of 32 or 64 pairs, and
     sum every token's slots.  ``ids`` are global expert ids [T, k]; pairs whose expert is not in
     ``[expert_offset, expert_offset + gate_up.experts)`` contribute nothing.  Returns f32 [T, D]."""
     lib = _lib()
