@@ -13,7 +13,6 @@ Data conventions
 """
 from __future__ import annotations
 
-import functools
 import math
 import os
 from dataclasses import dataclass, field
@@ -1333,17 +1332,14 @@ def moe_tile_list(flat: torch.Tensor, n_groups: int, bn: int):
     return order, tiles.contiguous()
 
 
-@functools.lru_cache(maxsize=1024)
 def _pair_tile(avg: int) -> int:
-    """Token tile of the grouped pair GEMM for groups of ``avg`` rows: the cost per useful row, from the kernel's cost of a tile
-    (csrc/gemm_tcgen05.cu: gemm_cost) and half an empty tile per group.  Half a tile is what groups of far apart sizes leave empty, as trained routers make
-    them; tiles that the average fills well gain little where all groups are alike and lose elsewhere.  Measured, an expert layer (us) with a tile for groups
-    that spread by 1.8 times the root of their average / this one, sizes spread by 1, by 13 to 18, by 28 to 30 and by 43 to 57 times that root: 256
-    experts of 2 x 512 x 2048, groups of 71 rows 446 / 447, 507 / 492, 499 / 466, 390 / 344, of 256 896 / 885, 920 / 868, 925 / 868, 818 / 740; 32 of 2 x 2880 x
-    2880, of 287 724 / 706, 750 / 673, 743 / 707, 735 / 694; 64 of 2 x 1536 x 2048, of 256 551 / 556, 585 / 548, 597 / 537, 538 / 481."""
-    def cost(bn):
-        return max(2.0 * bn, (128 + bn / 2) * 128 / 70) / bn * (1 + bn / (2 * avg))
-    return min(range(80, 257, 16), key=cost)
+    """Token tile of the grouped pair GEMM for groups of ``avg`` rows (more than 64): large ones, as measured over routers that fill the groups alike and unevenly.  A large
+    tile wins by more than its rows over the half of one that a group leaves empty, and small ones that even groups fill to the brim gain nothing there
+    and lose up to a fifth elsewhere.  An expert layer, us with tiles of 112 / 160 / 208 / 256, groups that spread by about 2, by 15 and by 45 times the root of their average:
+    256 experts of 2 x 512 x 2048, groups of 71 rows 443 / 443 / 447 / 456, 507 / 485 / 484 / 498, 390 / 360 / 343 / 345, of 256 1035 / 897 / 876 / 845, 1097 / 920 / 868 / 865,
+    957 / 818 / 740 / 741; 32 of 2 x 2880 x 2880, of 287 898 / 731 / 718 / 711, 936 / 769 / 673 / 672, 924 / 771 / 694 / 665, of 512 1406 / 1180 / 967 / 881, 1405 / 1099 / 962 / 942, 1408 /
+    1091 / 947 / 898; 64 of 2 x 1536 x 2048, of 143 479 / 378 / 354 / 358, 473 / 411 / 401 / 409, 456 / 399 / 379 / 374."""
+    return 192 if avg <= 100 else 208 if avg <= 160 else 256
 
 
 def _moe_grouped_gemm(a: Act, ids, local, weights, gate_up: QuantWeight, down: QuantWeight, act, gate_up_bias, down_bias,
