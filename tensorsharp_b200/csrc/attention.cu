@@ -527,6 +527,7 @@ extern "C" int tsb_attn_decode_noalloc(const AttnArgs* args, void* stream) {
     float* base = g_attn_noalloc_ptr[dev];
     a.part_o = base;                       // [B, Hq, splits, Dh]
     a.part_ml = base + slots * a.Dh;       // [B, Hq, splits, 2]
+    a.plan = nullptr;                      // whose parts have no place here
     // always the two-kernel form: the in-kernel split merge would bring in a second shared array (its arrival tickets)
     return attn_decode_impl(&a, stream, false);
 }
