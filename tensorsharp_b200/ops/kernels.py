@@ -1528,11 +1528,18 @@ def gdn_chunked(qkv, z, beta, alpha, dt_bias, a_log, norm_w, state, cu_q, h_cu_q
     nc = (max(h_cu_q[i + 1] - h_cu_q[i] for i in range(B)) + 63) // 64
     dev = qkv.device
     assert qkv.dtype == torch.float32 and beta.dtype == alpha.dtype and beta.stride(0) == alpha.stride(0)
-    assert state.dtype == torch.float32 and state.is_contiguous() and seq_slots.dtype == torch.int64
+    assert state.dtype == torch.float32 and seq_slots.dtype == torch.int64
     check_index("gdn_chunked", "state slot", seq_slots, state.shape[0])
     check_index("gdn_chunked", "row offset", cu_q, T + 1)
-    if qkv.stride(1) != 1 or qkv.stride(0) % 4 or qkv.data_ptr() % 16:
+    if not state.is_contiguous() or state.data_ptr() % 16:          # a slice of wider rows: the sequences' states dense, and back
+        dense = state[seq_slots].contiguous()
+        out = gdn_chunked(qkv, z, beta, alpha, dt_bias, a_log, norm_w, dense, cu_q, h_cu_q, torch.arange(B, device=dev), Hk=Hk, Hv=Hv, Dk=Dk, Dv=Dv, eps=eps)
+        state[seq_slots] = dense
+        return out
+    if qkv.stride(1) != 1 or qkv.stride(0) % 4:
         qkv = qkv.contiguous()
+    if qkv.data_ptr() % 16:
+        qkv = qkv.clone(memory_format=torch.contiguous_format)
     BH = B * Hv
     f32 = dict(dtype=torch.float32, device=dev)
     Ks, Qs = torch.empty((B * Hk, nc, 64 * Dk), **f32), torch.empty((B * Hk, nc, 64 * Dk), **f32)
